@@ -563,8 +563,13 @@ def run_gpu(args):
     noise_avg_s = statistics.mean(noise_ms) / 1e3 * args.steps / max(1, noise_launches)
     shots_per_noise_launch = shots * args.steps / max(1, noise_launches)
     noise_achieved = philox_per_shot * shots_per_noise_launch / noise_avg_s if noise_launches else None
+    if noise_launches == 0 and args.noise_mode == -1:  # symptom sampling draws the noise in its one kernel
+        noise_avg_s, shots_per_noise_launch = statistics.mean(frame_ms) / 1e3, shots
+        noise_achieved = philox_per_shot * shots / noise_avg_s
     link = measure_link(local)
     # Transpose: reads the detector-major rows (16 bytes per row per 128 shots) and writes the shot-major rows.
+    # (Symptom sampling is one kernel, reported as the frame kernel: no noise kernel and no transpose.)
+    symptoms = noise_launches == 0 and args.noise_mode == -1
     tr_ms = statistics.mean(t - f - z for t, f, z in zip(step_ms, frame_ms, noise_ms))
     tr_bytes = shots * ((D + O) / 8 + drow + orow)
     hbm_peak = _measured_hbm_peak()
@@ -618,7 +623,14 @@ def run_gpu(args):
                     if e2e_parts else None,
                     "tail": e2e_tail(e2e_times, e2e_parts)},
             "gpu_launches": launches,
-            "roofline": {"bound": "smem", "achieved": achieved_gbs, "peak": smem_peak, "unit": "GB/s",
+            "roofline": {"bound": "hbm", "achieved": shots * (drow + orow) / frame_avg_s / 1e9, "peak": hbm_peak,
+                         "unit": "GB/s", "frac": shots * (drow + orow) / frame_avg_s / 1e9 / hbm_peak,
+                         "traffic": (drow + orow) * shots_per_frame_launch,
+                         "traffic_note": "shot rows written per launch; the kernel reads only its lists (L2-resident)",
+                         "basis": "symptom kernel: shot-major rows written per step / its CUDA-event time; peak = "
+                                  "measured HBM copy bandwidth; instruction issue bounds it, see roofline_noise"}
+            if symptoms else
+                        {"bound": "smem", "achieved": achieved_gbs, "peak": smem_peak, "unit": "GB/s",
                          "frac": achieved_gbs / smem_peak,
                          "traffic": FRAME_DRAM_BYTES_PER_SHOT * shots_per_frame_launch,
                          "traffic_note": "DRAM bytes per frame-kernel launch (ncu per-shot figure x shots per "
@@ -636,7 +648,8 @@ def run_gpu(args):
                                         "launch / its CUDA-event time; peak = project Philox probe "
                                         "(gfs_measure_int_peaks)"},
             "lop3_peak_ops_per_s": int_peaks["lop3_per_s"],
-            "roofline_transpose": {"bound": "hbm", "achieved": tr_bytes / (tr_ms / 1e3) / 1e9, "peak": hbm_peak,
+            "roofline_transpose": None if symptoms else
+                                  {"bound": "hbm", "achieved": tr_bytes / (tr_ms / 1e3) / 1e9, "peak": hbm_peak,
                                    "unit": "GB/s", "frac": tr_bytes / (tr_ms / 1e3) / 1e9 / hbm_peak,
                                    "basis": "detector-major rows read + shot-major rows written per step; "
                                             "peak = measured HBM copy bandwidth"},

@@ -571,6 +571,7 @@ gfs_status gfs_sampler_set_shape(gfs_sampler *s, int blocks_per_cta, int threads
         }
         ck(cudaSetDevice(s->device), "cudaSetDevice");
         s->choose_shape(blocks_per_cta, threads, grid, s->ring_pref);
+        s->frame_chosen = true;
     });
 }
 

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include "program.h"
+#include "symptoms.h"
 
 namespace gfs {
 
@@ -113,6 +114,30 @@ cudaError_t batch_frame_kernel_max_ctas_per_sm(const LaunchShape &shape, int *ou
 cudaError_t launch_batch_noise_kernel(const BatchArgs &args, int blocks_per_cta, cudaStream_t stream);
 cudaError_t launch_batch_frame_kernel_lean(const BatchArgs &args, const LaunchShape &shape, cudaStream_t stream);
 cudaError_t batch_frame_kernel_lean_max_ctas_per_sm(const LaunchShape &shape, int *out);
+
+// Symptom sampling (symptoms.h, symptoms.cu).
+struct SymArgs {
+    const uint4 *entries;
+    const uint32_t *longs;
+    const SymItem *items;
+    const SymStage *stages;
+    uint32_t nstages;
+    const uint32_t *tables;
+    const DevChan *chans;
+    uint64_t seed;
+    uint64_t block0;   // stream position (global 128-shot block index) of local block 0
+    uint64_t nshots;
+    uint32_t ndet, nobs;
+    uint32_t words;       // detector words per shot row in shared memory
+    uint32_t stride;      // words per shot row, observables included (a multiple of four)
+    uint32_t log_blocks;  // 128-shot blocks per CTA, log2
+    // Shot-major outputs (null: not wanted); append: the observables follow the detectors in the detector rows.
+    uint8_t *dets, *obs;
+    uint64_t dets_stride, obs_stride;
+    int packed, append;
+};
+size_t symptom_smem_bytes(uint32_t stride, uint32_t log_blocks);
+cudaError_t launch_symptoms(const SymArgs &args, cudaStream_t stream);
 
 // Transposes [local block][rows] bit-rows (128 shots per entry) of up to three sources, concatenated
 // (src0 rows, then src1, then src2), into shot-major output rows.  `xor_rows` (optional) is a bit vector over the

@@ -6,6 +6,7 @@
 
 #include "circuit.h"
 #include "program.h"
+#include "symptoms.h"
 
 namespace gfs {
 
@@ -46,6 +47,7 @@ struct Program {
     std::vector<uint64_t> lean_inst;
     std::vector<OccXform> occ_xform;  // transforms of the hit occurrences the lean plan moved (NoiseOcc.xform)
     bool lean_ok = false;
+    SymptomTable symptoms;  // outputs flipped by each noise hit (detection sampling; symptoms.h)
 };
 
 struct LowerOptions {

@@ -160,6 +160,13 @@ struct gfs_sampler {
     int lean_pref = -1;  // -1 automatic (lean when possible), 0 never, 1 when possible
     bool lean_ready = false;
     gfs::LaunchShape shape_lean{};
+    // Symptom sampling (symptoms.h): detection calls run symptom_kernel when the program has an output table, unless the
+    // caller chose a frame kernel, its launch shape or its noise mode.
+    DevBuf d_sym_entries, d_sym_longs, d_sym_items, d_sym_stages;
+    gfs::SymArgs sym{};    // the constant arguments
+    size_t sym_items = 0;  // segments of a 128-shot block
+    bool sym_ready = false;
+    bool frame_chosen = false;  // a launch shape was set
     int occs_blocks = 0;          // blocks per slice the uploaded occurrence regions were planned for
     uint64_t slice_cap = 0;       // records per slice region
     uint64_t n_hit_overflows = 0;
@@ -402,7 +409,101 @@ struct gfs_sampler {
         ck(cudaHostGetDevicePointer((void **)&h_words_dev, h_words, 0), "cudaHostGetDevicePointer");
         ck(cudaMemsetAsync(d_status.p, 0, 16, stream), "memset");
         default_shape();
+        init_symptoms();
         ck(cudaStreamSynchronize(stream), "upload sync");
+    }
+
+    // Output lists, items and stages on the device, when the program has a table that is worth it.
+    void init_symptoms() {
+        gfs::SymptomTable &t = prog.symptoms;
+        const uint64_t D = prog.num_detectors, O = prog.num_observables;
+        // Lists so long that flipping outputs one by one costs more than walking the frames (prog.work: the frame rows
+        // a block touches; a hit costs a frame kernel about four of them) stay with the frame kernels.  No circuit of the
+        // test set or the benchmark comes near this line (d=25: 40 K flips against 537 K rows).
+        if (!t.ok || D + O == 0 || t.flips_per_block > prog.work + 4 * prog.hits_per_block) {
+            return;
+        }
+        // All outputs of a block at once while its rows take at most 50 KB (four CTAs per SM), else a window: 128 words a
+        // shot (three CTAs) where the stages fit (d=25: 2.46 ms per 2^20 shots; 64 words, six CTAs, twice the stages:
+        // 3.11; 96: 2.81; 160: 3.00), otherwise 256.
+        const uint32_t ow = (uint32_t)((O + 31) / 32);
+        gfs::SymptomPlan plan;
+        bool planned = false;
+        if ((D + O + 31) / 32 <= 96) {
+            planned = gfs::plan_symptoms(prog, 0, plan);
+        } else {
+            for (uint32_t w = 128; w <= 256 && !planned; w *= 2) {
+                planned = gfs::plan_symptoms(prog, w, plan);
+            }
+        }
+        uint32_t stride = (plan.words + ow + 3) / 4 * 4;
+        stride += stride % 32 == 0 ? 4 : 0;  // consecutive shots on different banks
+        if (!planned || gfs::symptom_smem_bytes(stride, 0) > (size_t)200 << 10) {
+            return;
+        }
+        try {
+            upload(d_sym_entries, t.entries, device, stream);
+            upload(d_sym_longs, t.longs, device, stream);
+            upload(d_sym_items, plan.items, device, stream);
+            upload(d_sym_stages, plan.stages, device, stream);
+            ck(cudaStreamSynchronize(stream), "upload sync");
+        } catch (const CudaError &e) {
+            if (e.code != cudaErrorMemoryAllocation) {
+                throw;
+            }
+            cudaGetLastError();  // no room for the lists: the frame kernels need none
+            for (DevBuf *b : {&d_sym_entries, &d_sym_longs, &d_sym_items, &d_sym_stages}) {
+                b->release();
+            }
+            return;
+        }
+        sym.entries = (const uint4 *)d_sym_entries.p;
+        sym.longs = (const uint32_t *)d_sym_longs.p;
+        sym.items = (const gfs::SymItem *)d_sym_items.p;
+        sym.stages = (const gfs::SymStage *)d_sym_stages.p;
+        sym.nstages = (uint32_t)plan.stages.size();
+        sym.tables = (const uint32_t *)d_tables.p;
+        sym.chans = (const gfs::DevChan *)d_chans.p;
+        sym.seed = seed;
+        sym.ndet = (uint32_t)D;
+        sym.nobs = (uint32_t)O;
+        sym.words = plan.words;
+        sym.stride = stride;
+        sym_items = plan.items.size();
+        std::vector<uint32_t>().swap(t.entries);  // on the device now
+        std::vector<uint32_t>().swap(t.longs);
+        sym_ready = true;
+    }
+
+    // Whether a detection call with these layout flags runs symptom_kernel.
+    bool symptoms_active(uint32_t flags) const {
+        return sym_ready && mode == GFS_MODE_DETECTIONS && !frame_chosen && hits_pref == -1 && lean_pref == -1 &&
+               ring_pref == -1 && hit_capacity_override == 0 && !(flags & GFS_PREPEND_OBSERVABLES);
+    }
+
+    // Enqueues the sampling of `cs` shots from stream block `block0` on into device rows.
+    void run_symptoms(uint64_t cs, uint64_t block0, uint32_t flags, uint8_t *dd, uint64_t ds, uint8_t *od, uint64_t os) {
+        gfs::SymArgs a = sym;
+        a.block0 = block0;
+        a.nshots = cs;
+        a.dets = dd;
+        a.dets_stride = ds;
+        a.obs = od;
+        a.obs_stride = os;
+        a.packed = flags & GFS_BIT_PACKED ? 1 : 0;
+        a.append = flags & GFS_APPEND_OBSERVABLES ? 1 : 0;
+        // Several blocks per CTA while a block has few segments for its 256 lanes and the grid still covers every SM
+        // twice (d=3, 30 segments, 2^20 shots: 72 us with one block per CTA, 41 with eight; d=9, 395 segments, 2^18
+        // shots: 57 and 48 with two; few blocks: 2^16 shots of d=3 take 12 us with one, 16 with eight).
+        const uint64_t nblk = (cs + 127) / 128;
+        uint32_t lb = 0;
+        while (lb < 3 && (nblk >> (lb + 1)) >= 2 * (uint64_t)num_sms && (sym_items << lb) < 512 &&
+               gfs::symptom_smem_bytes(a.stride, lb + 1) <= (size_t)48 << 10) {
+            lb++;
+        }
+        a.log_blocks = lb;
+        ck(gfs::launch_symptoms(a, stream), "symptom kernel launch");
+        n_frame++;
     }
 
     uint64_t per_block_bytes(uint64_t out_row_bytes) const {
@@ -655,6 +756,17 @@ struct gfs_sampler {
         return std::min<uint64_t>(cb, std::max<uint64_t>(1, wave));
     }
 
+    // Chunk size (in 128-shot blocks) for host destinations of symptom sampling: 64 MiB of rows, so that the pipeline's
+    // fill (the first chunk's kernel) and drain stay short while copies are long enough for the link's rate (d=25,
+    // 2^18 shots into page-locked arrays: 2.85 ms; 32 MiB 2.88, 128 MiB 3.0, 16 MiB 3.7).
+    uint64_t symptom_host_blocks(uint64_t nblk_total, uint64_t slot_row_bytes) const {
+        if (chunk_shots) {
+            return std::max<uint64_t>(1, chunk_shots / 128);
+        }
+        const uint64_t bytes = (uint64_t)64 << 20;
+        return std::min(nblk_total, std::max<uint64_t>(1, bytes / std::max<uint64_t>(1, 128 * slot_row_bytes)));
+    }
+
     // Device->host copy of `rows` rows of `width` bytes on copy_stream: one linear copy when both sides are
     // contiguous (a strided copy of narrow rows moves them one by one).
     void copy_rows(uint8_t *dst, uint64_t dpitch, const uint8_t *src, uint64_t spitch, uint64_t width, uint64_t rows,
@@ -690,10 +802,12 @@ struct gfs_sampler {
     }
 
     template <typename Produce, typename Copy>
-    void host_pipeline(uint64_t shots, uint64_t slot_row_bytes, Produce produce, Copy copy, bool eager = false) {
+    void host_pipeline(uint64_t shots, uint64_t slot_row_bytes, Produce produce, Copy copy, bool eager = false,
+                       bool symptoms = false) {
         const uint64_t first_block = next_block;
         uint64_t nblk_total = (shots + 127) / 128;
-        uint64_t cb = host_chunk_blocks(nblk_total, slot_row_bytes);
+        uint64_t cb = symptoms ? symptom_host_blocks(nblk_total, slot_row_bytes)
+                               : host_chunk_blocks(nblk_total, slot_row_bytes);
         uint64_t slot_bytes = cb * 128 * slot_row_bytes;
         out_tmp.ensure(std::max<uint64_t>(16, 2 * slot_bytes), device);
         uint8_t *slots[2] = {(uint8_t *)out_tmp.p, (uint8_t *)out_tmp.p + slot_bytes};
@@ -728,16 +842,21 @@ struct gfs_sampler {
             uint64_t cs = std::min<uint64_t>(shots - done, cb * 128);
             uint64_t nblk = (cs + 127) / 128;
             ck(cudaEventRecord(pev[slot][0], stream), "event");
-            cur_slot = slot;
-            try {
-                run_frame(nblk, next_block);
-            } catch (...) {
+            if (symptoms) {  // one kernel draws the noise and writes the rows
+                produce(done, cs, slots[slot]);
+                ck(cudaEventRecord(pev[slot][1], stream), "event");
+            } else {
+                cur_slot = slot;
+                try {
+                    run_frame(nblk, next_block);
+                } catch (...) {
+                    cur_slot = -1;
+                    throw;
+                }
                 cur_slot = -1;
-                throw;
+                ck(cudaEventRecord(pev[slot][1], stream), "event");
+                produce(done, cs, slots[slot]);
             }
-            cur_slot = -1;
-            ck(cudaEventRecord(pev[slot][1], stream), "event");
-            produce(done, cs, slots[slot]);
             ck(cudaEventRecord(pev[slot][2], stream), "event");
             inflight[slot] = Chunk{done, cs};
             used[slot] = true;
@@ -768,7 +887,7 @@ struct gfs_sampler {
         ck(cudaEventSynchronize(ev[1]), "sample");
         t_total = elapsed(0, 1);
         t_copy = std::max(0.0, t_total - t_frame - t_noise - t_transpose);
-        if (check_status()) {
+        if (!symptoms && check_status()) {
             // A hit list overflowed somewhere: redo the whole request with inline noise (same results).
             next_block = first_block;
             force_inline = true;
@@ -851,6 +970,7 @@ struct gfs_sampler {
         }
         ck(cudaSetDevice(device), "cudaSetDevice");
         reset_timings();
+        const bool symptoms = symptoms_active(flags);
         if (!device_out) {
             // Staging rows use the caller's stride when its rows are contiguous, so that each chunk leaves in
             // one linear copy; otherwise they are padded to 32 bytes and copied row by row.
@@ -858,6 +978,10 @@ struct gfs_sampler {
             host_pipeline(
                 shots, ds + os,
                 [&](uint64_t, uint64_t cs, uint8_t *buf) {
+                    if (symptoms) {
+                        run_symptoms(cs, next_block, flags, dets ? buf : nullptr, ds, obs ? buf + cs * ds : nullptr, os);
+                        return;
+                    }
                     transpose_detections(flags, cs, buf, ds, buf + cs * ds, os, dets != nullptr, obs != nullptr);
                 },
                 [&](uint64_t done, uint64_t cs, uint8_t *buf) {
@@ -868,7 +992,16 @@ struct gfs_sampler {
                         copy_rows(obs + done * ostride, ostride, buf + cs * ds, os, orow, cs, "copy obs");
                     }
                 },
-                page_locked({dets, obs}));
+                page_locked({dets, obs}), symptoms);
+            return;
+        }
+        if (symptoms) {
+            ck(cudaEventRecord(ev[0], stream), "event");
+            run_symptoms(shots, next_block, flags, dets, dstride, obs, ostride);
+            ck(cudaEventRecord(ev[1], stream), "event");
+            ck(cudaStreamSynchronize(stream), "sample");
+            next_block += (shots + 127) / 128;
+            t_frame = t_total = elapsed(0, 1);
             return;
         }
         ck(cudaEventRecord(ev[0], stream), "event");

@@ -1,0 +1,395 @@
+// Symptom sampling kernel for sm_103a (symptoms.h).
+//
+// A CTA owns one or more 128-shot blocks and holds their output rows, shot-major, in shared memory: all of the
+// outputs, or a window of detectors that moves through the circuit stage by stage (an error's detectors lie close to
+// it in time).  Lanes draw the noise contract (gfs_contract.h) segment by segment and XOR each hit's output list
+// into the hit's shot row, so the rows leave as they are: no frames, no hit lists in memory, no transposition.
+//
+// A lane holds one segment and the next one's descriptor (loaded while the first is drawn).  One iteration is one
+// Philox call and up to two hits: gap, choice, gap, choice for a channel that draws its Pauli; a channel that does not
+// uses two of the four draws as gaps.  Hits go to the warp's queue in shared memory and are applied 32 at a time, one
+// per lane, each list loaded one step before it is applied.
+//
+// What bounds it: instruction issue.  The output alone would take 0.31 ms at d=25 (2.05 GB per 2^20 shots at 6.7 TB/s),
+// the contract's Philox calls 0.18 ms (580 G calls/s).  d=25, p=1e-3, 2^20 shots: 2.46 ms where noise, frame and
+// transpose kernels took 7.81; d=11, p=5e-3: 0.64 ms (2.22); d=13 colour code, p=1e-2, 200,001 shots: 0.27 ms (0.97).
+// On the way: hits applied as each lane draws them, with the gap table for every draw, 5.2 ms; the float estimate of
+// the gap instead of the table and prefetched descriptors 3.7; the hit queue 2.9; rows written by bulk copies instead
+// of word stores 2.46.
+#include "frame_device.cuh"
+
+namespace gfs {
+
+namespace {
+
+// The position a gap draw leads to (as gfs_hit_after_draw), without the gap table where the float estimate decides.
+// e = log2(u / 2^32) / log2(1 - p) has G(u) = floor(e) unless e is close to an integer.  With c = -1 / log2(1 - p), the
+// error of e is below 3.6e-7 e (__log2f outside (0.5, 2): 2 ulp; the factor c and the product: one rounding each) plus
+// 4.3e-7 c (the conversion of u: 2^-24 relative; __log2f inside (0.5, 2): 2^-22; for u >= 2^24 the table's rounding to
+// 2^-32): eps is 1.2 times that, and exact subtractions of integers below 2^22 add nothing.  Smaller u belong to gaps
+// above 8 c: longer than a segment when that exceeds 2,060, else the table decides.
+__device__ __forceinline__ int32_t gap_step(uint32_t u, const SymArgs &a, uint32_t chan, float inv_c, int32_t pos,
+                                            int32_t trials) {
+    const int32_t room = trials - pos - 1;
+    const float e = fminf(__log2f(__uint2float_rn(u) * 2.3283064365386963e-10f) * -inv_c, 4096.0f);
+    const float magic = 12582912.0f;  // 1.5 * 2^23: adding it rounds to the nearest integer, left in the low bits
+    const float m = e + magic, d = e - (m - magic);
+    const int32_t k = __float_as_int(m) - 0x4B400000 - (d < 0.0f ? 1 : 0);  // floor(e)
+    const bool sure = fabsf(d) >= fmaf(e, 4.4e-7f, inv_c * 5.2e-7f) && (u >= (1u << 24) || inv_c > 257.5f);
+    if (!sure) {
+        return gfs_hit_after_draw(u, a.tables + __ldg(&a.chans[chan].table), inv_c, pos, room);
+    }
+    return k >= room ? -1 : pos + 1 + k;
+}
+
+// Bits by which a shot's detector columns are shifted in its shared-memory row, so that the row's 16-byte units are the
+// aligned ones of its (packed) destination.
+template <bool PACKED>
+__device__ __forceinline__ uint32_t row_shift(const SymArgs &a, uint32_t dst0, uint32_t r) {
+    return PACKED ? ((dst0 + r * (uint32_t)a.dets_stride) & 15u) * 8u : 0u;
+}
+
+// XORs one output list into shot row `row` (col0 = the row's column of relative code 0).
+__device__ __forceinline__ void flip_outputs(const SymArgs &a, uint32_t *row, uint32_t col0, uint4 e) {
+    auto det = [&](uint32_t code) {
+        const uint32_t col = col0 + code;
+        atomicXor(row + (col >> 5), 1u << (col & 31u));
+    };
+    auto obs = [&](uint32_t o) { atomicXor(row + a.words + (o >> 5), 1u << (o & 31u)); };
+    const uint32_t first = e.x & 0xFFFFu;
+    if (first == kSymLong) {
+        for (uint32_t j = 0; j < e.z; j++) {
+            const uint32_t c = __ldg(a.longs + e.y + j);
+            if (c & kSymObs) {
+                obs(c & ~kSymObs);
+            } else {
+                det(c);
+            }
+        }
+        return;
+    }
+    if ((e.w >> 16) != kSymNone) {
+        obs(e.w >> 16);
+    }
+    const uint32_t code[7] = {first, e.x >> 16, e.y & 0xFFFFu, e.y >> 16, e.z & 0xFFFFu, e.z >> 16, e.w & 0xFFFFu};
+#pragma unroll
+    for (int j = 0; j < 7; j++) {
+        if (code[j] == kSymNone) {
+            break;
+        }
+        det(code[j]);
+    }
+}
+
+constexpr uint32_t kThreads = 256;  // per CTA (d=25: 128 threads 3.57 ms per 2^20 shots, 192 2.82, 256 2.46)
+constexpr uint32_t kHitQueue = 96;  // hits a warp can hold: fewer than 32 left over and two per lane
+
+// Draws the stage's items: work index j is item item0 + j / blocks of the CTA's block j % blocks; a warp takes 32
+// indices at a time from the CTA's counter.  q: the warp's hit queue.
+template <bool PACKED>
+__device__ __forceinline__ void draw_stage(const SymArgs &a, const SymStage &st, uint32_t *win, uint32_t *next, uint2 *q,
+                                           uint32_t block0, uint32_t nblk, uint32_t dst0) {
+    const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+    const uint32_t lb = a.log_blocks, total = (st.item1 - st.item0) << lb;
+    const uint32_t k0 = (uint32_t)a.seed, k1 = (uint32_t)(a.seed >> 32);
+    const uint4 *const items = reinterpret_cast<const uint4 *>(a.items + st.item0);
+    uint32_t cur = 0, end = 0;  // this warp's unclaimed indices
+    bool more = true;
+    bool live = false, ready = false;  // a segment is being drawn / the next one's descriptor is loaded
+    uint4 lo = make_uint4(0, 0, 0, 0), hi = lo, nlo = lo, nhi = lo;
+    uint32_t blk = 0, nblk_idx = 0, draw = 0;
+    int32_t pos = -1;
+    uint32_t qn = 0;  // queued hits (warp-uniform)
+    uint4 list = lo;  // the list of a hit taken from the queue, applied when the next one is taken
+    uint32_t hit = 0;
+    bool pending = false;
+    auto apply = [&]() {
+        if (pending) {
+            const uint32_t r = hit >> 16;
+            flip_outputs(a, win + r * a.stride, (hit & 0xFFFFu) + row_shift<PACKED>(a, dst0, r), list);
+        }
+    };
+    for (;;) {
+        if (!live && ready) {
+            lo = nlo;
+            hi = nhi;
+            blk = nblk_idx;
+            draw = 0;
+            pos = -1;
+            live = true;
+            ready = false;
+        }
+        const uint32_t want = __ballot_sync(0xFFFFFFFFu, !ready);
+        if (want) {
+            if (cur >= end && more) {
+                if (lane == 0) {
+                    cur = atomicAdd(next, 32u);
+                }
+                cur = __shfl_sync(0xFFFFFFFFu, cur, 0);
+                more = cur < total;
+                end = min(cur + 32u, total);
+            }
+            const uint32_t j = cur + __popc(want & lt);
+            if (!ready && j < end) {
+                nblk_idx = j & ((1u << lb) - 1u);
+                if (nblk_idx < nblk) {
+                    nlo = __ldg(items + 2 * (j >> lb));
+                    nhi = __ldg(items + 2 * (j >> lb) + 1);
+                    ready = true;
+                }
+            }
+            cur = min(cur + __popc(want), max(cur, end));
+        }
+        uint2 hit0 = make_uint2(0, 0), hit1 = hit0;
+        bool g0 = false, g1 = false;
+        if (live) {
+            const uint32_t kind = hi.x & 0xFFu, pu = (hi.x >> 8) & 0xFFu;
+            const int32_t trials = (int32_t)(hi.x >> 16);
+            const bool choice = pu > 1;
+            const gfs_u32x4 r = gfs_philox(k0, k1, block0 + blk, lo.x, lo.y, lo.z | ((choice ? draw : draw >> 1) & 0xFFFFFu));
+            const bool odd = (draw & 1u) != 0;
+            const uint32_t u0 = choice || !odd ? r.v[0] : r.v[2];
+            const uint32_t u1 = choice ? r.v[2] : odd ? r.v[3] : r.v[1];
+            uint32_t v0 = gfs_choice_uniform(r.v[1], pu), v1 = gfs_choice_uniform(r.v[3], pu);
+            if (kind == KN_PC1) {
+                v0 = pauli_xz(1 + gfs_choice_weighted(r.v[1], a.chans[hi.w].cum, 3)) - 1;
+                v1 = pauli_xz(1 + gfs_choice_weighted(r.v[3], a.chans[hi.w].cum, 3)) - 1;
+            } else if (kind == KN_PC2) {
+                const uint32_t w0 = 1 + gfs_choice_weighted(r.v[1], a.chans[hi.w].cum, 15);
+                const uint32_t w1 = 1 + gfs_choice_weighted(r.v[3], a.chans[hi.w].cum, 15);
+                v0 = (pauli_xz(w0 >> 2) | (pauli_xz(w0 & 3) << 2)) - 1;
+                v1 = (pauli_xz(w1 >> 2) | (pauli_xz(w1 & 3) << 2)) - 1;
+            }
+            draw++;
+            const float inv_c = __uint_as_float(hi.z);
+            const uint32_t col = ((blk * GFS_BLOCK_SHOTS) << 16) + hi.y - st.flush0;
+            pos = gap_step(u0, a, hi.w, inv_c, pos, trials);
+            g0 = pos >= 0;
+            if (g0) {
+                const uint32_t p = (uint32_t)pos;
+                hit0 = make_uint2(lo.w + (p >> 7) * pu + v0, ((p & 127u) << 16) + col);
+                if (pos + 1 < trials) {
+                    pos = gap_step(u1, a, hi.w, inv_c, pos, trials);
+                    g1 = pos >= 0;
+                }
+            }
+            if (g1) {
+                const uint32_t p = (uint32_t)pos;
+                hit1 = make_uint2(lo.w + (p >> 7) * pu + v1, ((p & 127u) << 16) + col);
+            }
+            live = g1 && pos + 1 < trials;
+        }
+        const uint32_t m0 = __ballot_sync(0xFFFFFFFFu, g0), m1 = __ballot_sync(0xFFFFFFFFu, g1);
+        if (g0) {
+            q[qn + __popc(m0 & lt)] = hit0;
+        }
+        qn += __popc(m0);
+        if (g1) {
+            q[qn + __popc(m1 & lt)] = hit1;
+        }
+        qn += __popc(m1);
+        __syncwarp();
+        while (qn >= 32) {
+            apply();
+            qn -= 32;
+            const uint2 h = q[qn + lane];
+            list = __ldg(a.entries + h.x);
+            hit = h.y;
+            pending = true;
+            __syncwarp();
+        }
+        if (!more && cur >= end && !__any_sync(0xFFFFFFFFu, live || ready)) {
+            break;
+        }
+    }
+    apply();
+    pending = lane < qn;
+    if (pending) {
+        const uint2 h = q[lane];
+        list = __ldg(a.entries + h.x);
+        hit = h.y;
+    }
+    apply();
+}
+
+template <bool PACKED>
+__device__ __forceinline__ uint32_t out_byte(const uint32_t *row, uint32_t q) {
+    return PACKED ? (row[q >> 2] >> (8 * (q & 3))) & 0xFFu : (row[q >> 5] >> (q & 31)) & 1u;
+}
+
+// Packed rows: a row's 16-byte units are those of its destination, so whole units leave by bulk copies (one per row,
+// issued by one thread, read from shared memory by the copy engine), and only the bytes that share a unit with a
+// neighbouring row, at the ends of the row, are stored singly.
+__device__ __forceinline__ void write_packed(const SymArgs &a, const SymStage &st, const uint32_t *win, uint32_t c1,
+                                             uint64_t shot0, uint32_t nvalid, uint32_t dst0, bool last) {
+    const uint32_t tid = threadIdx.x, nt = blockDim.x;
+    for (uint32_t r = tid; r < nvalid; r += nt) {
+        const uint32_t mis = row_shift<true>(a, dst0, r) >> 3;
+        const uint32_t begin = st.flush0 == 0 && mis ? 16u : 0u;  // byte offsets within the row piece
+        const uint32_t end = last ? (mis + (c1 + 7) / 8 - st.flush0 / 8) & ~15u : (c1 - st.flush0) / 8;
+        if (begin < end) {
+            const uint8_t *src = reinterpret_cast<const uint8_t *>(win + (size_t)r * a.stride) + begin;
+            uint8_t *dst = a.dets + (shot0 + r) * a.dets_stride - mis + st.flush0 / 8 + begin;
+            asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst),
+                         "r"((uint32_t)__cvta_generic_to_shared(src)), "r"(end - begin)
+                         : "memory");
+        }
+    }
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    if (st.flush0 == 0 || last) {
+        const uint32_t half = tid & 15u;  // sixteen threads a row, one byte each of the first and of the last unit
+        for (uint32_t r = tid >> 4; r < nvalid; r += nt >> 4) {
+            const uint8_t *row = reinterpret_cast<const uint8_t *>(win + (size_t)r * a.stride);
+            const uint32_t mis = row_shift<true>(a, dst0, r) >> 3;
+            uint8_t *dst = a.dets + (shot0 + r) * a.dets_stride - mis + st.flush0 / 8;
+            const uint32_t bytes = mis + (c1 + 7) / 8 - st.flush0 / 8;  // past the last byte (last stage)
+            if (st.flush0 == 0 && mis && half >= mis && (!last || half < bytes)) {
+                dst[half] = row[half];
+            }
+            const uint32_t b = (bytes & ~15u) + half;
+            if (last && b < bytes && !(st.flush0 == 0 && mis && b < 16)) {
+                dst[b] = row[b];
+            }
+        }
+    }
+    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the rows may be changed
+}
+
+// Unpacked rows (columns [c0, c1) of every shot): one warp per row, consecutive lanes writing consecutive aligned
+// 32-bit words of four expanded bits; the partial words at the ends byte by byte.
+__device__ __forceinline__ void write_unpacked(const SymArgs &a, const uint32_t *win, uint32_t c0, uint32_t c1,
+                                               uint64_t shot0, uint32_t nvalid) {
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const int32_t nbytes = (int32_t)(c1 - c0);
+    for (uint32_t r = warp; r < nvalid; r += nwarps) {
+        const uint32_t *row = win + (size_t)r * a.stride;
+        uint8_t *const d = a.dets + (shot0 + r) * a.dets_stride + c0;
+        const int32_t mis = (int32_t)((uintptr_t)d & 3u);
+        uint32_t *const dw = reinterpret_cast<uint32_t *>(d - mis);
+        for (int32_t q = (int32_t)lane; 4 * q < mis + nbytes; q += 32) {
+            const int32_t o = 4 * q - mis;  // first byte (column) of this word within the piece
+            if (o >= 0 && o + 4 <= nbytes) {
+                const uint32_t w = (uint32_t)o >> 5;
+                const uint32_t v = __funnelshift_r(row[w], row[w + 1], o & 31);
+                dw[q] = (v & 1u) | (v & 2u) << 7 | (v & 4u) << 14 | (v & 8u) << 21;
+            } else {
+                for (int32_t b = max(o, 0); b < min(o + 4, nbytes); b++) {
+                    d[b] = (uint8_t)out_byte<false>(row, (uint32_t)b);
+                }
+            }
+        }
+    }
+}
+
+// Between stages: the words after the written piece move to the front of their row, the rest is cleared.  All in
+// 16-byte units; a thread owns (row, unit) pairs, the rows of one pass split over the CTA.
+__device__ __forceinline__ void next_window(const SymArgs &a, const SymStage &st, uint32_t *win, uint32_t rows) {
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const uint32_t n = (st.flush1 - st.flush0) / kSymAlign, keep = st.keep / (kSymAlign / 32);  // units
+    for (uint32_t r = warp; r < rows; r += nwarps) {
+        uint4 *const row = reinterpret_cast<uint4 *>(win + (size_t)r * a.stride);
+        for (uint32_t i0 = 0; i0 < n + keep; i0 += 32) {  // a pass reads ahead of what it and earlier ones write
+            const uint32_t i = i0 + lane;
+            const uint4 v = i < keep ? row[n + i] : zero4();
+            __syncwarp();
+            if (i < n + keep) {
+                row[i] = v;
+            }
+            __syncwarp();
+        }
+    }
+}
+
+template <bool PACKED>
+__global__ void __launch_bounds__(kThreads) symptom_kernel(const SymArgs a) {
+    extern __shared__ __align__(16) uint32_t win[];  // [shot][stride]: detector words, then observable words
+    __shared__ uint32_t next;
+    __shared__ uint2 queue[kThreads / 32][kHitQueue];
+    const uint32_t tid = threadIdx.x, nt = blockDim.x;
+    const uint32_t rows = GFS_BLOCK_SHOTS << a.log_blocks;
+    const uint64_t blk0 = (uint64_t)blockIdx.x << a.log_blocks, shot0 = blk0 * GFS_BLOCK_SHOTS;
+    const uint32_t nvalid = a.nshots - shot0 < rows ? (uint32_t)(a.nshots - shot0) : rows;
+    const uint32_t nblk = (nvalid + GFS_BLOCK_SHOTS - 1) / GFS_BLOCK_SHOTS;
+    const uint32_t dst0 = (uint32_t)(uintptr_t)a.dets + (uint32_t)(shot0 * a.dets_stride);  // modulo 16 is what counts
+    for (uint32_t i = tid; i < rows * a.stride; i += nt) {
+        win[i] = 0;
+    }
+    if (tid == 0) {
+        next = 0;
+    }
+    __syncthreads();
+    for (uint32_t k = 0; k < a.nstages; k++) {
+        const SymStage st = a.stages[k];
+        draw_stage<PACKED>(a, st, win, &next, queue[tid >> 5], (uint32_t)(a.block0 + blk0), nblk, dst0);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the rows will be read by bulk copies
+        __syncthreads();
+        const bool last = k + 1 == a.nstages;
+        if (tid == 0) {
+            next = 0;
+        }
+        uint32_t c1 = st.flush1;
+        if (last && a.append && a.nobs) {
+            for (uint32_t r = tid; r < nvalid; r += nt) {
+                uint32_t *const row = win + (size_t)r * a.stride;
+                const uint32_t col0 = a.ndet - st.flush0 + row_shift<PACKED>(a, dst0, r);
+                for (uint32_t o = 0; o < a.nobs; o++) {
+                    row[(col0 + o) >> 5] ^= ((row[a.words + (o >> 5)] >> (o & 31)) & 1u) << ((col0 + o) & 31);
+                }
+            }
+            c1 = a.ndet + a.nobs;
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncthreads();
+        }
+        if (a.dets) {
+            if (PACKED) {
+                write_packed(a, st, win, c1, shot0, nvalid, dst0, last);
+            } else {
+                write_unpacked(a, win, st.flush0, c1, shot0, nvalid);
+            }
+        }
+        if (!last) {
+            __syncthreads();
+            next_window(a, st, win, rows);
+            __syncthreads();
+        }
+    }
+    if (a.obs && a.nobs) {
+        const uint32_t nbytes = PACKED ? (a.nobs + 7) / 8 : a.nobs;
+        for (uint32_t i = tid; i < nvalid * nbytes; i += nt) {
+            const uint32_t r = i / nbytes, q = i % nbytes;
+            a.obs[(shot0 + r) * a.obs_stride + q] = (uint8_t)out_byte<PACKED>(win + (size_t)r * a.stride + a.words, q);
+        }
+    }
+}
+
+template <bool PACKED>
+cudaError_t launch_packed(const SymArgs &args, uint32_t grid, size_t smem, cudaStream_t stream) {
+    cudaError_t e = cudaFuncSetAttribute(symptom_kernel<PACKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) {
+        return e;
+    }
+    symptom_kernel<PACKED><<<grid, kThreads, smem, stream>>>(args);
+    return cudaGetLastError();
+}
+
+}  // namespace
+
+size_t symptom_smem_bytes(uint32_t stride, uint32_t log_blocks) {
+    return ((size_t)GFS_BLOCK_SHOTS << log_blocks) * stride * sizeof(uint32_t);
+}
+
+cudaError_t launch_symptoms(const SymArgs &args, cudaStream_t stream) {
+    if (args.nshots == 0) {
+        return cudaSuccess;
+    }
+    const uint64_t rows = (uint64_t)GFS_BLOCK_SHOTS << args.log_blocks;
+    const uint64_t grid = (args.nshots + rows - 1) / rows;
+    const size_t smem = symptom_smem_bytes(args.stride, args.log_blocks);
+    if (grid > 0x7FFFFFFFull) {
+        return cudaErrorInvalidValue;
+    }
+    return args.packed ? launch_packed<true>(args, (uint32_t)grid, smem, stream)
+                       : launch_packed<false>(args, (uint32_t)grid, smem, stream);
+}
+
+}  // namespace gfs

@@ -1,0 +1,68 @@
+// Symptom sampling: detection sampling without walking the circuit per shot.
+//
+// Every detector and observable is a GF(2)-linear function of the noise hits (and of randomization, which a backward
+// pass shows to reach no output in the circuits this path takes).  That pass (output_analysis.h) therefore
+// also gives, for every unit of every noise occurrence and every Pauli a hit can apply, the outputs such a hit flips.
+// Sampling is then the noise contract alone: symptom_kernel (symptoms.cu) draws each segment's hits and XORs the
+// hits' output lists into shot rows held in shared memory, which leave as the caller's output rows.
+#pragma once
+
+#include <cstdint>
+#include <vector>
+
+#include "program.h"
+
+namespace gfs {
+
+struct Program;
+
+// Output list of one (unit, Pauli): 16 bytes.  Halfwords 0-6 hold detectors (relative to the item's base, 0xFFFF after
+// the last), halfword 7 an observable (0xFFFF: none).  A first halfword of kSymLong marks a list that does not fit:
+// .y = its first word in the long-list pool, .z = its length; pool words are relative detectors, or kSymObs | o.
+constexpr uint32_t kSymNone = 0xFFFFu, kSymLong = 0xFFFEu, kSymObs = 1u << 31;
+
+// One noise segment (gfs_contract.h) as symptom_kernel reads it: a work item.
+struct alignas(16) SymItem {
+    uint32_t c1, c2, c3;  // Philox counter words (segment, instance, purpose and instance; the draw group is added)
+    uint32_t entry;       // list of (unit u of the segment, Pauli v) = entries[entry + u * per_unit + v]
+    uint32_t kind;        // KN_* | per_unit << 8 | trials << 16
+    uint32_t base;        // detector of relative code 0
+    float inv_c;          // of the channel
+    uint32_t chan;
+};
+static_assert(sizeof(SymItem) == 32, "SymItem layout");
+
+constexpr uint32_t kSymAlign = 128;  // detectors per 16 bytes of a packed row, the unit of bulk copies
+
+// A stage draws items [item0, item1) and then writes detectors [flush0, flush1) out (flush0 and, except in the last
+// stage, flush1 are multiples of 32): no later item reaches them.  `keep` words past flush1 may hold flips already.
+struct alignas(16) SymStage {
+    uint32_t item0, item1, flush0, flush1, keep, pad[3];
+};
+
+// What the backward pass found for one occurrence, before stages are planned.
+struct SymList {
+    uint32_t entry = 0, per_unit = 0, kind = 0, n = 0, chan = 0;
+    uint32_t base = 0;      // detector of relative code 0
+    uint32_t lo = 1, hi = 0;  // detectors its lists touch (lo > hi: none)
+    double mean = 0;          // mean list length
+};
+
+// Output lists of a program's noise occurrences (ok = false: the program needs a frame kernel).
+struct SymptomTable {
+    bool ok = false;
+    std::vector<SymList> occ;
+    std::vector<uint32_t> entries;  // four words per list
+    std::vector<uint32_t> longs;
+    double flips_per_block = 0;  // expected output flips per 128-shot block
+};
+
+// Stages of a program for a window of `window_words` 32-detector words per shot (0: all outputs at once).
+struct SymptomPlan {
+    std::vector<SymItem> items;
+    std::vector<SymStage> stages;
+    uint32_t words = 0;  // detector words per shot row held in shared memory (kSymAlign spare for the row's alignment)
+};
+bool plan_symptoms(const Program &prog, uint32_t window_words, SymptomPlan &plan);
+
+}  // namespace gfs

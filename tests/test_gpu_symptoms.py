@@ -1,0 +1,91 @@
+"""Symptom sampling (symptoms.cu) against the frame kernels and the oracle, bit for bit: every layout it writes, shot
+counts around its blocks, destinations at every alignment, windows that move, and gap draws at probabilities where the
+float estimate or the gap table decides."""
+
+import numpy as np
+import pytest
+
+import stim_gb300
+from oracle.oracle import OracleCircuit
+from stim_gb300 import _native, workloads
+from test_symptoms import HAND
+
+pytestmark = pytest.mark.gpu
+
+CODES = [("surface_code:rotated_memory_z", 3, 0.01), ("surface_code:rotated_memory_z", 5, 0.004),
+         ("surface_code:rotated_memory_x", 11, 0.002), ("surface_code:rotated_memory_z", 17, 0.01),
+         ("surface_code:rotated_memory_z", 25, 0.001), ("repetition_code:memory", 51, 0.02),
+         ("color_code:memory_xyz", 15, 0.005)]
+
+
+def texts():
+    out = {f"{f.split(':')[0]}_d{d}": workloads.code_circuit(f, d, d, p) for f, d, p in CODES}
+    out.update(HAND)
+    return out
+
+
+def pair(text, seed):
+    """The sampler as it comes, and one that walks the frames."""
+    c = stim_gb300.Circuit(text)
+    a, b = c.compile_detector_sampler(seed=seed), c.compile_detector_sampler(seed=seed)
+    b.set_noise_mode(1)
+    return c, a, b
+
+
+@pytest.mark.parametrize("name", sorted(texts()))
+@pytest.mark.parametrize("packed", [True, False])
+def test_matches_the_frame_kernels(name, packed):
+    c, a, b = pair(texts()[name], 11)
+    for shots in (1, 127, 128, 129, 1000):  # the streams go on from call to call
+        for kw in ({}, {"append_observables": True}, {"separate_observables": True}, {"prepend_observables": True}):
+            x = a.sample(shots, bit_packed=packed, **kw)
+            y = b.sample(shots, bit_packed=packed, **kw)
+            for u, v in zip(x if isinstance(x, tuple) else (x,), y if isinstance(y, tuple) else (y,)):
+                np.testing.assert_array_equal(u, v)
+
+
+@pytest.mark.parametrize("name", ["surface_code_d3", "surface_code_d17", "surface_code_d25"])
+@pytest.mark.parametrize("packed", [True, False])
+def test_destinations_at_any_alignment(name, packed):
+    torch = pytest.importorskip("torch")
+    c, a, b = pair(texts()[name], 5)
+    shots = 300
+    row = (c.num_detectors + 7) // 8 if packed else c.num_detectors
+    want = b.sample(shots, bit_packed=packed).view(np.uint8)
+    flags = _native.BIT_PACKED if packed else 0
+    for offset, pad in [(k, (5 * k) % 19) for k in range(17)]:
+        buf = torch.full((offset + shots * (row + pad) + 64,), 0xA5, dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
+        a.set_stream_position(0)
+        _native.check(_native.lib().gfs_sample_detections_device(a._h, shots, flags, buf.data_ptr() + offset, row + pad,
+                                                                 None, 0))
+        got = buf.cpu().numpy()
+        rows = got[offset:offset + shots * (row + pad)].reshape(shots, row + pad)
+        np.testing.assert_array_equal(rows[:, :row], want)
+        assert (rows[:, row:] == 0xA5).all() and (got[:offset] == 0xA5).all()  # nothing else is written
+        assert (got[offset + shots * (row + pad):] == 0xA5).all()
+
+
+@pytest.mark.parametrize("p", [1e-7, 3e-6, 1e-5, 1e-4, 1e-3, 2.6e-3, 2.8e-3, 0.01, 0.05, 0.2, 0.6, 0.95])
+def test_gaps_at_any_probability(p):
+    # 40 qubits: two whole segments and a partial one; X flips draw gaps only, depolarizing noise a choice per hit.
+    qs = " ".join(str(q) for q in range(40))
+    text = (f"R {qs}\nX_ERROR({p}) {qs}\nDEPOLARIZE1({min(p, 0.7)}) {qs}\nM({p}) {qs}\n" +
+            "".join(f"DETECTOR rec[-{k + 1}]\n" for k in range(40)) + "OBSERVABLE_INCLUDE(0) rec[-1]\n")
+    shots = 1 << 16
+    s = stim_gb300.Circuit(text).compile_detector_sampler(seed=3)
+    d, o = s.sample(shots, bit_packed=True, separate_observables=True)
+    od, oo, _ = OracleCircuit(text).sample(shots, 3)
+    np.testing.assert_array_equal(d, od)
+    np.testing.assert_array_equal(o, oo)
+    assert s.last_timings()["noise_launches"] == 0  # one kernel
+
+
+def test_a_chosen_frame_kernel_is_used():
+    c = stim_gb300.Circuit(texts()["surface_code_d5"])
+    want = c.compile_detector_sampler(seed=9).sample(500, bit_packed=True)
+    for choose in (lambda s: s.set_noise_mode(1), lambda s: s.set_frame_kernel(1), lambda s: s.set_launch_shape(1, 128)):
+        s = c.compile_detector_sampler(seed=9)
+        choose(s)
+        np.testing.assert_array_equal(s.sample(500, bit_packed=True), want)
+        assert s.last_timings()["noise_launches"] == 1
