@@ -60,6 +60,7 @@ struct gfs_batch {
             throw std::invalid_argument("threads per CTA must be a multiple of 32 in [32, 256]");
         }
         eng.set_shape(progs, bpc, threads, ring);
+        eng.symptoms = false;
         drop_graph();
     }
 
@@ -74,7 +75,7 @@ struct gfs_batch {
 
     // Entries for these shot counts: circuit j continues samplers[j]'s stream (a sampler listed more than
     // once continues from one entry to the next).
-    std::vector<gfs_rt::BatchEntry> entries(const uint64_t *shots, uint8_t *const *dets, const uint64_t *dstride,
+    std::vector<gfs_rt::BatchEntry> entries(const uint64_t *shots, uint32_t flags, uint8_t *const *dets, const uint64_t *dstride,
                                             uint8_t *const *obs, const uint64_t *ostride) const {
         std::vector<gfs_rt::BatchEntry> es(samplers.size());
         std::unordered_map<const gfs_sampler *, uint64_t> next;
@@ -90,6 +91,7 @@ struct gfs_batch {
             e.dstride = dets && dets[j] ? dstride[j] : 0;
             e.obs = obs ? obs[j] : nullptr;
             e.ostride = obs && obs[j] ? ostride[j] : 0;
+            e.flags = flags;
             next[samplers[j]] = b0 + (shots[j] + 127) / 128;
         }
         return es;
@@ -111,8 +113,8 @@ struct gfs_batch {
         }
         ck(cudaSetDevice(eng.device), "cudaSetDevice");
         t_frame = t_transpose = t_copy = t_total = 0;
-        const std::vector<gfs_rt::BatchEntry> es = entries(shots, dets, dstride, obs, ostride);
-        const uint32_t items = eng.prepare(es, order);
+        const std::vector<gfs_rt::BatchEntry> es = entries(shots, flags, dets, dstride, obs, ostride);
+        const uint64_t items = eng.prepare(es, order);
         if (items == 0) {
             return;
         }
@@ -124,6 +126,9 @@ struct gfs_batch {
                                      (uint64_t)(uintptr_t)eng.obs_arena.p, (uint64_t)(uintptr_t)eng.d_desc.p,
                                      (uint64_t)(uintptr_t)eng.d_prefix.p, (uint64_t)(uintptr_t)eng.ring_buf.p,
                                      (uint64_t)eng.lean, (uint64_t)eng.lean_shape.grid, eng.lean_shape.smem};
+        for (const auto &g : eng.groups) {
+            key.insert(key.end(), {(uint64_t)(uintptr_t)g.d_args.p, (uint64_t)(uintptr_t)g.d_prefix.p, g.args.size(), g.smem});
+        }
         for (const auto &e : es) {
             key.push_back(e.shots);
             key.push_back((uint64_t)(uintptr_t)e.dets);
@@ -157,7 +162,7 @@ struct gfs_batch {
             n_graph_builds++;
         } else {
             for (const auto &e : es) {
-                calls += e.shots ? (e.dets ? 1 : 0) + (e.obs ? 1 : 0) : 0;
+                calls += e.shots && !eng.takes_symptoms(e) ? (e.dets ? 1 : 0) + (e.obs ? 1 : 0) : 0;
             }
         }
         ck(cudaEventRecord(eng.ev[0], eng.stream), "event");
@@ -263,8 +268,17 @@ struct gfs_batch {
         };
         const Cand cands[] = {{1, 256, 0}, {1, 256, 1}, {1, 128, 0}, {1, 128, 1}, {2, 256, 0},
                               {2, 256, 1}, {2, 128, 0}, {2, 128, 1}, {4, 256, 0}, {4, 256, 1}};
-        const std::vector<gfs_rt::BatchEntry> es = entries(shots, nullptr, nullptr, nullptr, nullptr);
+        const std::vector<gfs_rt::BatchEntry> es = entries(shots, 0, nullptr, nullptr, nullptr, nullptr);
         double best = -1;
+        const bool symptoms = eng.symptoms;  // the shape is the frame kernel's, so that is what is timed
+        eng.symptoms = false;
+        struct Restore {
+            gfs_rt::BatchEngine &e;
+            bool v;
+            ~Restore() {
+                e.symptoms = v;
+            }
+        } restore{eng, symptoms};
         gfs::LaunchShape best_shape = eng.shape;
         uint64_t best_stride = eng.ring_stride_cur;
         for (const Cand &c : cands) {
@@ -276,8 +290,7 @@ struct gfs_batch {
             if ((c.ring == 1) != eng.shape.ring_global) {
                 continue;
             }
-            const uint32_t items = eng.prepare(es, order);
-            if (items == 0) {
+            if (eng.prepare(es, order) == 0) {
                 break;
             }
             float ms = 0;

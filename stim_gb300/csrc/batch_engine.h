@@ -19,6 +19,7 @@ struct BatchEntry {
     uint64_t dstride = 0;
     uint8_t *obs = nullptr;
     uint64_t ostride = 0;
+    uint32_t flags = 0;  // layout of its rows
 };
 
 inline void layout_rows(const gfs_sampler *s, uint32_t flags, uint64_t *drow, uint64_t *orow) {
@@ -54,6 +55,23 @@ struct BatchEngine {
     std::vector<uint64_t> wprefix;
     uint64_t noise_warps = 0;
 
+    // Symptom sampling (symptoms.h): entries whose sampler takes it are left out of the frame launches and sampled by
+    // up to kGroups batched symptom launches, one per (shared-memory class, packed or not): entries whose rows leave
+    // room for four CTAs per SM do not share a launch, and so its shared-memory size, with those that do not.
+    static constexpr int kGroups = 4;
+    static constexpr size_t kSmallSmem = (size_t)49 << 10;
+    struct SymGroup {
+        std::vector<gfs::SymArgs> args;
+        std::vector<uint32_t> prefix;
+        DevBuf d_args, d_prefix;
+        size_t smem = 0;
+    };
+    SymGroup groups[kGroups];
+    cudaStream_t side[kGroups - 1] = {};  // the groups run side by side
+    cudaEvent_t fork = nullptr, join[kGroups - 1] = {};
+    bool symptoms = true;  // false: the caller chose a launch shape of the frame kernel
+    std::vector<uint8_t> by_symptoms;  // per entry (input order)
+
     // Current plan (set by prepare()).
     std::vector<gfs::KernelArgs> desc;
     std::vector<uint32_t> prefix;
@@ -74,6 +92,18 @@ struct BatchEngine {
                 }
             }
             cudaStreamDestroy(stream);
+            for (int g = 0; g < kGroups - 1; g++) {
+                if (side[g]) {
+                    cudaStreamSynchronize(side[g]);
+                    cudaStreamDestroy(side[g]);
+                }
+                if (join[g]) {
+                    cudaEventDestroy(join[g]);
+                }
+            }
+            if (fork) {
+                cudaEventDestroy(fork);
+            }
         }
     }
 
@@ -88,6 +118,11 @@ struct BatchEngine {
         for (auto &e : ev) {
             ck(cudaEventCreate(&e), "cudaEventCreate");
         }
+        for (int g = 0; g < kGroups - 1; g++) {
+            ck(cudaStreamCreateWithFlags(&side[g], cudaStreamNonBlocking), "cudaStreamCreate");
+            ck(cudaEventCreateWithFlags(&join[g], cudaEventDisableTiming), "cudaEventCreate");
+        }
+        ck(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming), "cudaEventCreate");
         d_counter.ensure(16, device);
         d_status.ensure(16, device);
         ck(cudaMemsetAsync(d_status.p, 0, 16, stream), "memset");
@@ -196,11 +231,95 @@ struct BatchEngine {
         set_shape(progs, 1, 128, -1);
     }
 
+    // Whether entry e is sampled by its output lists.
+    bool takes_symptoms(const BatchEntry &e) const {
+        return symptoms && e.prog->symptoms_active(e.flags);
+    }
+
+    // The symptom launches of the plan (launch order as prepare's).
+    uint64_t prepare_symptoms(const std::vector<BatchEntry> &entries, const std::vector<uint32_t> &order) {
+        uint64_t ctas = 0, blocks = 0;
+        by_symptoms.assign(entries.size(), 0);
+        for (const BatchEntry &e : entries) {
+            blocks += (e.shots + 127) / 128;
+        }
+        for (SymGroup &g : groups) {
+            g.args.clear();
+            g.prefix.assign(1, 0);
+            g.smem = 0;
+        }
+        for (size_t k = 0; k < entries.size(); k++) {
+            const size_t j = order.empty() ? k : order[k];
+            const BatchEntry &e = entries[j];
+            if (!takes_symptoms(e)) {
+                continue;
+            }
+            by_symptoms[j] = 1;
+            if (e.shots == 0) {
+                continue;
+            }
+            gfs::SymArgs a = e.prog->symptom_args(e.shots, e.block0, e.flags, e.dets, e.dstride, e.obs, e.ostride, blocks);
+            a.seed = e.seed;
+            const size_t smem = gfs::symptom_smem_bytes(a.stride, a.log_blocks);
+            SymGroup &g = groups[(smem > kSmallSmem ? 0 : 2) + (a.packed ? 0 : 1)];
+            const uint64_t per = (uint64_t)128 << a.log_blocks;
+            const uint64_t upto = g.prefix.back() + (e.shots + per - 1) / per;
+            if (upto > 0x7FFFFFFFull) {
+                throw std::invalid_argument("batch has too many 128-shot slices for one launch");
+            }
+            g.args.push_back(a);
+            g.prefix.push_back((uint32_t)upto);
+            g.smem = std::max(g.smem, smem);
+            ctas += (e.shots + per - 1) / per;
+        }
+        for (SymGroup &g : groups) {
+            if (g.args.empty()) {
+                continue;
+            }
+            upload(g.d_args, g.args, device, stream);
+            upload(g.d_prefix, g.prefix, device, stream);
+        }
+        return ctas;
+    }
+
+    void enqueue_symptoms() {
+        bool first = true, forked = false;
+        int used = 0;
+        for (SymGroup &g : groups) {
+            if (g.args.empty()) {
+                continue;
+            }
+            cudaStream_t st = stream;
+            if (!first) {
+                if (!forked) {
+                    throw std::logic_error("symptom launches without a fork");
+                }
+                st = side[used];
+                ck(cudaStreamWaitEvent(st, fork, 0), "fork");
+            } else {
+                ck(cudaEventRecord(fork, stream), "fork");
+                forked = true;
+            }
+            ck(gfs::launch_batch_symptoms((const gfs::SymArgs *)g.d_args.p, (const uint32_t *)g.d_prefix.p,
+                                          (uint32_t)g.args.size(), g.prefix.back(), g.smem, g.args[0].packed != 0, st),
+               "batch symptom kernel launch");
+            if (!first) {
+                ck(cudaEventRecord(join[used], st), "join");
+                used++;
+            }
+            first = false;
+        }
+        for (int k = 0; k < used; k++) {
+            ck(cudaStreamWaitEvent(stream, join[k], 0), "join");
+        }
+    }
+
     // Plans the entries (launch order = `order`, or input order when empty), allocates the arenas and
-    // uploads the descriptors.  Returns the number of work items.
-    uint32_t prepare(const std::vector<BatchEntry> &entries, const std::vector<uint32_t> &order) {
-        const uint64_t B = (uint64_t)shape.blocks_per_cta;
+    // uploads the descriptors.  Returns the number of work items (frame slices and symptom CTAs).
+    uint64_t prepare(const std::vector<BatchEntry> &entries, const std::vector<uint32_t> &order) {
+        const uint64_t B = std::max<uint64_t>(1, (uint64_t)shape.blocks_per_cta);  // no shape: no frame launches
         const size_t n = entries.size();
+        const uint64_t ctas = prepare_symptoms(entries, order);
         desc.clear();
         prefix.assign(1, 0);
         det_off.assign(n, 0);
@@ -214,7 +333,7 @@ struct BatchEngine {
             const BatchEntry &e = entries[j];
             const gfs_sampler *s = e.prog;
             const uint64_t nslices = ((e.shots + 127) / 128 + B - 1) / B;
-            if (nslices == 0) {
+            if (nslices == 0 || by_symptoms[j]) {
                 continue;
             }
             det_off[j] = det_total;
@@ -285,7 +404,7 @@ struct BatchEngine {
         size_t k = 0;
         for (size_t q = 0; q < n; q++) {
             const size_t j = order.empty() ? q : order[q];
-            if (entries[j].shots == 0) {
+            if (entries[j].shots == 0 || by_symptoms[j]) {
                 continue;
             }
             gfs::KernelArgs &a = desc[k++];
@@ -308,10 +427,14 @@ struct BatchEngine {
                "descriptor upload");
         }
         items = prefix.back();
-        return items;
+        return items + ctas;
     }
 
     void enqueue_frame() {
+        enqueue_symptoms();
+        if (items == 0) {
+            return;
+        }
         ck(cudaMemsetAsync(d_counter.p, 0, 4, stream), "memset");
         gfs::BatchArgs b{};
         b.circuits = (const gfs::KernelArgs *)d_desc.p;
@@ -369,7 +492,7 @@ struct BatchEngine {
         uint64_t calls = 0;
         for (size_t j = 0; j < entries.size(); j++) {
             const BatchEntry &e = entries[j];
-            if (e.shots == 0) {
+            if (e.shots == 0 || by_symptoms[j]) {
                 continue;
             }
             const uint64_t D = e.prog->prog.num_detectors, O = e.prog->prog.num_observables;
@@ -412,6 +535,9 @@ struct BatchEngine {
     // Reads and clears the kernels' status word (after the stream has drained).  Bits 1 and 2 are errors;
     // bit 4 (a hit list overflowed) is returned as true: the caller redoes the batch with inline noise.
     bool check_status() {
+        if (items == 0) {
+            return false;
+        }
         uint32_t st = 0;
         ck(cudaMemcpy(&st, d_status.p, 4, cudaMemcpyDeviceToHost), "status read");
         if (st) {

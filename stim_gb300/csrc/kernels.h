@@ -138,6 +138,10 @@ struct SymArgs {
 };
 size_t symptom_smem_bytes(uint32_t stride, uint32_t log_blocks);
 cudaError_t launch_symptoms(const SymArgs &args, cudaStream_t stream);
+// Many circuits in one launch: CTA c works for the entry j with prefix[j] <= c < prefix[j + 1] (both in device memory);
+// all entries packed or all unpacked, `smem` that of the largest.
+cudaError_t launch_batch_symptoms(const SymArgs *entries, const uint32_t *prefix, uint32_t n, uint32_t grid, size_t smem,
+                                  bool packed, cudaStream_t stream);
 
 // Transposes [local block][rows] bit-rows (128 shots per entry) of up to three sources, concatenated
 // (src0 rows, then src1, then src2), into shot-major output rows.  `xor_rows` (optional) is a bit vector over the

@@ -481,8 +481,10 @@ struct gfs_sampler {
                ring_pref == -1 && hit_capacity_override == 0 && !(flags & GFS_PREPEND_OBSERVABLES);
     }
 
-    // Enqueues the sampling of `cs` shots from stream block `block0` on into device rows.
-    void run_symptoms(uint64_t cs, uint64_t block0, uint32_t flags, uint8_t *dd, uint64_t ds, uint8_t *od, uint64_t os) {
+    // Kernel arguments for `cs` shots from stream block `block0` on into device rows.  `launch_blocks`: 128-shot blocks
+    // the launch has in all (this sampler's, or a batch's).
+    gfs::SymArgs symptom_args(uint64_t cs, uint64_t block0, uint32_t flags, uint8_t *dd, uint64_t ds, uint8_t *od,
+                              uint64_t os, uint64_t launch_blocks) const {
         gfs::SymArgs a = sym;
         a.block0 = block0;
         a.nshots = cs;
@@ -495,14 +497,19 @@ struct gfs_sampler {
         // Several blocks per CTA while a block has few segments for its 256 lanes and the grid still covers every SM
         // twice (d=3, 30 segments, 2^20 shots: 72 us with one block per CTA, 41 with eight; d=9, 395 segments, 2^18
         // shots: 57 and 48 with two; few blocks: 2^16 shots of d=3 take 12 us with one, 16 with eight).
-        const uint64_t nblk = (cs + 127) / 128;
         uint32_t lb = 0;
-        while (lb < 3 && (nblk >> (lb + 1)) >= 2 * (uint64_t)num_sms && (sym_items << lb) < 512 &&
+        while (lb < 3 && (launch_blocks >> (lb + 1)) >= 2 * (uint64_t)num_sms && (sym_items << lb) < 512 &&
                gfs::symptom_smem_bytes(a.stride, lb + 1) <= (size_t)48 << 10) {
             lb++;
         }
         a.log_blocks = lb;
-        ck(gfs::launch_symptoms(a, stream), "symptom kernel launch");
+        return a;
+    }
+
+    // Enqueues the sampling of `cs` shots from stream block `block0` on into device rows.
+    void run_symptoms(uint64_t cs, uint64_t block0, uint32_t flags, uint8_t *dd, uint64_t ds, uint8_t *od, uint64_t os) {
+        ck(gfs::launch_symptoms(symptom_args(cs, block0, flags, dd, ds, od, os, (cs + 127) / 128), stream),
+           "symptom kernel launch");
         n_frame++;
     }
 

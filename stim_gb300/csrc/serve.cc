@@ -339,7 +339,6 @@ struct gfs_server {
         for (size_t i = 0; i < mem.size(); i++) {
             const Chunk &c = slot.chunks[mem[i]];
             const Request &r = *c.req;
-            progs.push_back(r.prog->s.get());
             gfs_rt::BatchEntry &e = es[i];
             e.prog = r.prog->s.get();
             e.seed = r.seed;
@@ -357,8 +356,14 @@ struct gfs_server {
                 e.obs = r.obs ? base + (r.dets ? c.shots * pad32(r.drow) : 0) : nullptr;
                 e.ostride = pad32(r.orow);
             }
+            e.flags = r.flags;
+            if (!eng.takes_symptoms(e)) {
+                progs.push_back(e.prog);
+            }
         }
-        eng.default_shape(progs);
+        if (!progs.empty()) {  // the frame kernel's shape, for the entries that need it
+            eng.default_shape(progs);
+        }
         if (eng.prepare(es, {}) == 0) {
             ck(cudaEventRecord(eng.ev[2], eng.stream), "event");
             return;

@@ -300,14 +300,15 @@ __device__ __forceinline__ void next_window(const SymArgs &a, const SymStage &st
     }
 }
 
+// Samples CTA `cta`'s blocks from the circuit's start to its end.
 template <bool PACKED>
-__global__ void __launch_bounds__(kThreads) symptom_kernel(const SymArgs a) {
+__device__ __forceinline__ void sample_blocks(const SymArgs &a, uint32_t cta) {
     extern __shared__ __align__(16) uint32_t win[];  // [shot][stride]: detector words, then observable words
     __shared__ uint32_t next;
     __shared__ uint2 queue[kThreads / 32][kHitQueue];
     const uint32_t tid = threadIdx.x, nt = blockDim.x;
     const uint32_t rows = GFS_BLOCK_SHOTS << a.log_blocks;
-    const uint64_t blk0 = (uint64_t)blockIdx.x << a.log_blocks, shot0 = blk0 * GFS_BLOCK_SHOTS;
+    const uint64_t blk0 = (uint64_t)cta << a.log_blocks, shot0 = blk0 * GFS_BLOCK_SHOTS;
     const uint32_t nvalid = a.nshots - shot0 < rows ? (uint32_t)(a.nshots - shot0) : rows;
     const uint32_t nblk = (nvalid + GFS_BLOCK_SHOTS - 1) / GFS_BLOCK_SHOTS;
     const uint32_t dst0 = (uint32_t)(uintptr_t)a.dets + (uint32_t)(shot0 * a.dets_stride);  // modulo 16 is what counts
@@ -363,12 +364,51 @@ __global__ void __launch_bounds__(kThreads) symptom_kernel(const SymArgs a) {
 }
 
 template <bool PACKED>
+__global__ void __launch_bounds__(kThreads) symptom_kernel(const SymArgs a) {
+    sample_blocks<PACKED>(a, blockIdx.x);
+}
+
+template <bool PACKED>
+__global__ void __launch_bounds__(kThreads)
+    batch_symptom_kernel(const SymArgs *entries, const uint32_t *prefix, uint32_t n) {
+    __shared__ SymArgs a;
+    uint32_t lo = 0, hi = n;  // last j with prefix[j] <= blockIdx.x
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) / 2;
+        if (__ldg(prefix + mid) <= blockIdx.x) {
+            lo = mid;
+        } else {
+            hi = mid;
+        }
+    }
+    constexpr uint32_t kWords = sizeof(SymArgs) / 4;
+    static_assert(sizeof(SymArgs) % 4 == 0, "copied by words");
+    if (threadIdx.x < kWords) {
+        reinterpret_cast<uint32_t *>(&a)[threadIdx.x] = __ldg(reinterpret_cast<const uint32_t *>(entries + lo) + threadIdx.x);
+    }
+    __syncthreads();
+    sample_blocks<PACKED>(a, blockIdx.x - __ldg(prefix + lo));
+}
+
+template <bool PACKED>
 cudaError_t launch_packed(const SymArgs &args, uint32_t grid, size_t smem, cudaStream_t stream) {
     cudaError_t e = cudaFuncSetAttribute(symptom_kernel<PACKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) {
         return e;
     }
     symptom_kernel<PACKED><<<grid, kThreads, smem, stream>>>(args);
+    return cudaGetLastError();
+}
+
+template <bool PACKED>
+cudaError_t launch_batch(const SymArgs *entries, const uint32_t *prefix, uint32_t n, uint32_t grid, size_t smem,
+                         cudaStream_t stream) {
+    cudaError_t e =
+        cudaFuncSetAttribute(batch_symptom_kernel<PACKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) {
+        return e;
+    }
+    batch_symptom_kernel<PACKED><<<grid, kThreads, smem, stream>>>(entries, prefix, n);
     return cudaGetLastError();
 }
 
@@ -390,6 +430,15 @@ cudaError_t launch_symptoms(const SymArgs &args, cudaStream_t stream) {
     }
     return args.packed ? launch_packed<true>(args, (uint32_t)grid, smem, stream)
                        : launch_packed<false>(args, (uint32_t)grid, smem, stream);
+}
+
+cudaError_t launch_batch_symptoms(const SymArgs *entries, const uint32_t *prefix, uint32_t n, uint32_t grid, size_t smem,
+                                  bool packed, cudaStream_t stream) {
+    if (n == 0 || grid == 0) {
+        return cudaSuccess;
+    }
+    return packed ? launch_batch<true>(entries, prefix, n, grid, smem, stream)
+                  : launch_batch<false>(entries, prefix, n, grid, smem, stream);
 }
 
 }  // namespace gfs

@@ -89,3 +89,30 @@ def test_a_chosen_frame_kernel_is_used():
         choose(s)
         np.testing.assert_array_equal(s.sample(500, bit_packed=True), want)
         assert s.last_timings()["noise_launches"] == 1
+
+
+def test_batch_mixes_symptom_and_frame_entries():
+    # Small and windowed codes, a circuit whose randomization reaches its outputs, and a sampler with a chosen kernel, in
+    # one batch, replayed; then the server with packed and unpacked requests of the same circuits.
+    t = texts()
+    circuits = [t["surface_code_d3"], t["surface_code_d17"], workloads.random_clifford_circuit(16, 20, 4), t["channels"],
+                t["repetition_code_d51"], t["surface_code_d3"]]
+    shots = [1000, 300, 129, 1, 4096, 0]
+    mk = lambda: [stim_gb300.Circuit(c).compile_detector_sampler(seed=7 + j) for j, c in enumerate(circuits)]
+    for kw in ({"bit_packed": True, "separate_observables": True}, {"append_observables": True}):
+        ones, many = mk(), mk()
+        for s in (ones[4], many[4]):
+            s.set_noise_mode(1)
+        batch = stim_gb300.BatchSampler(many)
+        for _ in range(2):
+            for got, s, n in zip(batch.sample(shots, **kw), ones, shots):
+                want = s.sample(n, **kw)
+                for u, v in zip(got if isinstance(got, tuple) else (got,), want if isinstance(want, tuple) else (want,)):
+                    np.testing.assert_array_equal(u, v)
+        assert batch.last_timings()["graph_builds"] == 1
+    with stim_gb300.Server() as server:
+        reqs = [(c, n, packed, server.submit(c, n, seed=50 + j, bit_packed=packed))
+                for j, (c, n) in enumerate(zip(circuits, shots)) if n for packed in (True, False)]
+        for k, (c, n, packed, r) in enumerate(reqs):
+            want = stim_gb300.Circuit(c).compile_detector_sampler(seed=50 + k // 2).sample(n, bit_packed=packed)
+            np.testing.assert_array_equal(r.result(), want)
