@@ -59,7 +59,7 @@ struct BatchEngine {
     // up to kGroups batched symptom launches, one per (shared-memory class, packed or not): entries whose rows leave
     // room for four CTAs per SM do not share a launch, and so its shared-memory size, with those that do not.
     static constexpr int kGroups = 4;
-    static constexpr size_t kSmallSmem = (size_t)49 << 10;
+    static constexpr size_t kSmallSmem = (size_t)47 << 10;
     struct SymGroup {
         std::vector<gfs::SymArgs> args;
         std::vector<uint32_t> prefix;

@@ -423,16 +423,19 @@ struct gfs_sampler {
         if (!t.ok || D + O == 0 || t.flips_per_block > prog.work + 4 * prog.hits_per_block) {
             return;
         }
-        // All outputs of a block at once while its rows take at most 50 KB (four CTAs per SM), else a window: 128 words a
-        // shot (three CTAs) where the stages fit (d=25: 2.46 ms per 2^20 shots; 64 words, six CTAs, twice the stages:
-        // 3.11; 96: 2.81; 160: 3.00), otherwise 256.
+        // All outputs of a block at once while its rows take at most 50 KB, else a window: 124 words a shot, the most that
+        // leaves three CTAs per SM, where the stages fit (d=25: 2.04 ms per 2^20 shots; 112 words, six stages for five:
+        // 2.12; 76, four CTAs: 2.58; 56, five: 3.25), otherwise 248.
         const uint32_t ow = (uint32_t)((O + 31) / 32);
         gfs::SymptomPlan plan;
         bool planned = false;
         if ((D + O + 31) / 32 <= 96) {
             planned = gfs::plan_symptoms(prog, 0, plan);
         } else {
-            for (uint32_t w = 128; w <= 256 && !planned; w *= 2) {
+            for (uint32_t w : {124u, 248u}) {
+                if (planned) {
+                    break;
+                }
                 planned = gfs::plan_symptoms(prog, w, plan);
             }
         }

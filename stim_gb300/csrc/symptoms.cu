@@ -5,41 +5,60 @@
 // it in time).  Lanes draw the noise contract (gfs_contract.h) segment by segment and XOR each hit's output list
 // into the hit's shot row, so the rows leave as they are: no frames, no hit lists in memory, no transposition.
 //
-// A lane holds one segment and the next one's descriptor (loaded while the first is drawn).  One iteration is one
-// Philox call and up to two hits: gap, choice, gap, choice for a channel that draws its Pauli; a channel that does not
-// uses two of the four draws as gaps.  Hits go to the warp's queue in shared memory and are applied 32 at a time, one
-// per lane, each list loaded one step before it is applied.
+// One iteration of a warp draws 32 segments: one Philox call and two gap draws a lane, up to two hits (gap, choice, gap,
+// choice for a channel that draws its Pauli; a channel that does not uses two of the four draws as gaps).  Segments with
+// draws left wait in a queue of the warp until they fill an iteration, so every iteration but a stage's last few is
+// full.  Hits go to a second queue and are applied 32 at a time, one per lane, each list loaded one step before it is
+// applied.
 //
-// What bounds it: instruction issue.  The output alone would take 0.31 ms at d=25 (2.05 GB per 2^20 shots at 6.7 TB/s),
-// the contract's Philox calls 0.18 ms (580 G calls/s).  d=25, p=1e-3, 2^20 shots: 2.46 ms where noise, frame and
-// transpose kernels took 7.81; d=11, p=5e-3: 0.64 ms (2.22); d=13 colour code, p=1e-2, 200,001 shots: 0.27 ms (0.97).
-// On the way: hits applied as each lane draws them, with the gap table for every draw, 5.2 ms; the float estimate of
-// the gap instead of the table and prefetched descriptors 3.7; the hit queue 2.9; rows written by bulk copies instead
-// of word stores 2.46.
+// What bounds it: instruction issue (d=25: 210 K warp instructions per block, a quarter of them Philox and gap
+// arithmetic that the contract asks for; 0.55 of the issue slots used, the rest fixed latencies and barriers).  The output
+// alone would take 0.31 ms at d=25 (2.05 GB per 2^20 shots at 6.7 TB/s), the contract's Philox calls 0.18 ms (580 G
+// calls/s).  d=25, p=1e-3, 2^20 shots: 2.04 ms where noise, frame and transpose kernels took 7.81; d=11, p=5e-3: 0.58 ms
+// (2.22); d=13 colour code, p=1e-2, 200,001 shots: 0.25 ms (0.97).  On the way at d=25: hits applied as each lane draws
+// them, with the gap table for every draw, 5.2 ms; the float estimate of the gap instead of the table and prefetched
+// descriptors 3.7; the hit queue 2.9; rows written by bulk copies instead of word stores 2.46; queued segments instead of
+// lanes that refill one by one 2.36; hits queued behind the next items' loads 2.19; fewer gap instructions 2.12; items in
+// turn 2.04.
 #include "frame_device.cuh"
 
 namespace gfs {
 
 namespace {
 
-// The position a gap draw leads to (as gfs_hit_after_draw), without the gap table where the float estimate decides.
+// The position a gap draw leads to (as gfs_hit_after_draw; `trials` or more: past the segment), without the gap table where the float estimate decides.
 // e = log2(u / 2^32) / log2(1 - p) has G(u) = floor(e) unless e is close to an integer.  With c = -1 / log2(1 - p), the
 // error of e is below 3.6e-7 e (__log2f outside (0.5, 2): 2 ulp; the factor c and the product: one rounding each) plus
 // 4.3e-7 c (the conversion of u: 2^-24 relative; __log2f inside (0.5, 2): 2^-22; for u >= 2^24 the table's rounding to
-// 2^-32): eps is 1.2 times that, and exact subtractions of integers below 2^22 add nothing.  Smaller u belong to gaps
-// above 8 c: longer than a segment when that exceeds 2,060, else the table decides.
+// 2^-32): eps is 1.2 times that, and exact subtractions of integers below 2^22 add nothing.  Within eps of the integer
+// m, G(u) is m or m - 1, and the table's entry m says which.  Smaller u belong to gaps above 8 c: longer than a segment
+// when that exceeds 2,060, else the table is searched.
 __device__ __forceinline__ int32_t gap_step(uint32_t u, const SymArgs &a, uint32_t chan, float inv_c, int32_t pos,
                                             int32_t trials) {
-    const int32_t room = trials - pos - 1;
-    const float e = fminf(__log2f(__uint2float_rn(u) * 2.3283064365386963e-10f) * -inv_c, 4096.0f);
+    float lg;  // __log2f without its care for subnormal arguments, which u / 2^32 never is
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(lg) : "f"(__uint2float_rn(u) * 2.3283064365386963e-10f));
+    const float e = fminf(lg * -inv_c, 4096.0f);
     const float magic = 12582912.0f;  // 1.5 * 2^23: adding it rounds to the nearest integer, left in the low bits
-    const float m = e + magic, d = e - (m - magic);
-    const int32_t k = __float_as_int(m) - 0x4B400000 - (d < 0.0f ? 1 : 0);  // floor(e)
-    const bool sure = fabsf(d) >= fmaf(e, 4.4e-7f, inv_c * 5.2e-7f) && (u >= (1u << 24) || inv_c > 257.5f);
-    if (!sure) {
-        return gfs_hit_after_draw(u, a.tables + __ldg(&a.chans[chan].table), inv_c, pos, room);
+    const float r = e + magic, d = e - (r - magic);
+    const int32_t m = __float_as_int(r) - 0x4B400000;
+    int32_t k = m - (d < 0.0f ? 1 : 0);  // floor(e)
+    const float eps = fmaf(e, 4.4e-7f, inv_c * 5.2e-7f);
+    const bool large = u >= (1u << 24) || inv_c > 257.5f;
+    if (fabsf(d) < eps || !large) {
+        const int32_t room = trials - pos - 1;
+        const uint32_t *T = a.tables + __ldg(&a.chans[chan].table);
+        if (room <= 0) {
+            return trials;
+        }
+        if (!large || eps >= 0.25f) {
+            const int32_t at = gfs_hit_after_draw(u, T, inv_c, pos, room);
+            return at < 0 ? trials : at;
+        }
+        if (m <= room) {
+            k = m > 0 && u >= __ldg(T + m) ? m - 1 : m;
+        }
     }
-    return k >= room ? -1 : pos + 1 + k;
+    return pos + 1 + k;
 }
 
 // Bits by which a shot's detector columns are shifted in its shared-memory row, so that the row's 16-byte units are the
@@ -68,39 +87,44 @@ __device__ __forceinline__ void flip_outputs(const SymArgs &a, uint32_t *row, ui
         }
         return;
     }
+    auto maybe = [&](uint32_t code) {  // predicated: shorter than leaving a loop lane by lane
+        if (code != kSymNone) {
+            det(code);
+        }
+    };
+    maybe(first);
+    maybe(e.x >> 16);
+    maybe(e.y & 0xFFFFu);
+    maybe(e.y >> 16);
+    if ((e.z & 0xFFFFu) != kSymNone) {
+        maybe(e.z & 0xFFFFu);
+        maybe(e.z >> 16);
+        maybe(e.w & 0xFFFFu);
+    }
     if ((e.w >> 16) != kSymNone) {
         obs(e.w >> 16);
     }
-    const uint32_t code[7] = {first, e.x >> 16, e.y & 0xFFFFu, e.y >> 16, e.z & 0xFFFFu, e.z >> 16, e.w & 0xFFFFu};
-#pragma unroll
-    for (int j = 0; j < 7; j++) {
-        if (code[j] == kSymNone) {
-            break;
-        }
-        det(code[j]);
-    }
 }
 
-constexpr uint32_t kThreads = 256;  // per CTA (d=25: 128 threads 3.57 ms per 2^20 shots, 192 2.82, 256 2.46)
-constexpr uint32_t kHitQueue = 96;  // hits a warp can hold: fewer than 32 left over and two per lane
+constexpr uint32_t kThreads = 256;  // per CTA (d=25: 320 threads 1.98 ms for 2.04, but d=11 0.64 for 0.58)
+constexpr uint32_t kQueue = 64;     // hits, and segments with draws left, a warp can hold: under 32 left over, 32 more
 
-// Draws the stage's items: work index j is item item0 + j / blocks of the CTA's block j % blocks; a warp takes 32
-// indices at a time from the CTA's counter.  q: the warp's hit queue.
+struct WarpQueues {
+    uint2 hits[kQueue];  // output list; shot row << 16 | column of relative code 0
+    uint2 cont[kQueue];  // work index; position of the last hit | iterations done << 16
+};
+
+// Draws the stage's items: work index j is item item0 + j / blocks of the CTA's block j % blocks; the warps take 32
+// consecutive indices in turn (from a shared counter instead: 2.12 ms for 2.04).
 template <bool PACKED>
-__device__ __forceinline__ void draw_stage(const SymArgs &a, const SymStage &st, uint32_t *win, uint32_t *next, uint2 *q,
+__device__ __forceinline__ void draw_stage(const SymArgs &a, const SymStage &st, uint32_t *win, WarpQueues &q,
                                            uint32_t block0, uint32_t nblk, uint32_t dst0) {
     const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
-    const uint32_t lb = a.log_blocks, total = (st.item1 - st.item0) << lb;
+    const uint32_t lb = a.log_blocks, bmask = (1u << lb) - 1u, total = (st.item1 - st.item0) << lb;
     const uint32_t k0 = (uint32_t)a.seed, k1 = (uint32_t)(a.seed >> 32);
     const uint4 *const items = reinterpret_cast<const uint4 *>(a.items + st.item0);
-    uint32_t cur = 0, end = 0;  // this warp's unclaimed indices
-    bool more = true;
-    bool live = false, ready = false;  // a segment is being drawn / the next one's descriptor is loaded
-    uint4 lo = make_uint4(0, 0, 0, 0), hi = lo, nlo = lo, nhi = lo;
-    uint32_t blk = 0, nblk_idx = 0, draw = 0;
-    int32_t pos = -1;
-    uint32_t qn = 0;  // queued hits (warp-uniform)
-    uint4 list = lo;  // the list of a hit taken from the queue, applied when the next one is taken
+    uint32_t hn = 0, cn = 0;  // queued hits and segments (warp-uniform)
+    uint4 list = make_uint4(0, 0, 0, 0);  // the list of a hit taken from the queue, applied when the next one is taken
     uint32_t hit = 0;
     bool pending = false;
     auto apply = [&]() {
@@ -109,45 +133,69 @@ __device__ __forceinline__ void draw_stage(const SymArgs &a, const SymStage &st,
             flip_outputs(a, win + r * a.stride, (hit & 0xFFFFu) + row_shift<PACKED>(a, dst0, r), list);
         }
     };
+    auto push_hits = [&](bool got, uint2 h) {
+        const uint32_t mask = __ballot_sync(0xFFFFFFFFu, got);
+        if (got) {
+            q.hits[hn + __popc(mask & lt)] = h;
+        }
+        hn += __popc(mask);
+        if (hn >= 32) {
+            __syncwarp();
+            apply();
+            hn -= 32;
+            const uint2 x = q.hits[hn + lane];
+            list = __ldg(a.entries + x.x);
+            hit = x.y;
+            pending = true;
+            __syncwarp();
+        }
+    };
+    // The next 32 fresh items, loaded while the present ones are drawn.
+    uint32_t cur = threadIdx.x & ~31u;
+    uint4 flo = make_uint4(0, 0, 0, 0), fhi = flo;
+    auto fetch = [&]() {
+        if (cur + lane < total) {
+            flo = __ldg(items + 2 * ((cur + lane) >> lb));
+            fhi = __ldg(items + 2 * ((cur + lane) >> lb) + 1);
+        }
+    };
+    fetch();
+    bool g0 = false, g1 = false;  // hits of the previous iteration: queued once this one's items are on their way
+    uint2 hit0 = make_uint2(0, 0), hit1 = hit0;
     for (;;) {
-        if (!live && ready) {
-            lo = nlo;
-            hi = nhi;
-            blk = nblk_idx;
-            draw = 0;
-            pos = -1;
-            live = true;
-            ready = false;
+        uint4 lo, hi;
+        uint32_t j, draw = 0;
+        int32_t pos = -1;
+        bool act;
+        if (cn >= 32 || (cur >= total && cn)) {  // segments with draws left, a full warp of them while there are fresh ones
+            const uint32_t take = min(cn, 32u);
+            cn -= take;
+            act = lane < take;
+            const uint2 c = q.cont[cn + min(lane, take - 1)];
+            j = c.x;
+            pos = (int32_t)(c.y & 0xFFFFu);
+            draw = c.y >> 16;
+            lo = __ldg(items + 2 * (j >> lb));
+            hi = __ldg(items + 2 * (j >> lb) + 1);
+            __syncwarp();
+        } else if (cur < total) {
+            j = cur + lane;
+            act = j < total && (j & bmask) < nblk;
+            lo = flo;
+            hi = fhi;
+            cur += kThreads;
+            fetch();
+        } else {
+            break;
         }
-        const uint32_t want = __ballot_sync(0xFFFFFFFFu, !ready);
-        if (want) {
-            if (cur >= end && more) {
-                if (lane == 0) {
-                    cur = atomicAdd(next, 32u);
-                }
-                cur = __shfl_sync(0xFFFFFFFFu, cur, 0);
-                more = cur < total;
-                end = min(cur + 32u, total);
-            }
-            const uint32_t j = cur + __popc(want & lt);
-            if (!ready && j < end) {
-                nblk_idx = j & ((1u << lb) - 1u);
-                if (nblk_idx < nblk) {
-                    nlo = __ldg(items + 2 * (j >> lb));
-                    nhi = __ldg(items + 2 * (j >> lb) + 1);
-                    ready = true;
-                }
-            }
-            cur = min(cur + __popc(want), max(cur, end));
-        }
-        uint2 hit0 = make_uint2(0, 0), hit1 = hit0;
-        bool g0 = false, g1 = false;
-        if (live) {
-            const uint32_t kind = hi.x & 0xFFu, pu = (hi.x >> 8) & 0xFFu;
+        push_hits(g0, hit0);
+        push_hits(g1, hit1);
+        g0 = g1 = false;
+        if (act) {
+            const uint32_t kind = hi.x & 0xFFu, pu = (hi.x >> 8) & 0xFFu, blk = j & bmask;
             const int32_t trials = (int32_t)(hi.x >> 16);
-            const bool choice = pu > 1;
+            const bool choice = pu > 1, odd = (draw & 1u) != 0;
             const gfs_u32x4 r = gfs_philox(k0, k1, block0 + blk, lo.x, lo.y, lo.z | ((choice ? draw : draw >> 1) & 0xFFFFFu));
-            const bool odd = (draw & 1u) != 0;
             const uint32_t u0 = choice || !odd ? r.v[0] : r.v[2];
             const uint32_t u1 = choice ? r.v[2] : odd ? r.v[3] : r.v[1];
             uint32_t v0 = gfs_choice_uniform(r.v[1], pu), v1 = gfs_choice_uniform(r.v[3], pu);
@@ -160,54 +208,31 @@ __device__ __forceinline__ void draw_stage(const SymArgs &a, const SymStage &st,
                 v0 = (pauli_xz(w0 >> 2) | (pauli_xz(w0 & 3) << 2)) - 1;
                 v1 = (pauli_xz(w1 >> 2) | (pauli_xz(w1 & 3) << 2)) - 1;
             }
-            draw++;
             const float inv_c = __uint_as_float(hi.z);
             const uint32_t col = ((blk * GFS_BLOCK_SHOTS) << 16) + hi.y - st.flush0;
-            pos = gap_step(u0, a, hi.w, inv_c, pos, trials);
-            g0 = pos >= 0;
-            if (g0) {
-                const uint32_t p = (uint32_t)pos;
-                hit0 = make_uint2(lo.w + (p >> 7) * pu + v0, ((p & 127u) << 16) + col);
-                if (pos + 1 < trials) {
-                    pos = gap_step(u1, a, hi.w, inv_c, pos, trials);
-                    g1 = pos >= 0;
-                }
-            }
-            if (g1) {
-                const uint32_t p = (uint32_t)pos;
-                hit1 = make_uint2(lo.w + (p >> 7) * pu + v1, ((p & 127u) << 16) + col);
-            }
-            live = g1 && pos + 1 < trials;
+            const int32_t p0 = gap_step(u0, a, hi.w, inv_c, pos, trials);
+            pos = gap_step(u1, a, hi.w, inv_c, p0, trials);
+            g0 = p0 < trials;
+            g1 = pos < trials;
+            hit0 = make_uint2(lo.w + ((uint32_t)p0 >> 7) * pu + v0, (((uint32_t)p0 & 127u) << 16) + col);
+            hit1 = make_uint2(lo.w + ((uint32_t)pos >> 7) * pu + v1, (((uint32_t)pos & 127u) << 16) + col);
         }
-        const uint32_t m0 = __ballot_sync(0xFFFFFFFFu, g0), m1 = __ballot_sync(0xFFFFFFFFu, g1);
-        if (g0) {
-            q[qn + __popc(m0 & lt)] = hit0;
-        }
-        qn += __popc(m0);
+        const uint32_t more = __ballot_sync(0xFFFFFFFFu, g1);
         if (g1) {
-            q[qn + __popc(m1 & lt)] = hit1;
+            q.cont[cn + __popc(more & lt)] = make_uint2(j, (uint32_t)pos | ((draw + 1) << 16));
         }
-        qn += __popc(m1);
+        cn += __popc(more);
         __syncwarp();
-        while (qn >= 32) {
-            apply();
-            qn -= 32;
-            const uint2 h = q[qn + lane];
-            list = __ldg(a.entries + h.x);
-            hit = h.y;
-            pending = true;
-            __syncwarp();
-        }
-        if (!more && cur >= end && !__any_sync(0xFFFFFFFFu, live || ready)) {
-            break;
-        }
     }
+    push_hits(g0, hit0);
+    push_hits(g1, hit1);
+    __syncwarp();
     apply();
-    pending = lane < qn;
+    pending = lane < hn;
     if (pending) {
-        const uint2 h = q[lane];
-        list = __ldg(a.entries + h.x);
-        hit = h.y;
+        const uint2 x = q.hits[lane];
+        list = __ldg(a.entries + x.x);
+        hit = x.y;
     }
     apply();
 }
@@ -281,21 +306,24 @@ __device__ __forceinline__ void write_unpacked(const SymArgs &a, const uint32_t 
     }
 }
 
-// Between stages: the words after the written piece move to the front of their row, the rest is cleared.  All in
-// 16-byte units; a thread owns (row, unit) pairs, the rows of one pass split over the CTA.
+// Between stages: the words after the written piece move to the front of their row, the rest is cleared.  In 16-byte
+// units, eight lanes a row.
 __device__ __forceinline__ void next_window(const SymArgs &a, const SymStage &st, uint32_t *win, uint32_t rows) {
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     const uint32_t n = (st.flush1 - st.flush0) / kSymAlign, keep = st.keep / (kSymAlign / 32);  // units
-    for (uint32_t r = warp; r < rows; r += nwarps) {
+    const uint32_t l = threadIdx.x & 7u;
+    for (uint32_t r = threadIdx.x >> 3; r < rows; r += kThreads >> 3) {  // rows is a multiple of 128
         uint4 *const row = reinterpret_cast<uint4 *>(win + (size_t)r * a.stride);
-        for (uint32_t i0 = 0; i0 < n + keep; i0 += 32) {  // a pass reads ahead of what it and earlier ones write
-            const uint32_t i = i0 + lane;
+        for (uint32_t i0 = 0; i0 < keep; i0 += 8) {  // a pass reads ahead of what it and earlier ones write
+            const uint32_t i = i0 + l;
             const uint4 v = i < keep ? row[n + i] : zero4();
             __syncwarp();
-            if (i < n + keep) {
+            if (i < keep) {
                 row[i] = v;
             }
             __syncwarp();
+        }
+        for (uint32_t i = keep + l; i < n + keep; i += 8) {
+            row[i] = zero4();
         }
     }
 }
@@ -304,8 +332,7 @@ __device__ __forceinline__ void next_window(const SymArgs &a, const SymStage &st
 template <bool PACKED>
 __device__ __forceinline__ void sample_blocks(const SymArgs &a, uint32_t cta) {
     extern __shared__ __align__(16) uint32_t win[];  // [shot][stride]: detector words, then observable words
-    __shared__ uint32_t next;
-    __shared__ uint2 queue[kThreads / 32][kHitQueue];
+    __shared__ WarpQueues queue[kThreads / 32];
     const uint32_t tid = threadIdx.x, nt = blockDim.x;
     const uint32_t rows = GFS_BLOCK_SHOTS << a.log_blocks;
     const uint64_t blk0 = (uint64_t)cta << a.log_blocks, shot0 = blk0 * GFS_BLOCK_SHOTS;
@@ -315,19 +342,13 @@ __device__ __forceinline__ void sample_blocks(const SymArgs &a, uint32_t cta) {
     for (uint32_t i = tid; i < rows * a.stride; i += nt) {
         win[i] = 0;
     }
-    if (tid == 0) {
-        next = 0;
-    }
     __syncthreads();
     for (uint32_t k = 0; k < a.nstages; k++) {
         const SymStage st = a.stages[k];
-        draw_stage<PACKED>(a, st, win, &next, queue[tid >> 5], (uint32_t)(a.block0 + blk0), nblk, dst0);
+        draw_stage<PACKED>(a, st, win, queue[tid >> 5], (uint32_t)(a.block0 + blk0), nblk, dst0);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the rows will be read by bulk copies
         __syncthreads();
         const bool last = k + 1 == a.nstages;
-        if (tid == 0) {
-            next = 0;
-        }
         uint32_t c1 = st.flush1;
         if (last && a.append && a.nobs) {
             for (uint32_t r = tid; r < nvalid; r += nt) {
