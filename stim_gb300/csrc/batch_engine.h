@@ -258,7 +258,8 @@ struct BatchEngine {
             if (e.shots == 0) {
                 continue;
             }
-            gfs::SymArgs a = e.prog->symptom_args(e.shots, e.block0, e.flags, e.dets, e.dstride, e.obs, e.ostride, blocks);
+            gfs::SymArgs a =
+                e.prog->sym.call(e.shots, e.block0, e.flags, e.dets, e.dstride, e.obs, e.ostride, blocks, num_sms);
             a.seed = e.seed;
             const size_t smem = gfs::symptom_smem_bytes(a.stride, a.log_blocks);
             SymGroup &g = groups[(smem > kSmallSmem ? 0 : 2) + (a.packed ? 0 : 1)];

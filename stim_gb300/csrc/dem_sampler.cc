@@ -9,6 +9,7 @@
 // shot-major transposes.  Replayed errors take the converter's path instead: their rows are transposed in
 // and folded into the outputs (each output the XOR of the mechanisms that list it).
 #include "dem.h"
+#include "gfs_contract.h"
 #include "sampler.h"
 
 using namespace gfs_rt;
@@ -24,6 +25,10 @@ struct gfs_dem {
     // Two pipeline slots: chunk k runs on slot k % 2, so its device->host copies overlap chunk k + 1's kernels.
     cudaStream_t streams[2] = {nullptr, nullptr};
     DevBuf det_buf[2], obs_buf[2], err_buf[2], in_buf[2], out_buf[2];
+    // Symptom sampling (symptoms.h) of calls that do not return errors: the mechanisms' symptoms are the output lists.
+    DevBuf d_chans;
+    gfs_rt::SymptomDevice sym;
+    int num_sms = 0;
 
     ~gfs_dem() {
         for (cudaStream_t st : streams) {
@@ -36,6 +41,124 @@ struct gfs_dem {
 };
 
 namespace {
+
+// The segments of every group as symptom items, in order of their lowest detector, with the symptoms of their
+// mechanisms as output lists.
+void init_symptoms(gfs_dem *d) {
+    const gfs::DemModel &m = d->model;
+    const gfs::DemLayout &L = d->lay;
+    const uint64_t D = m.num_detectors, O = m.num_observables;
+    if (D + O == 0 || D >= gfs::kSymObs || O >= gfs::kSymObs) {
+        return;
+    }
+    std::vector<gfs::DevChan> chans;
+    std::vector<gfs::SymItem> items;
+    std::vector<gfs::SymSpan> at;  // detectors of items[k]
+    gfs::SymLists lists;
+    std::vector<std::vector<uint32_t>> seg(GFS_DEM_SEG_UNITS);
+    std::vector<uint32_t> all, part;
+    constexpr uint32_t kSpread = 2048;
+    for (uint32_t g = 0; g < (uint32_t)L.groups.size(); g++) {
+        const gfs::DemGroup &G = L.groups[g];
+        gfs::DevChan ch{};
+        ch.table = G.table;
+        ch.active = G.flags & 1u;
+        ch.inv_c = G.inv_c;
+        chans.push_back(ch);
+        if (G.flags & 2u) {
+            return;  // p >= 1: every trial hits
+        }
+        if (!(G.flags & 1u)) {
+            continue;
+        }
+        for (uint32_t u0 = 0; u0 < G.n; u0 += GFS_DEM_SEG_UNITS) {
+            const uint32_t n = std::min(GFS_DEM_SEG_UNITS, G.n - u0);
+            for (uint32_t u = 0; u < n; u++) {
+                const uint32_t e = L.units[G.first + u0 + u];
+                std::vector<uint32_t> &v = seg[u];
+                v.assign(m.sym.begin() + m.sym_off[e], m.sym.begin() + m.sym_off[e + 1]);
+                for (uint32_t &o : v) {
+                    o = o < D ? o : gfs::kSymObs | (uint32_t)(o - D);
+                }
+                std::sort(v.begin(), v.end());
+                size_t k = 0;
+                for (size_t j = 0; j < v.size();) {  // a symptom listed twice cancels
+                    if (j + 1 < v.size() && v[j] == v[j + 1]) {
+                        j += 2;
+                    } else {
+                        v[k++] = v[j++];
+                    }
+                }
+                v.resize(k);
+            }
+            // Mechanisms of a rare probability can lie anywhere in the model: a segment whose detectors spread over more
+            // than kSpread is drawn once per cluster of them, each time with its lists cut down to that cluster (the
+            // observables with the first).  d=25: 9 of 81,743 segments.
+            all.clear();
+            for (uint32_t u = 0; u < n; u++) {
+                for (uint32_t o : seg[u]) {
+                    if (!(o & gfs::kSymObs)) {
+                        all.push_back(o);
+                    }
+                }
+            }
+            std::sort(all.begin(), all.end());
+            for (size_t k = 0; k < all.size() || k == 0;) {
+                gfs::SymSpan s{0, 1, 0};
+                const size_t k0 = k;
+                while (k < all.size() && all[k] - all[k0] < kSpread) {
+                    k++;
+                }
+                if (k > k0) {
+                    s.lo = all[k0];
+                    s.hi = all[k - 1];
+                }
+                gfs::SymItem it{};
+                it.c1 = u0 / GFS_DEM_SEG_UNITS;
+                it.c2 = g;
+                it.c3 = gfs_c3(GFS_P_DEM, g, 0);
+                it.entry = (uint32_t)(lists.entries.size() / 4);
+                it.kind = gfs::KN_FLIP | 1u << 8 | (n * GFS_BLOCK_SHOTS) << 16;
+                it.base = s.lo <= s.hi ? s.lo : 0;
+                it.inv_c = G.inv_c;
+                it.chan = g;
+                for (uint32_t u = 0; u < n; u++) {
+                    part.clear();
+                    for (uint32_t o : seg[u]) {
+                        if (o & gfs::kSymObs ? k0 == 0 : o >= s.lo && o <= s.hi) {
+                            part.push_back(o);
+                        }
+                    }
+                    lists.add(part.data(), part.size(), it.base);
+                }
+                items.push_back(it);
+                at.push_back(s);
+                if (all.empty()) {
+                    break;
+                }
+            }
+        }
+    }
+    std::vector<uint32_t> order(items.size());
+    for (uint32_t k = 0; k < order.size(); k++) {
+        order[k] = k;
+    }
+    std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return at[a].lo < at[b].lo; });
+    if (chans.empty()) {
+        chans.resize(1);
+    }
+    upload(d->d_chans, chans, d->device, d->stream);
+    d->sym.init(d->device, d->stream, lists, D, O, d->seed, d->d_tables.p, d->d_chans.p,
+                [&](uint32_t words, gfs::SymptomPlan &plan) {
+                    plan = gfs::SymptomPlan();
+                    std::vector<gfs::SymSpan> spans;
+                    for (uint32_t k : order) {
+                        plan.items.push_back(items[k]);
+                        spans.push_back({(uint32_t)plan.items.size(), at[k].lo, at[k].hi});
+                    }
+                    return gfs::plan_stages(spans, D, O, words, plan);
+                });
+}
 
 void create(gfs_dem *d, const char *text, size_t len, uint64_t seed, int device) {
     d->model = gfs::parse_dem(std::string_view(text ? text : "", text ? len : 0));
@@ -65,6 +188,8 @@ void create(gfs_dem *d, const char *text, size_t len, uint64_t seed, int device)
     upload(d->d_out_mech, L.out_mech, device, d->stream);
     std::vector<uint8_t> zeros((d->model.num_detectors + d->model.num_observables + 7) / 8 + 1, 0);
     upload(d->d_expect, zeros, device, d->stream);
+    ck(cudaDeviceGetAttribute(&d->num_sms, cudaDevAttrMultiProcessorCount, device), "attribute");
+    init_symptoms(d);
     ck(cudaStreamSynchronize(d->stream), "upload");
 }
 
@@ -94,13 +219,21 @@ void sample(gfs_dem *d, uint64_t shots, uint32_t flags, uint8_t *dets, uint64_t 
     }
     ck(cudaSetDevice(d->device), "cudaSetDevice");
     const bool want_errs = errs != nullptr && !replay;
+    const bool symptoms = d->sym.ready && !want_errs && !replay;
     const uint64_t per_block = (D + O) * 16 + ((want_errs || replay) ? E * 16 : 0) +
                                128 * (drow + orow + (want_errs ? erow : 0) + (replay ? rrow : 0));
-    const uint64_t cb = std::max<uint64_t>(1, std::min<uint64_t>(512, ((uint64_t)1 << 30) / std::max<uint64_t>(1, per_block)));
+    uint64_t cb = std::max<uint64_t>(1, std::min<uint64_t>(512, ((uint64_t)1 << 30) / std::max<uint64_t>(1, per_block)));
+    if (symptoms) {
+        // 64 MiB of rows per chunk, as the circuit sampler's host pipeline.
+        cb = std::max<uint64_t>(1, ((uint64_t)64 << 20) / std::max<uint64_t>(1, 128 * (drow + orow)));
+        cb = std::min<uint64_t>(cb, (shots + 127) / 128);
+    }
     const uint64_t chunk = cb * 128;
     for (int k = 0; k < 2; k++) {
-        d->det_buf[k].ensure(std::max<uint64_t>(16, cb * D * 16), d->device);
-        d->obs_buf[k].ensure(std::max<uint64_t>(16, cb * O * 16), d->device);
+        if (!symptoms) {
+            d->det_buf[k].ensure(std::max<uint64_t>(16, cb * D * 16), d->device);
+            d->obs_buf[k].ensure(std::max<uint64_t>(16, cb * O * 16), d->device);
+        }
         if (want_errs || replay) {
             d->err_buf[k].ensure(std::max<uint64_t>(16, cb * E * 16), d->device);
         }
@@ -114,6 +247,14 @@ void sample(gfs_dem *d, uint64_t shots, uint32_t flags, uint8_t *dets, uint64_t 
     auto compute = [&](int k, uint64_t done, uint64_t cs, uint64_t block0) {
         cudaStream_t st = d->streams[k];
         const uint64_t nblk = (cs + 127) / 128;
+        uint8_t *dout = (uint8_t *)d->out_buf[k].p, *oout = dout + chunk * drow, *eout = oout + chunk * orow;
+        if (symptoms) {
+            ck(gfs::launch_symptoms(d->sym.call(cs, block0, flags & GFS_BIT_PACKED, dets && drow ? dout : nullptr, drow,
+                                                obs && orow ? oout : nullptr, orow, nblk, d->num_sms),
+                                    st),
+               "symptom kernel launch");
+            return;
+        }
         if (replay) {
             copy2d(d->in_buf[k].p, rrow, replay + done * rstride, rstride, rrow, cs, cudaMemcpyHostToDevice, st,
                    "copy recorded errors");
@@ -150,7 +291,6 @@ void sample(gfs_dem *d, uint64_t shots, uint32_t flags, uint8_t *dets, uint64_t 
             a.errs = want_errs ? (uint4 *)d->err_buf[k].p : nullptr;
             ck(gfs::launch_dem_sample(a, st), "dem kernel launch");
         }
-        uint8_t *dout = (uint8_t *)d->out_buf[k].p, *oout = dout + chunk * drow, *eout = oout + chunk * orow;
         auto tr = [&](const uint4 *src, uint64_t n, uint8_t *out, uint64_t stride) {
             gfs::TransposeArgs t{};
             t.src0 = src;

@@ -139,36 +139,6 @@ class OutputAnalysis {
     }
 
     // ---- output lists of a noise occurrence --------------------------------------------------------------------
-    // Appends the list s[0..n).
-    void add_list(const uint32_t *s, size_t n, uint32_t base) {
-        SymptomTable &t = prog.symptoms;
-        uint32_t h[8] = {kSymNone, kSymNone, kSymNone, kSymNone, kSymNone, kSymNone, kSymNone, kSymNone};
-        size_t nd = 0, no = 0;
-        bool fits = true;
-        for (size_t j = 0; j < n; j++) {
-            const uint32_t id = s[j];
-            if (id & kSymObs) {
-                fits &= no++ == 0 && (id & ~kSymObs) < kSymLong;
-                h[7] = id & ~kSymObs;
-            } else {
-                fits &= nd < 7 && id - base < kSymLong;
-                h[nd < 7 ? nd++ : 6] = id - base;
-            }
-        }
-        if (fits) {
-            const size_t at = t.entries.size();
-            t.entries.resize(at + 4);
-            for (int j = 0; j < 4; j++) {
-                t.entries[at + j] = h[2 * j] | (h[2 * j + 1] << 16);
-            }
-            return;
-        }
-        t.entries.insert(t.entries.end(), {kSymLong, (uint32_t)t.longs.size(), (uint32_t)n, 0u});
-        for (size_t j = 0; j < n; j++) {
-            t.longs.push_back(s[j] & kSymObs ? s[j] : s[j] - base);
-        }
-    }
-
     // out = a XOR b of sorted lists; returns its length.
     static size_t merge(const uint32_t *a, size_t na, const uint32_t *b, size_t nb, uint32_t *out) {
         size_t i = 0, j = 0, n = 0;
@@ -233,8 +203,8 @@ class OutputAnalysis {
                 break;
         }
         l.per_unit = fixed ? 1u : (1u << gens) - 1;
-        l.entry = (uint32_t)(t.entries.size() / 4);
-        if (t.entries.size() / 4 + (size_t)n * l.per_unit > kMaxEntries || t.longs.size() > kMaxLongs) {
+        l.entry = (uint32_t)(t.lists.entries.size() / 4);
+        if (t.lists.entries.size() / 4 + (size_t)n * l.per_unit > kMaxEntries || t.lists.longs.size() > kMaxLongs) {
             drop();
             return;
         }
@@ -269,7 +239,7 @@ class OutputAnalysis {
                 const uint32_t c = b & (b - 1);
                 len[b] = merge(pattern.data() + c * most, len[c], g.data(), g.size(), pattern.data() + b * most);
                 if (!fixed || b == fixed) {
-                    add_list(pattern.data() + b * most, len[b], l.base);
+                    t.lists.add(pattern.data() + b * most, len[b], l.base);
                     flips += len[b];
                 }
             }

@@ -100,6 +100,94 @@ gfs_status guarded(F f) {
     }
 }
 
+// Symptom sampling's tables on the device and the arguments that no call changes (symptoms.h).
+struct SymptomDevice {
+    DevBuf entries, longs, items, stages;
+    gfs::SymArgs args{};
+    size_t nitems = 0;  // segments of a 128-shot block
+    bool ready = false;
+
+    // Plans the stages with plan(window words) and uploads everything; not ready when no window follows the items or the
+    // device has no room (the other kernels need none of it).
+    //
+    // All outputs of a block at once while its rows take at most 50 KB, else a window: 124 words a shot, the most that
+    // leaves three CTAs per SM, where the stages fit (d=25: 2.04 ms per 2^20 shots; 112 words, six stages for five: 2.12;
+    // 76, four CTAs: 2.58; 56, five: 3.25), otherwise 248.
+    template <typename Plan>
+    void init(int device, cudaStream_t stream, const gfs::SymLists &lists, uint64_t D, uint64_t O, uint64_t seed,
+              const void *tables, const void *chans, Plan make) {
+        gfs::SymptomPlan plan;
+        bool planned = false;
+        if ((D + O + 31) / 32 <= 96) {
+            planned = make(0u, plan);
+        } else {
+            for (uint32_t w : {124u, 248u}) {
+                planned = planned || make(w, plan);
+            }
+        }
+        uint32_t stride = (plan.words + (uint32_t)((O + 31) / 32) + 3) / 4 * 4;
+        stride += stride % 32 == 0 ? 4 : 0;  // consecutive shots on different banks
+        if (!planned || gfs::symptom_smem_bytes(stride, 0) > (size_t)200 << 10) {
+            return;
+        }
+        try {
+            upload(entries, lists.entries, device, stream);
+            upload(longs, lists.longs, device, stream);
+            upload(items, plan.items, device, stream);
+            upload(stages, plan.stages, device, stream);
+            ck(cudaStreamSynchronize(stream), "upload sync");
+        } catch (const CudaError &e) {
+            if (e.code != cudaErrorMemoryAllocation) {
+                throw;
+            }
+            cudaGetLastError();
+            for (DevBuf *b : {&entries, &longs, &items, &stages}) {
+                b->release();
+            }
+            return;
+        }
+        args.entries = (const uint4 *)entries.p;
+        args.longs = (const uint32_t *)longs.p;
+        args.items = (const gfs::SymItem *)items.p;
+        args.stages = (const gfs::SymStage *)stages.p;
+        args.nstages = (uint32_t)plan.stages.size();
+        args.tables = (const uint32_t *)tables;
+        args.chans = (const gfs::DevChan *)chans;
+        args.seed = seed;
+        args.ndet = (uint32_t)D;
+        args.nobs = (uint32_t)O;
+        args.words = plan.words;
+        args.stride = stride;
+        nitems = plan.items.size();
+        ready = true;
+    }
+
+    // Kernel arguments for `cs` shots from stream block `block0` on into device rows.  `launch_blocks`: 128-shot blocks
+    // the launch has in all (this call's, or a batch's).
+    gfs::SymArgs call(uint64_t cs, uint64_t block0, uint32_t flags, uint8_t *dd, uint64_t ds, uint8_t *od, uint64_t os,
+                      uint64_t launch_blocks, int num_sms) const {
+        gfs::SymArgs a = args;
+        a.block0 = block0;
+        a.nshots = cs;
+        a.dets = dd;
+        a.dets_stride = ds;
+        a.obs = od;
+        a.obs_stride = os;
+        a.packed = flags & GFS_BIT_PACKED ? 1 : 0;
+        a.append = flags & GFS_APPEND_OBSERVABLES ? 1 : 0;
+        // Several blocks per CTA while a block has few segments for its 256 lanes and the grid still covers every SM
+        // twice (d=3, 30 segments, 2^20 shots: 72 us with one block per CTA, 41 with eight; d=9, 395 segments, 2^18
+        // shots: 57 and 48 with two; few blocks: 2^16 shots of d=3 take 12 us with one, 16 with eight).
+        uint32_t lb = 0;
+        while (lb < 3 && (launch_blocks >> (lb + 1)) >= 2 * (uint64_t)num_sms && (nitems << lb) < 512 &&
+               gfs::symptom_smem_bytes(a.stride, lb + 1) <= (size_t)48 << 10) {
+            lb++;
+        }
+        a.log_blocks = lb;
+        return a;
+    }
+};
+
 }  // namespace gfs_rt
 
 // Internal header: the runtime's own translation units use these helpers unqualified.
@@ -162,10 +250,7 @@ struct gfs_sampler {
     gfs::LaunchShape shape_lean{};
     // Symptom sampling (symptoms.h): detection calls run symptom_kernel when the program has an output table, unless the
     // caller chose a frame kernel, its launch shape or its noise mode.
-    DevBuf d_sym_entries, d_sym_longs, d_sym_items, d_sym_stages;
-    gfs::SymArgs sym{};    // the constant arguments
-    size_t sym_items = 0;  // segments of a 128-shot block
-    bool sym_ready = false;
+    gfs_rt::SymptomDevice sym;
     bool frame_chosen = false;  // a launch shape was set
     int occs_blocks = 0;          // blocks per slice the uploaded occurrence regions were planned for
     uint64_t slice_cap = 0;       // records per slice region
@@ -423,95 +508,20 @@ struct gfs_sampler {
         if (!t.ok || D + O == 0 || t.flips_per_block > prog.work + 4 * prog.hits_per_block) {
             return;
         }
-        // All outputs of a block at once while its rows take at most 50 KB, else a window: 124 words a shot, the most that
-        // leaves three CTAs per SM, where the stages fit (d=25: 2.04 ms per 2^20 shots; 112 words, six stages for five:
-        // 2.12; 76, four CTAs: 2.58; 56, five: 3.25), otherwise 248.
-        const uint32_t ow = (uint32_t)((O + 31) / 32);
-        gfs::SymptomPlan plan;
-        bool planned = false;
-        if ((D + O + 31) / 32 <= 96) {
-            planned = gfs::plan_symptoms(prog, 0, plan);
-        } else {
-            for (uint32_t w : {124u, 248u}) {
-                if (planned) {
-                    break;
-                }
-                planned = gfs::plan_symptoms(prog, w, plan);
-            }
-        }
-        uint32_t stride = (plan.words + ow + 3) / 4 * 4;
-        stride += stride % 32 == 0 ? 4 : 0;  // consecutive shots on different banks
-        if (!planned || gfs::symptom_smem_bytes(stride, 0) > (size_t)200 << 10) {
-            return;
-        }
-        try {
-            upload(d_sym_entries, t.entries, device, stream);
-            upload(d_sym_longs, t.longs, device, stream);
-            upload(d_sym_items, plan.items, device, stream);
-            upload(d_sym_stages, plan.stages, device, stream);
-            ck(cudaStreamSynchronize(stream), "upload sync");
-        } catch (const CudaError &e) {
-            if (e.code != cudaErrorMemoryAllocation) {
-                throw;
-            }
-            cudaGetLastError();  // no room for the lists: the frame kernels need none
-            for (DevBuf *b : {&d_sym_entries, &d_sym_longs, &d_sym_items, &d_sym_stages}) {
-                b->release();
-            }
-            return;
-        }
-        sym.entries = (const uint4 *)d_sym_entries.p;
-        sym.longs = (const uint32_t *)d_sym_longs.p;
-        sym.items = (const gfs::SymItem *)d_sym_items.p;
-        sym.stages = (const gfs::SymStage *)d_sym_stages.p;
-        sym.nstages = (uint32_t)plan.stages.size();
-        sym.tables = (const uint32_t *)d_tables.p;
-        sym.chans = (const gfs::DevChan *)d_chans.p;
-        sym.seed = seed;
-        sym.ndet = (uint32_t)D;
-        sym.nobs = (uint32_t)O;
-        sym.words = plan.words;
-        sym.stride = stride;
-        sym_items = plan.items.size();
-        std::vector<uint32_t>().swap(t.entries);  // on the device now
-        std::vector<uint32_t>().swap(t.longs);
-        sym_ready = true;
+        sym.init(device, stream, t.lists, D, O, seed, d_tables.p, d_chans.p,
+                 [&](uint32_t words, gfs::SymptomPlan &plan) { return gfs::plan_symptoms(prog, words, plan); });
+        t.lists = gfs::SymLists();  // on the device now
     }
 
     // Whether a detection call with these layout flags runs symptom_kernel.
     bool symptoms_active(uint32_t flags) const {
-        return sym_ready && mode == GFS_MODE_DETECTIONS && !frame_chosen && hits_pref == -1 && lean_pref == -1 &&
+        return sym.ready && mode == GFS_MODE_DETECTIONS && !frame_chosen && hits_pref == -1 && lean_pref == -1 &&
                ring_pref == -1 && hit_capacity_override == 0 && !(flags & GFS_PREPEND_OBSERVABLES);
-    }
-
-    // Kernel arguments for `cs` shots from stream block `block0` on into device rows.  `launch_blocks`: 128-shot blocks
-    // the launch has in all (this sampler's, or a batch's).
-    gfs::SymArgs symptom_args(uint64_t cs, uint64_t block0, uint32_t flags, uint8_t *dd, uint64_t ds, uint8_t *od,
-                              uint64_t os, uint64_t launch_blocks) const {
-        gfs::SymArgs a = sym;
-        a.block0 = block0;
-        a.nshots = cs;
-        a.dets = dd;
-        a.dets_stride = ds;
-        a.obs = od;
-        a.obs_stride = os;
-        a.packed = flags & GFS_BIT_PACKED ? 1 : 0;
-        a.append = flags & GFS_APPEND_OBSERVABLES ? 1 : 0;
-        // Several blocks per CTA while a block has few segments for its 256 lanes and the grid still covers every SM
-        // twice (d=3, 30 segments, 2^20 shots: 72 us with one block per CTA, 41 with eight; d=9, 395 segments, 2^18
-        // shots: 57 and 48 with two; few blocks: 2^16 shots of d=3 take 12 us with one, 16 with eight).
-        uint32_t lb = 0;
-        while (lb < 3 && (launch_blocks >> (lb + 1)) >= 2 * (uint64_t)num_sms && (sym_items << lb) < 512 &&
-               gfs::symptom_smem_bytes(a.stride, lb + 1) <= (size_t)48 << 10) {
-            lb++;
-        }
-        a.log_blocks = lb;
-        return a;
     }
 
     // Enqueues the sampling of `cs` shots from stream block `block0` on into device rows.
     void run_symptoms(uint64_t cs, uint64_t block0, uint32_t flags, uint8_t *dd, uint64_t ds, uint8_t *od, uint64_t os) {
-        ck(gfs::launch_symptoms(symptom_args(cs, block0, flags, dd, ds, od, os, (cs + 127) / 128), stream),
+        ck(gfs::launch_symptoms(sym.call(cs, block0, flags, dd, ds, od, os, (cs + 127) / 128, num_sms), stream),
            "symptom kernel launch");
         n_frame++;
     }

@@ -43,26 +43,69 @@ struct alignas(16) SymStage {
 // What the backward pass found for one occurrence, before stages are planned.
 struct SymList {
     uint32_t entry = 0, per_unit = 0, kind = 0, n = 0, chan = 0;
-    uint32_t base = 0;      // detector of relative code 0
+    uint32_t base = 0;        // detector of relative code 0
     uint32_t lo = 1, hi = 0;  // detectors its lists touch (lo > hi: none)
     double mean = 0;          // mean list length
+};
+
+// Output lists in the form the kernel reads.
+struct SymLists {
+    std::vector<uint32_t> entries;  // four words per list
+    std::vector<uint32_t> longs;
+
+    // Appends the sorted list s[0..n) of detectors (at least `base`) and kSymObs | observables.
+    void add(const uint32_t *s, size_t n, uint32_t base) {
+        uint32_t h[8] = {kSymNone, kSymNone, kSymNone, kSymNone, kSymNone, kSymNone, kSymNone, kSymNone};
+        size_t nd = 0, no = 0;
+        bool fits = true;
+        for (size_t j = 0; j < n; j++) {
+            const uint32_t id = s[j];
+            if (id & kSymObs) {
+                fits &= no++ == 0 && (id & ~kSymObs) < kSymLong;
+                h[7] = id & ~kSymObs;
+            } else {
+                fits &= nd < 7 && id - base < kSymLong;
+                h[nd < 7 ? nd++ : 6] = id - base;
+            }
+        }
+        if (fits) {
+            const size_t at = entries.size();
+            entries.resize(at + 4);
+            for (int j = 0; j < 4; j++) {
+                entries[at + j] = h[2 * j] | (h[2 * j + 1] << 16);
+            }
+            return;
+        }
+        entries.insert(entries.end(), {kSymLong, (uint32_t)longs.size(), (uint32_t)n, 0u});
+        for (size_t j = 0; j < n; j++) {
+            longs.push_back(s[j] & kSymObs ? s[j] : s[j] - base);
+        }
+    }
 };
 
 // Output lists of a program's noise occurrences (ok = false: the program needs a frame kernel).
 struct SymptomTable {
     bool ok = false;
     std::vector<SymList> occ;
-    std::vector<uint32_t> entries;  // four words per list
-    std::vector<uint32_t> longs;
+    SymLists lists;
     double flips_per_block = 0;  // expected output flips per 128-shot block
 };
 
-// Stages of a program for a window of `window_words` 32-detector words per shot (0: all outputs at once).
+// Stages for a window of `window_words` 32-detector words per shot (0: all outputs at once).
 struct SymptomPlan {
     std::vector<SymItem> items;
     std::vector<SymStage> stages;
     uint32_t words = 0;  // detector words per shot row held in shared memory (kSymAlign spare for the row's alignment)
 };
+
+// Consecutive items [.., end) whose lists touch detectors lo..hi (lo > hi: none), kept in one stage.
+struct SymSpan {
+    uint32_t end, lo, hi;
+};
+
+// Stages over plan.items, given as spans in order; false when the window cannot follow them.
+bool plan_stages(const std::vector<SymSpan> &spans, uint64_t num_detectors, uint64_t num_observables,
+                 uint32_t window_words, SymptomPlan &plan);
 bool plan_symptoms(const Program &prog, uint32_t window_words, SymptomPlan &plan);
 
 }  // namespace gfs

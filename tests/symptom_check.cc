@@ -4,7 +4,8 @@
 // stage by stage in shifted row windows as symptom_kernel holds them, and every detector written must agree, for
 // several window sizes.
 //
-// Usage: symptom_check CIRCUIT_FILE  ->  prints "ok <occurrences> <lists> <stages>..." (stages per window, 0: does not
+// Usage: symptom_check spans SEED checks stages over random spans alone;
+// symptom_check CIRCUIT_FILE  ->  prints "ok <occurrences> <lists> <stages>..." (stages per window, 0: does not
 // fit), "no-table" when the program keeps its frames, or a mismatch, exit 1.
 // Test infrastructure (tests/test_symptoms.py compiles it); the product never uses it.
 #include <cstdio>
@@ -201,11 +202,11 @@ bool check_plan(const Program &p, const SymptomPlan &plan, const Forward &want) 
             for (const Hit &h : hits_of(occ, l.n, l.per_unit)) {
                 const SymItem &it = plan.items[item + h.unit / GFS_SEG_UNITS];
                 const uint32_t list = it.entry + (h.unit % GFS_SEG_UNITS) * l.per_unit + h.pattern;
-                const uint32_t *e = t.entries.data() + 4 * (size_t)list;
+                const uint32_t *e = t.lists.entries.data() + 4 * (size_t)list;
                 std::vector<uint32_t> codes;  // detectors (absolute) and kSymObs | observable
                 if ((e[0] & 0xFFFFu) == kSymLong) {
                     for (uint32_t j = 0; j < e[2]; j++) {
-                        const uint32_t c = t.longs[e[1] + j];
+                        const uint32_t c = t.lists.longs[e[1] + j];
                         codes.push_back(c & kSymObs ? c : it.base + c);
                     }
                 } else {
@@ -237,6 +238,10 @@ bool check_plan(const Program &p, const SymptomPlan &plan, const Forward &want) 
             return false;
         }
         const uint32_t n = (st.flush1 - st.flush0) / 32;
+        if (!last && (st.flush1 - st.flush0) / 32 + st.keep > plan.words) {
+            std::printf("stage %zu writes past its window\n", s);
+            return false;
+        }
         for (uint32_t lane = 0; lane < 32; lane++) {
             const uint32_t shift = 8 * (lane % 16);
             // Detectors complete in the written words (the last ones of a stage stay behind the shift).
@@ -272,9 +277,74 @@ bool check_plan(const Program &p, const SymptomPlan &plan, const Forward &want) 
     return true;
 }
 
+// Stages over random spans (sorted, some far apart or empty) for random windows: every stage stays inside its window,
+// which its spans fit, and nothing is written before the spans that touch it are done.
+bool check_spans(uint32_t seed) {
+    std::srand(seed);
+    auto upto = [](uint32_t n) { return (uint32_t)std::rand() % n; };
+    for (int trial = 0; trial < 400; trial++) {
+        const uint32_t gap = 1u << upto(14), len = 1u << upto(12), obs = upto(3) * 40;
+        std::vector<SymSpan> spans;
+        SymptomPlan plan;
+        uint64_t lo = upto(1 + 40 * upto(2) * gap), D = 1 + upto(300);
+        for (uint32_t k = 0, n = upto(300); k < n; k++) {
+            for (uint32_t j = 0, n = 1 + upto(4); j < n; j++) {
+                plan.items.push_back(SymItem{});
+            }
+            const bool empty = upto(9) == 0;
+            const uint32_t l = empty ? 1 : (uint32_t)lo, h = empty ? 0 : (uint32_t)lo + upto(len);
+            spans.push_back({(uint32_t)plan.items.size(), l, h});
+            D = std::max<uint64_t>(D, (uint64_t)h + 1 + upto(2) * upto(9000));
+            lo += upto(gap + 1);
+        }
+        const uint32_t words = 4 * upto(64);
+        if (!plan_stages(spans, D, obs, words, plan)) {
+            if (words == 0 || (words * 32 > len + 256 && words * 32 > 128 + obs + 128)) {
+                std::printf("a window of %u words should follow spans of %u\n", words, len);
+                return false;
+            }
+            continue;
+        }
+        uint32_t at = 0, item = 0;
+        size_t span = 0;
+        for (size_t s = 0; s < plan.stages.size(); s++) {
+            const SymStage &st = plan.stages[s];
+            const bool last = s + 1 == plan.stages.size();
+            const uint64_t end = st.flush0 + (words ? 32ull * words : 32ull * plan.words - kSymAlign);
+            bool good = st.flush0 == at && st.item0 == item && st.flush1 >= at && st.item1 >= item &&
+                        (last ? st.flush1 == D && D + obs <= end : st.flush1 % kSymAlign == 0 && st.flush1 > at) &&
+                        (last || ((st.flush1 - st.flush0) / 32 + st.keep <= plan.words && st.keep >= 4 && st.keep % 4 == 0));
+            for (; span < spans.size() && spans[span].end <= st.item1; span++) {
+                good = good && (spans[span].lo > spans[span].hi || (spans[span].lo >= st.flush0 && spans[span].hi < end));
+                good = good && (last || spans[span].lo > spans[span].hi ||
+                                spans[span].hi < st.flush1 + 32ull * st.keep - kSymAlign || spans[span].hi < st.flush1);
+            }
+            for (uint32_t k = st.item0; k < st.item1; k++) {
+                good = good && plan.items[k].base <= end;
+            }
+            if (!good) {
+                std::printf("stage %zu of %zu of trial %d (seed %u, %u words) is wrong: items %u-%u, detectors %u-%u of %llu, "
+                            "keep %u of %u\n", s, plan.stages.size(), trial, seed, words, st.item0, st.item1, st.flush0,
+                            st.flush1, (unsigned long long)D, st.keep, plan.words);
+                return false;
+            }
+            at = st.flush1;
+            item = st.item1;
+        }
+    }
+    return true;
+}
+
 }  // namespace
 
 int main(int argc, char **argv) {
+    if (argc == 3 && std::string(argv[1]) == "spans") {
+        if (!check_spans((uint32_t)std::atoi(argv[2]))) {
+            return 1;
+        }
+        std::printf("ok\n");
+        return 0;
+    }
     if (argc != 2) {
         std::fprintf(stderr, "usage: symptom_check CIRCUIT_FILE\n");
         return 2;
@@ -306,6 +376,6 @@ int main(int argc, char **argv) {
         }
         stages += " " + std::to_string(fits ? plan.stages.size() : 0);
     }
-    std::printf("ok %zu %zu%s\n", p.symptoms.occ.size(), p.symptoms.entries.size() / 4, stages.c_str());
+    std::printf("ok %zu %zu%s\n", p.symptoms.occ.size(), p.symptoms.lists.entries.size() / 4, stages.c_str());
     return 0;
 }

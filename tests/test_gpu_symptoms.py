@@ -8,6 +8,7 @@ import pytest
 import stim_gb300
 from oracle.oracle import OracleCircuit
 from stim_gb300 import _native, workloads
+from test_dem_oracle import load_dem
 from test_symptoms import HAND
 
 pytestmark = pytest.mark.gpu
@@ -116,3 +117,28 @@ def test_batch_mixes_symptom_and_frame_entries():
         for k, (c, n, packed, r) in enumerate(reqs):
             want = stim_gb300.Circuit(c).compile_detector_sampler(seed=50 + k // 2).sample(n, bit_packed=packed)
             np.testing.assert_array_equal(r.result(), want)
+
+
+def dem_text(name):
+    if name == "surface_rz_d25":
+        return workloads.dem_d25_text()
+    if name == "hand":  # repeated symptoms, a long list, observables alone, loops, p = 0
+        return ("error(0.1) D0 D0 D1\nerror(0.2) L0 L40\nerror(0) D3\nrepeat 9 {\n error(0.01) D0 ^ D1\n"
+                " error(0.3) D0 D1 D2 D3 D4 D5 D6 D7 D8 L1\n shift_detectors 3\n}\nerror(0.001) D40\n")
+    if name == "far_apart":  # one probability whose mechanisms lie thousands of detectors apart, more than a window
+        return "".join(f"error(0.02) D{3000 * k} D{3000 * k + 7} L{k % 3}\nerror(0.0{1 + k % 3}) D{3000 * k + 5}\n"
+                       for k in range(20)) + "error(0.02) L2\nerror(0.3) D0\n"
+    return str(load_dem(name)["model"])
+
+
+@pytest.mark.parametrize("name", ["surface_rz_d25", "hand", "far_apart", "rep_d9_r9", "color_d5_r5"])
+def test_error_models(name):
+    # Without errors returned the model is sampled by its symptoms; with them, mechanism by mechanism.
+    text = dem_text(name)
+    a, b = (stim_gb300.DetectorErrorModel(text).compile_sampler(seed=21) for _ in range(2))
+    for shots in (1, 130, 1000) if name == "surface_rz_d25" else (1, 128, 70001):
+        for packed in (True, False):
+            d, o, _ = a.sample(shots, bit_packed=packed)
+            wd, wo, _ = b.sample(shots, bit_packed=packed, return_errors=True)
+            np.testing.assert_array_equal(d, wd)
+            np.testing.assert_array_equal(o, wo)

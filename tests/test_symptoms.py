@@ -32,6 +32,8 @@ HAND = {
                 + "".join(f"OBSERVABLE_INCLUDE({k}) rec[-{1 + k % 4}]\n" for k in range(40)),
     "pauli_observable": "RX 0\nR 1\nZ_ERROR(0.2) 0\nX_ERROR(0.3) 1\nOBSERVABLE_INCLUDE(0) X0\nOBSERVABLE_INCLUDE(2) Z1\n",
     "far_apart": "R 0\n" + "R 1\nX_ERROR(0.01) 0\nM 1\nDETECTOR rec[-1]\n" * 400 + "M 0\nDETECTOR rec[-1]\n",
+    "quiet_stretch": "R 0 1\nX_ERROR(0.1) 0\nM 0\nDETECTOR rec[-1]\nREPEAT 9000 {\n M 1\n DETECTOR rec[-1]\n}\n"
+                     "X_ERROR(0.1) 1\nM 1\nDETECTOR rec[-1]\n",
     "noiseless": "R 0\nM 0\nDETECTOR rec[-1]\n",
 }
 
@@ -69,6 +71,12 @@ def test_hand_circuits(checker, name, tmp_path):
     path = tmp_path / "c.stim"
     path.write_text(HAND[name])
     assert run(checker, str(path))[0] == "ok"
+
+
+@pytest.mark.parametrize("seed", range(5))
+def test_stages_over_random_spans(checker, seed):
+    out = subprocess.run([checker, "spans", str(seed)], capture_output=True, text=True)
+    assert out.returncode == 0, out.stdout + out.stderr
 
 
 @pytest.mark.parametrize("path", sorted(glob.glob(os.path.join(HERE, "golden", "*.npz"))), ids=os.path.basename)
