@@ -7,7 +7,7 @@
 // on the host, the noise fused into a gate split into its own hit phase), which the CTA keeps in shared
 // memory.  Each thread works one phase ahead: before the barrier that ends phase k it has already done the
 // loop bookkeeping that leads to phase k+1, read k+1's descriptor and loaded the unit-list entries of its
-// first kLeanJ items of k+1 into registers.
+// first kLeanJ items of k+1 into registers (kLeanShort: two phases ahead).
 //
 // Hit records reach shared memory ahead of time: each hit phase copies (cp.async) the record that this thread
 // applies first two noise occurrences later into a per-thread staging slot, so that when a hit phase starts its
@@ -24,7 +24,13 @@ namespace gfs {
 
 namespace {
 
-constexpr int kLeanJ = 6;  // unit-list entries per thread prefetched one phase ahead
+// Unit-list entries per thread loaded ahead.  kLeanJ: one phase ahead, for circuits whose phases keep every thread busy.
+// kLeanShort: circuits whose phases have at most about two items a thread.  There a phase is one chain of latencies,
+// whatever the launch shape (64-qubit Clifford layers: 1,250 cycles, 800 of them work, most of it the wait for the
+// unit-list entry loaded just before, 400 to resolve the next phase, 17 at the barrier), so entries are loaded two phases
+// ahead and a thread runs through two of them instead of six: 800 cycles a phase, 453 -> 324 us per 2^17 shots; d=9
+// measurements 124 -> 103 us per 2^16.
+constexpr int kLeanJ = 6, kLeanShort = 2;
 
 struct LeanLoops {
     int depth;
@@ -83,43 +89,43 @@ __device__ __forceinline__ uint32_t lean_next(const LeanPhase *ph, const uint64_
     }
 }
 
-// Unit-list entries of this thread's first kLeanJ items of phase `d` (items i = tid + j * nt, item = unit * B
+// Unit-list entries of this thread's first J items of phase `d` (items i = tid + j * nt, item = unit * B
 // + block).  16-bit lists for one-qubit gates, measurements and resets, 32-bit words for pairs and detectors.
-template <int B>
+template <int B, int J>
 __device__ __forceinline__ void lean_prefetch(const LeanPhase &d, const uint32_t *pool, uint32_t tid, uint32_t nt,
-                                              uint32_t (&E)[kLeanJ]) {
+                                              uint32_t (&E)[J]) {
     const uint32_t kind = d.op & 0xFFu;
     const uint32_t items = d.n * B;
     if (kind == LK_1Q || kind == LK_MEAS || kind == LK_RESET) {
         const unsigned short *l = reinterpret_cast<const unsigned short *>(pool + d.a);
 #pragma unroll
-        for (int j = 0; j < kLeanJ; j++) {
+        for (int j = 0; j < J; j++) {
             const uint32_t i = tid + (uint32_t)j * nt;
             E[j] = i < items ? (uint32_t)__ldg(l + i / B) : 0u;
         }
     } else if (kind == LK_CX || kind == LK_CZ || kind == LK_2Q || kind == LK_DETS2) {
         const uint32_t *l = pool + d.a;
 #pragma unroll
-        for (int j = 0; j < kLeanJ; j++) {
+        for (int j = 0; j < J; j++) {
             const uint32_t i = tid + (uint32_t)j * nt;
             E[j] = i < items ? __ldg(l + i / B) : 0u;
         }
     }
 }
 
-// f(unit, block, entry) over this thread's items: the first kLeanJ from the prefetched entries, the rest (units
-// beyond kLeanJ * nt items) loaded here.
-template <int B, bool HALF, typename F>
-__device__ __forceinline__ void lean_items(const uint32_t (&E)[kLeanJ], const uint32_t *list, uint32_t items,
+// f(unit, block, entry) over this thread's items: the first J from the prefetched entries, the rest (units
+// beyond J * nt items) loaded here.
+template <int B, bool HALF, int J, typename F>
+__device__ __forceinline__ void lean_items(const uint32_t (&E)[J], const uint32_t *list, uint32_t items,
                                            uint32_t tid, uint32_t nt, F f) {
 #pragma unroll
-    for (int j = 0; j < kLeanJ; j++) {
+    for (int j = 0; j < J; j++) {
         const uint32_t i = tid + (uint32_t)j * nt;
         if (i < items) {
             f(i / B, i % B, E[j]);
         }
     }
-    for (uint32_t i = tid + (uint32_t)kLeanJ * nt; i < items; i += nt) {
+    for (uint32_t i = tid + (uint32_t)J * nt; i < items; i += nt) {
         const uint32_t w = HALF ? (uint32_t)__ldg(reinterpret_cast<const unsigned short *>(list) + i / B)
                                 : __ldg(list + i / B);
         f(i / B, i % B, w);
@@ -127,8 +133,8 @@ __device__ __forceinline__ void lean_items(const uint32_t (&E)[kLeanJ], const ui
 }
 
 // CX / CZ over this thread's pairs, two pairs' loads in flight together.
-template <int B>
-__device__ __forceinline__ void lean_cx_cz(const uint32_t (&E)[kLeanJ], const uint32_t *list, bool cz, uint32_t items,
+template <int B, int J>
+__device__ __forceinline__ void lean_cx_cz(const uint32_t (&E)[J], const uint32_t *list, bool cz, uint32_t items,
                                            uint4 *X, uint4 *Z, uint32_t tid, uint32_t nt) {
     auto pair2 = [&](uint32_t ia, uint32_t wa, uint32_t ib, uint32_t wb) {
         const bool two = ib < items;
@@ -159,13 +165,13 @@ __device__ __forceinline__ void lean_cx_cz(const uint32_t (&E)[kLeanJ], const ui
         }
     };
 #pragma unroll
-    for (int j = 0; j < kLeanJ; j += 2) {
+    for (int j = 0; j < J; j += 2) {
         const uint32_t ia = tid + (uint32_t)j * nt;
         if (ia < items) {
             pair2(ia, E[j], ia + nt, E[j + 1]);
         }
     }
-    for (uint32_t ia = tid + (uint32_t)kLeanJ * nt; ia < items; ia += 2 * nt) {
+    for (uint32_t ia = tid + (uint32_t)J * nt; ia < items; ia += 2 * nt) {
         const uint32_t ib = ia + nt;
         pair2(ia, __ldg(list + ia / B), ib, ib < items ? __ldg(list + ib / B) : 0u);
     }
@@ -243,8 +249,18 @@ __device__ __forceinline__ LeanState lean_state(const KernelArgs &p, uint4 *sm) 
     return st;
 }
 
-template <int B>
+// A phase resolved ahead of its turn: its descriptor, index, instance base and this thread's unit-list entries.
+template <int J>
+struct LeanAhead {
+    LeanPhase d;
+    uint32_t pc;
+    uint64_t inst_base;
+    uint32_t E[J];
+};
+
+template <int B, int J>
 __device__ __forceinline__ void lean_slice(const KernelArgs &p, const LeanState &st, uint32_t slice) {
+    constexpr bool kTwoAhead = J == kLeanShort;
     const uint32_t nr = p.nrows, L = p.ring, NO = p.nobs;
     uint4 *const X = st.X, *const Z = st.Z, *const R = st.R, *const O = st.O;
     const LeanPhase *const ph = st.ph;
@@ -276,15 +292,31 @@ __device__ __forceinline__ void lean_slice(const KernelArgs &p, const LeanState 
     lean_stage(st.stg + nt, hb, st.oc[1], tid);
 
     LeanLoops lp{};
-    uint64_t inst_base = 0;
+    uint64_t inst_base = 0;  // of the phase being resolved
     uint32_t rec = 0, occ = 0;
     uint64_t det_base = 0, meas_base = 0;
-    uint32_t pc = lean_next(ph, p.lean_inst, 0, lp, inst_base);
-    LeanPhase d = ph[pc];
-    uint32_t E[kLeanJ];
-    lean_prefetch<B>(d, pool, tid, nt, E);
+    // Resolves the phase at or after `at` into `a`; the end of the list stays where it is.
+    auto resolve = [&](uint32_t at, LeanAhead<J> &a) {
+        a.pc = at;
+        a.d = ph[at];
+        if ((a.d.op & 0xFFu) == LK_LOOP_BEGIN || (a.d.op & 0xFFu) == LK_LOOP_END) {
+            a.pc = lean_next(ph, p.lean_inst, at, lp, inst_base);
+            a.d = ph[a.pc];
+        }
+        a.inst_base = inst_base;
+        lean_prefetch<B>(a.d, pool, tid, nt, a.E);
+    };
+    LeanAhead<J> cur, ahead;
+    resolve(0, cur);
+    if (kTwoAhead) {
+        resolve((cur.d.op & 0xFFu) == LK_END ? cur.pc : cur.pc + 1, ahead);
+    }
 
     for (;;) {
+        const LeanPhase d = cur.d;
+        const uint32_t pc = cur.pc;
+        const uint64_t inst_base = cur.inst_base;
+        uint32_t(&E)[J] = cur.E;
         const uint32_t kind = d.op & 0xFFu, sub = (d.op >> 8) & 0xFFu;
         const uint32_t n = d.n, items = n * B;
         if (kind == LK_END) {
@@ -355,9 +387,9 @@ __device__ __forceinline__ void lean_slice(const KernelArgs &p, const LeanState 
                 uint4 *const out = p.det_out;
                 const uint64_t ndet = p.ndet;
                 // All of this thread's prefetched detectors' records are loaded before any result is stored.
-                uint4 acc[kLeanJ];
+                uint4 acc[J];
 #pragma unroll
-                for (int j = 0; j < kLeanJ; j++) {
+                for (int j = 0; j < J; j++) {
                     const uint32_t i = tid + (uint32_t)j * nt;
                     const uint32_t blk = i % B, k1 = E[j] & 0xFFFFu, k2 = E[j] >> 16;
                     acc[j] = zero4();
@@ -369,13 +401,13 @@ __device__ __forceinline__ void lean_slice(const KernelArgs &p, const LeanState 
                     }
                 }
 #pragma unroll
-                for (int j = 0; j < kLeanJ; j++) {
+                for (int j = 0; j < J; j++) {
                     const uint32_t i = tid + (uint32_t)j * nt;
                     if (i < items) {
                         out[(lb0 + i % B) * ndet + det_base + i / B] = acc[j];
                     }
                 }
-                for (uint32_t i = tid + (uint32_t)kLeanJ * nt; i < items; i += nt) {
+                for (uint32_t i = tid + (uint32_t)J * nt; i < items; i += nt) {
                     const uint32_t w = __ldg(list + i / B), blk = i % B, k1 = w & 0xFFFFu, k2 = w >> 16;
                     uint4 a = zero4();
                     if (k1) {
@@ -449,15 +481,14 @@ __device__ __forceinline__ void lean_slice(const KernelArgs &p, const LeanState 
                 }
                 break;
         }
-        // Phase k+1 is resolved and its entries are on their way before the barrier that ends phase k.
+        // The next phase is resolved and its entries are on their way before the barrier that ends this one.
         const bool bar = (d.op & kLeanNoBarrier) == 0;
-        pc++;
-        d = ph[pc];
-        if ((d.op & 0xFFu) == LK_LOOP_BEGIN || (d.op & 0xFFu) == LK_LOOP_END) {
-            pc = lean_next(ph, p.lean_inst, pc, lp, inst_base);
-            d = ph[pc];
+        if (kTwoAhead) {
+            cur = ahead;
+            resolve((cur.d.op & 0xFFu) == LK_END ? cur.pc : cur.pc + 1, ahead);
+        } else {
+            resolve(pc + 1, cur);
         }
-        lean_prefetch<B>(d, pool, tid, nt, E);
         if (bar) {
             __syncthreads();
         }
@@ -471,12 +502,12 @@ __device__ __forceinline__ void lean_slice(const KernelArgs &p, const LeanState 
     __syncthreads();
 }
 
-template <int B>
+template <int B, int J>
 __global__ void __maxnreg__(96) frame_kernel_lean(const KernelArgs p) {
     extern __shared__ uint4 sm[];
     const LeanState st = lean_state<B>(p, sm);
     for (uint32_t slice = blockIdx.x; slice < p.nslices; slice += gridDim.x) {
-        lean_slice<B>(p, st, slice);
+        lean_slice<B, J>(p, st, slice);
     }
 }
 
@@ -518,7 +549,7 @@ __global__ void __maxnreg__(96) batch_frame_kernel_lean(const BatchArgs b) {
             st = lean_state<B>(cur, sm);
             have = j;
         }
-        lean_slice<B>(cur, st, item - b.slice_prefix[j]);
+        lean_slice<B, kLeanJ>(cur, st, item - b.slice_prefix[j]);
     }
 }
 
@@ -547,23 +578,35 @@ cudaError_t lean_batch_occ_b(const LaunchShape &s, int *out) {
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, batch_frame_kernel_lean<B>, s.threads, s.smem);
 }
 
-template <int B>
-cudaError_t lean_launch_b(const KernelArgs &args, const LaunchShape &s, cudaStream_t stream) {
-    cudaError_t e = cudaFuncSetAttribute(frame_kernel_lean<B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
+template <int B, int J>
+cudaError_t lean_launch_j(const KernelArgs &args, const LaunchShape &s, cudaStream_t stream) {
+    cudaError_t e =
+        cudaFuncSetAttribute(frame_kernel_lean<B, J>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
     if (e != cudaSuccess) {
         return e;
     }
-    frame_kernel_lean<B><<<s.grid, s.threads, s.smem, stream>>>(args);
+    frame_kernel_lean<B, J><<<s.grid, s.threads, s.smem, stream>>>(args);
     return cudaGetLastError();
 }
 
 template <int B>
-cudaError_t lean_occ_b(const LaunchShape &s, int *out) {
-    cudaError_t e = cudaFuncSetAttribute(frame_kernel_lean<B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
+cudaError_t lean_launch_b(const KernelArgs &args, const LaunchShape &s, cudaStream_t stream) {
+    return s.short_phases ? lean_launch_j<B, kLeanShort>(args, s, stream) : lean_launch_j<B, kLeanJ>(args, s, stream);
+}
+
+template <int B, int J>
+cudaError_t lean_occ_j(const LaunchShape &s, int *out) {
+    cudaError_t e =
+        cudaFuncSetAttribute(frame_kernel_lean<B, J>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
     if (e != cudaSuccess) {
         return e;
     }
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, frame_kernel_lean<B>, s.threads, s.smem);
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, frame_kernel_lean<B, J>, s.threads, s.smem);
+}
+
+template <int B>
+cudaError_t lean_occ_b(const LaunchShape &s, int *out) {
+    return s.short_phases ? lean_occ_j<B, kLeanShort>(s, out) : lean_occ_j<B, kLeanJ>(s, out);
 }
 
 }  // namespace

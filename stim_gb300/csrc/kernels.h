@@ -79,6 +79,7 @@ struct LaunchShape {
     bool ring_global;    // measurement ring in global memory (per-CTA region) instead of shared memory
     bool hits = false;   // hit-list mode (noise precomputed by noise_kernel)
     bool frames_global = false;  // X / Z frames in global memory (one block per CTA only)
+    bool short_phases = false;   // lean kernel: phases of at most about two items a thread
 };
 
 // `nrows` = frame rows held in shared memory (0 when the frames are in global memory).

@@ -142,3 +142,17 @@ def test_error_models(name):
             wd, wo, _ = b.sample(shots, bit_packed=packed, return_errors=True)
             np.testing.assert_array_equal(d, wd)
             np.testing.assert_array_equal(o, wo)
+
+
+@pytest.mark.parametrize("qubits,shots", [(2, 1), (64, 129), (65, 1000), (128, 513), (130, 300), (300, 140)])
+def test_short_phases_around_two_items_a_thread(qubits, shots):
+    # The lean frame kernel that works two phases ahead, against the generic one: circuits whose phases have fewer and more
+    # items than its threads take (four blocks per CTA: 2 * 256 / 4 = 128 rows), with and without a loop.
+    text = workloads.random_clifford_circuit(qubits, 40, 3)
+    for t in (text, "REPEAT 3 {\n" + text + "}\n" + text):
+        c = stim_gb300.Circuit(t)
+        for make in (c.compile_detector_sampler, c.compile_sampler):
+            a, b = make(seed=4), make(seed=4)
+            b.set_noise_mode(1)
+            b.set_frame_kernel(0)
+            np.testing.assert_array_equal(a.sample(shots, bit_packed=True), b.sample(shots, bit_packed=True))
