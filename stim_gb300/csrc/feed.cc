@@ -50,6 +50,12 @@ void sample_for_decoder(gfs_sampler *s, uint64_t shots, const uint8_t *mask, uin
     const uint64_t per_shot = std::max<uint64_t>(1, drow + orow);
     const uint64_t wave = std::max<uint64_t>(128, (uint64_t)s->shape.grid * (uint64_t)s->shape.blocks_per_cta * 128);
     uint64_t chunk = std::max<uint64_t>(1, ((uint64_t)512 << 20) / per_shot / wave) * wave;
+    const bool symptoms = s->symptoms_active(GFS_BIT_PACKED);
+    if (symptoms) {
+        // Symptom sampling has no waves to fill: 40 MiB of rows per chunk, so that copies of kept rows overlap the next
+        // chunk's kernels from early on (d=15, 2^18 shots: 667 us; 24 MiB 705, 32 689, 48 688, one chunk 809).
+        chunk = std::max<uint64_t>(128, ((uint64_t)40 << 20) / per_shot / 128 * 128);
+    }
     chunk = std::min<uint64_t>(chunk, (shots + 127) / 128 * 128);
     chunk = std::max<uint64_t>(chunk, 128);
     const uint64_t groups = (chunk + gfs::kFeedGroup - 1) / gfs::kFeedGroup;
@@ -89,37 +95,18 @@ void sample_for_decoder(gfs_sampler *s, uint64_t shots, const uint8_t *mask, uin
         a.dst = (uint32_t *)(aux + aux_dst);
     }
     ck(cudaStreamSynchronize(s->stream), "mask upload");
-    // Two slots: chunk n samples into slot n % 2 while the kept rows of chunk n - 1 leave on the copy stream (with
-    // page-locked destinations the copy overlaps the next chunk's kernels).  The per-chunk counts reach the host
-    // through mapped memory (launch_publish_words), not a copy that would queue behind the rows on the copy
-    // engine.  A slot is reused once its copy has ended.
+    // Two slots: chunk n is sampled, counted and compacted into slot n % 2; its counts reach the host through mapped memory
+    // (launch_publish_words), not a copy that would queue behind the rows on the copy engine.  The host then waits for the
+    // counts of chunk n - 1, whose kept rows leave on the copy stream (with page-locked destinations beside chunk n's
+    // kernels), so the device always has a chunk to work on.  A slot is reused once its copy has ended.
     uint64_t kept_total = 0, dropped = 0, events = 0;
     bool copying[2] = {false, false};
-    uint64_t n = 0;
-    for (uint64_t done = 0; done < shots; n++) {
-        const int k = (int)(n & 1);
-        gfs::FeedArgs &a = args[k];
-        if (copying[k]) {
-            ck(cudaEventSynchronize(s->pev[k][3]), "feed copy");
-            copying[k] = false;
-        }
-        const uint64_t cs = std::min<uint64_t>(shots - done, chunk);
-        // detections() leaves the rows written and s->stream idle.
-        s->detections(cs, GFS_BIT_PACKED, drow ? (uint8_t *)a.dets : nullptr, drow,
-                      orow ? (uint8_t *)a.obs : nullptr, orow, true);
-        a.nshots = cs;
-        ck(cudaMemsetAsync(a.counts, 0, 16, s->stream), "memset");
-        ck(gfs::launch_feed_popcount(a, s->stream), "popcount launch");
-        if (nmask) {
-            ck(gfs::launch_feed_flags(a, s->stream), "flags launch");
-            ck(gfs::launch_feed_scan(a, s->stream), "scan launch");
-            ck(gfs::launch_feed_compact(a, s->stream), "compact launch");
-        }
-        ck(gfs::launch_publish_words((const uint32_t *)a.counts, s->h_words_dev + 4, 4, s->stream), "counts publish");
-        ck(cudaStreamSynchronize(s->stream), "feed");
-        const volatile uint32_t *w = s->h_words + 4;
+    auto finish = [&](int k) {
+        const gfs::FeedArgs &a = args[k];
+        ck(cudaEventSynchronize(s->pev[k][2]), "feed");
+        const volatile uint32_t *w = s->h_words + 4 + 4 * k;
         const uint64_t ev = (uint64_t)w[0] | ((uint64_t)w[1] << 32), dr = (uint64_t)w[2] | ((uint64_t)w[3] << 32);
-        const uint64_t kept = cs - dr;
+        const uint64_t kept = a.nshots - dr;
         dropped += dr;
         events += ev;
         const uint8_t *src = nmask ? a.cdets : a.dets;
@@ -133,7 +120,44 @@ void sample_for_decoder(gfs_sampler *s, uint64_t shots, const uint8_t *mask, uin
         ck(cudaEventRecord(s->pev[k][3], s->copy_stream), "event");
         copying[k] = true;
         kept_total += kept;
+    };
+    if (symptoms) {
+        s->reset_timings();
+    }
+    uint64_t n = 0;
+    for (uint64_t done = 0; done < shots; n++) {
+        const int k = (int)(n & 1);
+        gfs::FeedArgs &a = args[k];
+        if (copying[k]) {
+            ck(cudaEventSynchronize(s->pev[k][3]), "feed copy");
+            copying[k] = false;
+        }
+        const uint64_t cs = std::min<uint64_t>(shots - done, chunk);
+        uint8_t *const rows = drow ? (uint8_t *)a.dets : nullptr, *const orows = orow ? (uint8_t *)a.obs : nullptr;
+        if (symptoms) {
+            s->run_symptoms(cs, s->next_block, GFS_BIT_PACKED, rows, drow, orows, orow);
+            s->next_block += (cs + 127) / 128;
+        } else {
+            s->detections(cs, GFS_BIT_PACKED, rows, drow, orows, orow, true);
+        }
+        a.nshots = cs;
+        ck(cudaMemsetAsync(a.counts, 0, 16, s->stream), "memset");
+        ck(gfs::launch_feed_popcount(a, s->stream), "popcount launch");
+        if (nmask) {
+            ck(gfs::launch_feed_flags(a, s->stream), "flags launch");
+            ck(gfs::launch_feed_scan(a, s->stream), "scan launch");
+            ck(gfs::launch_feed_compact(a, s->stream), "compact launch");
+        }
+        ck(gfs::launch_publish_words((const uint32_t *)a.counts, s->h_words_dev + 4 + 4 * k, 4, s->stream),
+           "counts publish");
+        ck(cudaEventRecord(s->pev[k][2], s->stream), "event");
+        if (n > 0) {
+            finish(k ^ 1);
+        }
         done += cs;
+    }
+    if (n > 0) {
+        finish((int)((n - 1) & 1));
     }
     ck(cudaStreamSynchronize(s->copy_stream), "copy");
     out3[0] = kept_total;

@@ -156,3 +156,25 @@ def test_short_phases_around_two_items_a_thread(qubits, shots):
             b.set_noise_mode(1)
             b.set_frame_kernel(0)
             np.testing.assert_array_equal(a.sample(shots, bit_packed=True), b.sample(shots, bit_packed=True))
+
+
+@pytest.mark.parametrize("family,distance,ndet_mask", [("surface_code:rotated_memory_z", 3, 2), ("color_code:memory_xyz", 7, 9),
+                                                       ("surface_code:rotated_memory_z", 15, 24),
+                                                       ("surface_code:rotated_memory_z", 9, 400)])
+@pytest.mark.parametrize("shots", [127, 20_011])
+def test_decoder_feed_rows_of_any_width(family, distance, ndet_mask, shots):
+    # Rows of 3, 21, 421 and 90 bytes, masks of a few bytes and of many, several chunks, against numpy on plain samples.
+    text = workloads.code_circuit(family, distance, distance, 0.003)
+    c = stim_gb300.Circuit(text)
+    bits = np.zeros(c.num_detectors, np.bool_)
+    bits[np.random.default_rng(5).choice(c.num_detectors, ndet_mask, replace=False)] = True
+    mask = np.packbits(bits, bitorder="little")
+    a, b = c.compile_detector_sampler(seed=8), c.compile_detector_sampler(seed=8)
+    b.set_noise_mode(1)
+    for _ in range(2):
+        d, o = b.sample(shots, bit_packed=True, separate_observables=True)
+        drop = (d & mask).any(axis=1)
+        got = a.sample_for_decoder(shots, postselection_mask=mask)
+        np.testing.assert_array_equal(got[0], d[~drop])
+        np.testing.assert_array_equal(got[1], o[~drop])
+        assert got[2:] == (int(drop.sum()), int(np.unpackbits(d).sum()))
