@@ -275,4 +275,32 @@ __device__ __forceinline__ void hit_prefetch(const KernelArgs &p, const uint32_t
     }
 }
 
+// Lane r holds row r of a 32x32 bit matrix (bit c = column c); afterwards lane c holds column c.  Stage s
+// (16, 8, 4, 2, 1) swaps the off-diagonal s x s sub-blocks between lanes l and l^s: the partner's word is
+// rotated by s toward the bits this lane takes (left when lane bit s is clear, right when set) and merged
+// under this lane's mask.  keep[k] / rot[k] depend only on the lane, so a stage is a shuffle, a funnel
+// shift and one bitwise select.
+struct Transpose32 {
+    uint32_t keep[5], rot[5];
+    __device__ __forceinline__ explicit Transpose32(uint32_t lane) {
+        const uint32_t lo[5] = {0x0000FFFFu, 0x00FF00FFu, 0x0F0F0F0Fu, 0x33333333u, 0x55555555u};
+#pragma unroll
+        for (int k = 0; k < 5; k++) {
+            const uint32_t s = 16u >> k;
+            const bool hi = (lane & s) != 0;
+            keep[k] = hi ? ~lo[k] : lo[k];
+            rot[k] = hi ? 32u - s : s;
+        }
+    }
+    __device__ __forceinline__ uint32_t operator()(uint32_t x) const {
+#pragma unroll
+        for (int k = 0; k < 5; k++) {
+            const uint32_t y = __shfl_xor_sync(0xFFFFFFFFu, x, 16u >> k);
+            const uint32_t r = __funnelshift_l(y, y, rot[k]);
+            x = (x & keep[k]) | (r & ~keep[k]);
+        }
+        return x;
+    }
+};
+
 }  // namespace gfs

@@ -191,6 +191,23 @@ struct FoldArgs {
 };
 cudaError_t launch_fold(const FoldArgs &args, cudaStream_t stream);
 
+// The whole conversion of bit-packed records in one kernel (m2d_block.cu), for circuits whose records and outputs of 128
+// shots fit in shared memory.  lists: per output eight 16-bit measurement indices, kFoldNone after the last; a first one
+// of kFoldLong marks an output with more (off / idx).  Rows in and out are contiguous (mrow, drow, orow bytes a shot).
+constexpr uint32_t kFoldNone = 0xFFFFu, kFoldLong = 0xFFFEu;
+struct ConvertArgs {
+    const uint8_t *in;  // 16-byte aligned; device memory, or host memory the device can read
+    uint64_t nshots;
+    uint32_t M, D, O;
+    const uint4 *lists;
+    const uint32_t *off, *idx;
+    const uint8_t *expect;
+    uint8_t *dets, *obs;  // null: not wanted
+    int append;           // the observables follow the detectors in the detector rows
+};
+size_t convert_smem_bytes(uint32_t M, uint32_t D, uint32_t O, bool append);
+cudaError_t launch_convert(const ConvertArgs &args, cudaStream_t stream);
+
 // Detector-error-model sampling (gfs_dem_*).  A probability group of error mechanisms: its mechanisms are
 // units[first .. first + n); gap table at tables[table] (when 0 < p < 1).
 struct DemGroup {

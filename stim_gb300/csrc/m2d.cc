@@ -28,7 +28,9 @@ struct gfs_m2d {
     bool sweep_controlled = false;  // the circuit has sweep-controlled operations
     std::vector<uint32_t> off, idx;
     std::vector<uint8_t> expect;
-    DevBuf d_off, d_idx, d_expect, sweep_in, sweep_rows;
+    DevBuf d_off, d_idx, d_expect, d_lists, sweep_in, sweep_rows;
+    bool small = false;  // every measurement index fits the short lists of launch_convert
+    bool reads_host = false;  // the device reads pageable host memory through the host's page tables
     // Three pipeline slots: chunk k runs on slot k % 3 (its own stream and buffers), so chunk k's device->host
     // copy overlaps chunk k + 1's host->device copy and kernels, and chunk k + 2's copy in need not wait for it.
     static constexpr int kSlots = 3;
@@ -169,6 +171,25 @@ void create(gfs_m2d *m, const gfs_circuit *c, const uint8_t *ref, int device) {
     upload(m->d_off, m->off, device, m->stream);
     upload(m->d_idx, m->idx, device, m->stream);
     upload(m->d_expect, m->expect, device, m->stream);
+    int reads_host = 0;
+    ck(cudaDeviceGetAttribute(&reads_host, cudaDevAttrPageableMemoryAccess, device), "attribute");
+    m->reads_host = reads_host != 0;
+    std::vector<uint32_t> lists;
+    m->small = m->M < gfs::kFoldLong && n < 0xFFFFFFu;
+    if (m->small) {
+        lists.reserve(4 * n);
+        for (uint64_t k = 0; k < n; k++) {
+            uint32_t h[8];
+            const uint32_t len = m->off[k + 1] - m->off[k];
+            for (uint32_t j = 0; j < 8; j++) {
+                h[j] = len > 8 ? gfs::kFoldLong : j < len ? m->idx[m->off[k] + j] : gfs::kFoldNone;
+            }
+            for (uint32_t j = 0; j < 8; j += 2) {
+                lists.push_back(h[j] | (h[j + 1] << 16));
+            }
+        }
+        upload(m->d_lists, lists, device, m->stream);
+    }
     ck(cudaStreamSynchronize(m->stream), "upload");
 }
 
@@ -214,15 +235,35 @@ void convert(gfs_m2d *m, uint64_t shots, const uint8_t *meas, uint64_t meas_stri
         throw std::invalid_argument("obs row stride too small");
     }
     ck(cudaSetDevice(m->device), "cudaSetDevice");
+    // One kernel (launch_convert) for packed rows when 128 shots fit its shared memory (d=17 still does: 967 us -> 772 per
+    // 2^17 shots from pageable records).
+    const bool fused = packed && !use_sweep && m->small && !(flags & GFS_PREPEND_OBSERVABLES) &&
+                       gfs::convert_smem_bytes((uint32_t)M, (uint32_t)D, (uint32_t)O, flags & GFS_APPEND_OBSERVABLES) <=
+                           (size_t)200 << 10;
+    // The kernel reads contiguous aligned pageable records where they are instead of a copy of them, where the device can: a
+    // copy from pageable memory holds the calling thread and runs at half the link's rate (d=11, 2^18 shots: 508 us with
+    // copies, 468 without).  From page-locked memory the copy engine is the faster one, except for small calls, which a
+    // copy only delays (d=3, 1,024 shots: 31 us).
+    const bool direct = fused && m->reads_host && meas_stride == mrow && ((uintptr_t)meas & 15) == 0 &&
+                        (shots * mrow <= (1u << 20) || !gfs_sampler::page_locked({meas}));
     // Chunks of up to 2^16 shots, fewer when a circuit's rows are large (about 1 GiB of device buffers).
     const uint64_t per_block = (M + D + O) * 16 + 128 * (mrow + drow + orow);
     uint64_t cb = std::max<uint64_t>(1, std::min<uint64_t>(512, ((uint64_t)1 << 30) / std::max<uint64_t>(1, per_block)));
+    if (fused) {
+        // 8 MiB a chunk (d=11: 468 us; 2 MiB 537, 4 478, 16 465).
+        cb = std::max<uint64_t>(1, ((uint64_t)8 << 20) / std::max<uint64_t>(1, 128 * std::max(mrow, drow + orow)));
+        cb = std::min<uint64_t>(cb, (shots + 127) / 128);
+    }
     const uint64_t chunk = cb * 128;
     for (int k = 0; k < gfs_m2d::kSlots; k++) {
-        m->in_buf[k].ensure(std::max<uint64_t>(16, chunk * mrow), m->device);
-        m->rows_buf[k].ensure(std::max<uint64_t>(16, cb * M * 16), m->device);
-        m->det_buf[k].ensure(std::max<uint64_t>(16, cb * D * 16), m->device);
-        m->obs_buf[k].ensure(std::max<uint64_t>(16, cb * O * 16), m->device);
+        if (!direct) {
+            m->in_buf[k].ensure(std::max<uint64_t>(16, chunk * mrow), m->device);
+        }
+        if (!fused) {
+            m->rows_buf[k].ensure(std::max<uint64_t>(16, cb * M * 16), m->device);
+            m->det_buf[k].ensure(std::max<uint64_t>(16, cb * D * 16), m->device);
+            m->obs_buf[k].ensure(std::max<uint64_t>(16, cb * O * 16), m->device);
+        }
         m->out_buf[k].ensure(std::max<uint64_t>(16, chunk * (drow + orow)), m->device);
     }
     if (use_sweep) {
@@ -237,8 +278,27 @@ void convert(gfs_m2d *m, uint64_t shots, const uint8_t *meas, uint64_t meas_stri
     auto compute = [&](int k, uint64_t done, uint64_t cs, const uint4 *base_dets, const uint4 *base_obs) {
         cudaStream_t st = m->streams[k];
         const uint64_t nblk = (cs + 127) / 128;
-        copy2d(m->in_buf[k].p, mrow, meas + done * meas_stride, meas_stride, mrow, cs, cudaMemcpyHostToDevice, st,
-               "copy measurements");
+        if (!direct) {
+            copy2d(m->in_buf[k].p, mrow, meas + done * meas_stride, meas_stride, mrow, cs, cudaMemcpyHostToDevice, st,
+                   "copy measurements");
+        }
+        if (fused) {
+            gfs::ConvertArgs ca{};
+            ca.in = direct ? meas + done * mrow : (const uint8_t *)m->in_buf[k].p;
+            ca.nshots = cs;
+            ca.M = (uint32_t)M;
+            ca.D = (uint32_t)D;
+            ca.O = (uint32_t)O;
+            ca.lists = (const uint4 *)m->d_lists.p;
+            ca.off = (const uint32_t *)m->d_off.p;
+            ca.idx = (const uint32_t *)m->d_idx.p;
+            ca.expect = (const uint8_t *)m->d_expect.p;
+            ca.dets = dets && drow ? (uint8_t *)m->out_buf[k].p : nullptr;
+            ca.obs = obs && orow ? (uint8_t *)m->out_buf[k].p + chunk * drow : nullptr;
+            ca.append = flags & GFS_APPEND_OBSERVABLES ? 1 : 0;
+            ck(gfs::launch_convert(ca, st), "convert kernel launch");
+            return;
+        }
         if (M == 0) {
             ck(cudaMemsetAsync(m->rows_buf[k].p, 0, 16, st), "memset");
         }
