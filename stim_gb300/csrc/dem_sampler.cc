@@ -29,6 +29,7 @@ struct gfs_dem {
     DevBuf d_chans;
     gfs_rt::SymptomDevice sym;
     int num_sms = 0;
+    bool writes_host = false;
 
     ~gfs_dem() {
         for (cudaStream_t st : streams) {
@@ -189,6 +190,7 @@ void create(gfs_dem *d, const char *text, size_t len, uint64_t seed, int device)
     std::vector<uint8_t> zeros((d->model.num_detectors + d->model.num_observables + 7) / 8 + 1, 0);
     upload(d->d_expect, zeros, device, d->stream);
     ck(cudaDeviceGetAttribute(&d->num_sms, cudaDevAttrMultiProcessorCount, device), "attribute");
+    d->writes_host = device_shares_host_memory(device);
     init_symptoms(d);
     ck(cudaStreamSynchronize(d->stream), "upload");
 }
@@ -220,6 +222,16 @@ void sample(gfs_dem *d, uint64_t shots, uint32_t flags, uint8_t *dets, uint64_t 
     ck(cudaSetDevice(d->device), "cudaSetDevice");
     const bool want_errs = errs != nullptr && !replay;
     const bool symptoms = d->sym.ready && !want_errs && !replay;
+    if (symptoms && d->writes_host && shots &&
+        gfs_rt::write_in_place({{dets, shots * dstride}, {obs, shots * ostride}}, true, packed)) {
+        gfs::SymArgs a = d->sym.call(shots, d->next_block, flags & GFS_BIT_PACKED, drow ? dets : nullptr, dstride,
+                                     orow ? obs : nullptr, ostride, (shots + 127) / 128, d->num_sms);
+        a.host = 1;
+        ck(gfs::launch_symptoms(a, d->stream), "symptom kernel launch");
+        ck(cudaStreamSynchronize(d->stream), "dem sample");
+        d->next_block += (shots + 127) / 128;
+        return;
+    }
     const uint64_t per_block = (D + O) * 16 + ((want_errs || replay) ? E * 16 : 0) +
                                128 * (drow + orow + (want_errs ? erow : 0) + (replay ? rrow : 0));
     uint64_t cb = std::max<uint64_t>(1, std::min<uint64_t>(512, ((uint64_t)1 << 30) / std::max<uint64_t>(1, per_block)));

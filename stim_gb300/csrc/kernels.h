@@ -136,6 +136,7 @@ struct SymArgs {
     uint8_t *dets, *obs;
     uint64_t dets_stride, obs_stride;
     int packed, append;
+    int host;  // the rows lie in host memory: plain stores only
 };
 size_t symptom_smem_bytes(uint32_t stride, uint32_t log_blocks);
 cudaError_t launch_symptoms(const SymArgs &args, cudaStream_t stream);

@@ -171,9 +171,7 @@ void create(gfs_m2d *m, const gfs_circuit *c, const uint8_t *ref, int device) {
     upload(m->d_off, m->off, device, m->stream);
     upload(m->d_idx, m->idx, device, m->stream);
     upload(m->d_expect, m->expect, device, m->stream);
-    int reads_host = 0;
-    ck(cudaDeviceGetAttribute(&reads_host, cudaDevAttrPageableMemoryAccess, device), "attribute");
-    m->reads_host = reads_host != 0;
+    m->reads_host = device_shares_host_memory(device);
     std::vector<uint32_t> lists;
     m->small = m->M < gfs::kFoldLong && n < 0xFFFFFFu;
     if (m->small) {

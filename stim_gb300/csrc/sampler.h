@@ -3,6 +3,8 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <cstdio>
@@ -12,6 +14,7 @@
 #include <new>
 #include <stdexcept>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/stim_gb300.h"
@@ -98,6 +101,40 @@ gfs_status guarded(F f) {
     } catch (const std::exception &e) {
         return fail(GFS_ERR_INTERNAL, e.what());
     }
+}
+
+// Whether kernels may read and write any host memory of this process, pageable or not, where it lies.
+inline bool device_shares_host_memory(int device) {
+    int access = 0, tables = 0;
+    ck(cudaDeviceGetAttribute(&access, cudaDevAttrPageableMemoryAccess, device), "attribute");
+    ck(cudaDeviceGetAttribute(&tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, device), "attribute");
+    return access != 0 && tables != 0;
+}
+
+// Whether a call's results (address and bytes; null: none) are small enough for its last kernel to write them straight to
+// host memory instead of staging and copying them: each copy costs more latency than a small call's kernels (1,024 shots
+// of d=3: 56 us, 28 without).  Symptom sampling writes 4 MiB so (d=11, 2.6 MB: 68 us, 61 in place; 10.8 MB: 115 and 184),
+// unpacked rows, whose bytes are mostly expansion, 8 (d=25 repetition code, 6.3 MB: 104 and 87); other kernels 64 KiB (their
+// transposes write rows in 2-byte units; 6.6 MB of d=9 records: 253 and 322).  Pages that nothing has touched yet are
+// populated first: the device would fault on them one by one (21 us each, 3 here).
+inline bool write_in_place(std::initializer_list<std::pair<void *, uint64_t>> parts, bool symptoms, bool packed) {
+    uint64_t bytes = 0;
+    for (const auto &p : parts) {
+        bytes += p.first ? p.second : 0;
+    }
+    if (bytes > (symptoms ? (packed ? (uint64_t)4 << 20 : (uint64_t)8 << 20) : (uint64_t)64 << 10)) {
+        return false;
+    }
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+    for (const auto &p : parts) {
+        if (p.first && p.second > 16384) {
+            const uintptr_t lo = (uintptr_t)p.first & ~(page - 1);
+#ifdef MADV_POPULATE_WRITE
+            madvise((void *)lo, (uintptr_t)p.first + p.second - lo, MADV_POPULATE_WRITE);  // advice: errors do not matter
+#endif
+        }
+    }
+    return true;
 }
 
 // Symptom sampling's tables on the device and the arguments that no call changes (symptoms.h).
@@ -251,6 +288,7 @@ struct gfs_sampler {
     // Symptom sampling (symptoms.h): detection calls run symptom_kernel when the program has an output table, unless the
     // caller chose a frame kernel, its launch shape or its noise mode.
     gfs_rt::SymptomDevice sym;
+    bool writes_host = false;  // the device writes pageable host memory through the host's page tables
     bool frame_chosen = false;  // a launch shape was set
     int occs_blocks = 0;          // blocks per slice the uploaded occurrence regions were planned for
     uint64_t slice_cap = 0;       // records per slice region
@@ -489,6 +527,7 @@ struct gfs_sampler {
                 ck(cudaEventCreate(&e), "cudaEventCreate");
             }
         }
+        writes_host = gfs_rt::device_shares_host_memory(device);
         upload(d_ops, prog.ops, device, stream);
         upload(d_pool, prog.pool, device, stream);
         upload(d_tables, prog.tables, device, stream);
@@ -531,10 +570,12 @@ struct gfs_sampler {
                ring_pref == -1 && hit_capacity_override == 0 && !(flags & GFS_PREPEND_OBSERVABLES);
     }
 
-    // Enqueues the sampling of `cs` shots from stream block `block0` on into device rows.
-    void run_symptoms(uint64_t cs, uint64_t block0, uint32_t flags, uint8_t *dd, uint64_t ds, uint8_t *od, uint64_t os) {
-        ck(gfs::launch_symptoms(sym.call(cs, block0, flags, dd, ds, od, os, (cs + 127) / 128, num_sms), stream),
-           "symptom kernel launch");
+    // Enqueues the sampling of `cs` shots from stream block `block0` on into device rows (host: rows in host memory).
+    void run_symptoms(uint64_t cs, uint64_t block0, uint32_t flags, uint8_t *dd, uint64_t ds, uint8_t *od, uint64_t os,
+                      bool host = false) {
+        gfs::SymArgs a = sym.call(cs, block0, flags, dd, ds, od, os, (cs + 127) / 128, num_sms);
+        a.host = host ? 1 : 0;
+        ck(gfs::launch_symptoms(a, stream), "symptom kernel launch");
         n_frame++;
     }
 
@@ -1003,7 +1044,9 @@ struct gfs_sampler {
         ck(cudaSetDevice(device), "cudaSetDevice");
         reset_timings();
         const bool symptoms = symptoms_active(flags);
-        if (!device_out) {
+        const bool direct = !device_out && writes_host &&
+                            gfs_rt::write_in_place({{dets, shots * dstride}, {obs, shots * ostride}}, symptoms, packed);
+        if (!device_out && !direct) {
             // Staging rows use the caller's stride when its rows are contiguous, so that each chunk leaves in
             // one linear copy; otherwise they are padded to 32 bytes and copied row by row.
             const uint64_t ds = dstride == drow ? drow : pad32(drow), os = ostride == orow ? orow : pad32(orow);
@@ -1029,7 +1072,7 @@ struct gfs_sampler {
         }
         if (symptoms) {
             ck(cudaEventRecord(ev[0], stream), "event");
-            run_symptoms(shots, next_block, flags, dets, dstride, obs, ostride);
+            run_symptoms(shots, next_block, flags, dets, dstride, obs, ostride, direct);
             ck(cudaEventRecord(ev[1], stream), "event");
             ck(cudaStreamSynchronize(stream), "sample");
             next_block += (shots + 127) / 128;
@@ -1138,6 +1181,10 @@ struct gfs_sampler {
             ref_bits.ensure((M + 7) / 8, device);
             ck(cudaMemcpyAsync(ref_bits.p, ref, (M + 7) / 8, cudaMemcpyHostToDevice, stream), "ref upload");
             dref = (const uint8_t *)ref_bits.p;
+        }
+        if (writes_host && gfs_rt::write_in_place({{out, shots * stride}}, false, packed)) {
+            measurements_device(shots, flags, ref, out, stride);
+            return;
         }
         const uint64_t rs = stride == row ? row : pad32(row);
         host_pipeline(

@@ -280,15 +280,33 @@ __device__ __forceinline__ void write_packed(const SymArgs &a, const SymStage &s
     asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the rows may be changed
 }
 
-// Unpacked rows (columns [c0, c1) of every shot): one warp per row, consecutive lanes writing consecutive aligned
-// 32-bit words of four expanded bits; the partial words at the ends byte by byte.
-__device__ __forceinline__ void write_unpacked(const SymArgs &a, const uint32_t *win, uint32_t c0, uint32_t c1,
-                                               uint64_t shot0, uint32_t nvalid) {
+// Unpacked rows, and rows of any kind in host memory (columns [c0, c1) of every shot): one warp per row, consecutive lanes
+// writing consecutive aligned 32-bit words, of four expanded bits or (a packed row's words are its destination's) as they
+// are; the partial words at the ends byte by byte.
+template <bool PACKED>
+__device__ __forceinline__ void write_words(const SymArgs &a, const uint32_t *win, uint32_t c0, uint32_t c1,
+                                            uint64_t shot0, uint32_t nvalid, uint32_t dst0, bool last) {
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    const int32_t nbytes = (int32_t)(c1 - c0);
     for (uint32_t r = warp; r < nvalid; r += nwarps) {
         const uint32_t *row = win + (size_t)r * a.stride;
-        uint8_t *const d = a.dets + (shot0 + r) * a.dets_stride + c0;
+        uint8_t *const start = a.dets + (shot0 + r) * a.dets_stride;
+        if (PACKED) {
+            const uint32_t mis = row_shift<true>(a, dst0, r) >> 3;
+            uint8_t *const d = start - mis + c0 / 8;  // of the row's word 0: 16-byte aligned
+            const uint32_t begin = c0 == 0 ? mis : 0, end = last ? mis + (c1 + 7) / 8 - c0 / 8 : (c1 - c0) / 8;
+            for (uint32_t q = begin / 4 + lane; 4 * q < end; q += 32) {
+                if (4 * q >= begin && 4 * q + 4 <= end) {
+                    reinterpret_cast<uint32_t *>(d)[q] = row[q];
+                } else {
+                    for (uint32_t b = max(4 * q, begin); b < min(4 * q + 4, end); b++) {
+                        d[b] = (uint8_t)out_byte<true>(row, b);
+                    }
+                }
+            }
+            continue;
+        }
+        const int32_t nbytes = (int32_t)(c1 - c0);
+        uint8_t *const d = start + c0;
         const int32_t mis = (int32_t)((uintptr_t)d & 3u);
         uint32_t *const dw = reinterpret_cast<uint32_t *>(d - mis);
         for (int32_t q = (int32_t)lane; 4 * q < mis + nbytes; q += 32) {
@@ -363,10 +381,10 @@ __device__ __forceinline__ void sample_blocks(const SymArgs &a, uint32_t cta) {
             __syncthreads();
         }
         if (a.dets) {
-            if (PACKED) {
+            if (PACKED && !a.host) {
                 write_packed(a, st, win, c1, shot0, nvalid, dst0, last);
             } else {
-                write_unpacked(a, win, st.flush0, c1, shot0, nvalid);
+                write_words<PACKED>(a, win, st.flush0, c1, shot0, nvalid, dst0, last);
             }
         }
         if (!last) {
