@@ -408,14 +408,15 @@ __device__ __forceinline__ void noise_warp(const KernelArgs &p, uint64_t w, uint
     }
 }
 
+constexpr uint64_t kNoiseFewWarps = 152 * 16;  // see launch_noise_b
+
 template <int B>
 __host__ __device__ constexpr int noise_slices_per_warp() {
     return noise_slices_per_warp_for(B);
 }
 
-template <int B>
+template <int B, int SB>
 __global__ void __launch_bounds__(256) noise_kernel(const KernelArgs p) {
-    constexpr int SB = noise_slices_per_warp<B>();
     __shared__ NoiseQueued queue[8][64];
     __shared__ uint32_t counts[8 * SB];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
@@ -1282,16 +1283,28 @@ cudaError_t launch_frame_kernel(const KernelArgs &args, const LaunchShape &shape
     }
 }
 
-template <int B>
-static cudaError_t launch_noise_b(const KernelArgs &args, cudaStream_t stream) {
-    constexpr int SB = noise_slices_per_warp<B>();
-    const uint64_t warps = (uint64_t)((args.nslices + SB - 1) / SB) * args.n_occ;
+template <int B, int SB>
+static cudaError_t launch_noise_sb(const KernelArgs &args, uint64_t warps, cudaStream_t stream) {
     const uint64_t blocks = (warps + 7) / 8;
     if (blocks > 0x7FFFFFFFull) {
         return cudaErrorInvalidValue;
     }
-    noise_kernel<B><<<(unsigned)blocks, 256, 0, stream>>>(args);
+    noise_kernel<B, SB><<<(unsigned)blocks, 256, 0, stream>>>(args);
     return cudaGetLastError();
+}
+
+template <int B>
+static cudaError_t launch_noise_b(const KernelArgs &args, cudaStream_t stream) {
+    constexpr int SB = noise_slices_per_warp<B>(), kFew = 2;
+    // Small launches: with SB slices a warp the GPU holds a few warps per SM, each walking SB slices in turn; two slices a
+    // warp end sooner where their segments still fill half a warp's screening round (d=9 measurements, 2^16 shots: 39 -> 31
+    // us; 256-qubit Clifford layers, 2^15: 181 -> 68; d=15, 2^16: 91 -> 73).  Above 16 warps per SM it costs (64-qubit
+    // layers, 2^17 shots, 23 warps per SM: 60 -> 76), as with fewer segments (d=25 repetition code: 25 -> 28).
+    auto warps = [&](uint64_t sb) { return (args.nslices + sb - 1) / sb * args.n_occ; };
+    if (SB > kFew && warps(SB) < kNoiseFewWarps && args.mean_segments * B * kFew >= 16) {
+        return launch_noise_sb<B, kFew>(args, warps(kFew), stream);
+    }
+    return launch_noise_sb<B, SB>(args, warps(SB), stream);
 }
 
 cudaError_t launch_noise_kernel(const KernelArgs &args, int blocks_per_cta, cudaStream_t stream) {

@@ -41,6 +41,7 @@ struct KernelArgs {
     uint64_t slice_cap;      // records per slice region
     uint32_t smem_occ;       // n_occ when the occurrence offsets and the slice's counts are cached in shared
                              // memory, else 0
+    uint32_t mean_segments;  // of an occurrence (chooses the noise kernel's slices per warp)
     uint32_t reset_zero;     // 1: start every shot's Z frame at zero instead of random (Program::reset_norand)
     const uint4 *sweep;      // [local block][nsweep] sweep bits read by sweep feedback; null: all zero
     uint32_t nsweep;

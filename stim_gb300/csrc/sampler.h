@@ -292,6 +292,7 @@ struct gfs_sampler {
     bool frame_chosen = false;  // a launch shape was set
     int occs_blocks = 0;          // blocks per slice the uploaded occurrence regions were planned for
     uint64_t slice_cap = 0;       // records per slice region
+    uint32_t mean_segments = 0;   // noise segments per occurrence and 128-shot block
     uint64_t n_hit_overflows = 0;
     uint64_t hit_capacity_override = 0;  // records per occurrence region (0 = from the expected hits)
     uint64_t chunk_shots = 0;
@@ -540,6 +541,11 @@ struct gfs_sampler {
                 upload(d_occ_xform, prog.occ_xform, device, stream);
             }
         }
+        uint64_t segments = 0;
+        for (const gfs::NoiseOcc &o : prog.occs) {
+            segments += (prog.ops[o.pc].n + GFS_SEG_UNITS - 1) / GFS_SEG_UNITS;
+        }
+        mean_segments = (uint32_t)(segments / std::max<size_t>(1, prog.occs.size()));
         d_status.ensure(16, device);
         ck(cudaHostAlloc((void **)&h_words, 64, cudaHostAllocMapped), "cudaHostAlloc");
         ck(cudaHostGetDevicePointer((void **)&h_words_dev, h_words, 0), "cudaHostGetDevicePointer");
@@ -703,6 +709,7 @@ struct gfs_sampler {
             a.hit_count = (uint32_t *)hit_count.p;
             a.occs = (const gfs::NoiseOcc *)d_occs.p;
             a.n_occ = (uint32_t)prog.occs.size();
+            a.mean_segments = mean_segments;
             a.slice_cap = slice_cap;
             a.smem_occ = smem_occ(true);
             a.occ_xform = lean ? occ_xform() : nullptr;  // records for the lean plan's moved hit phases
@@ -743,11 +750,15 @@ struct gfs_sampler {
         n_transpose++;
     }
 
-    // Reads and clears the kernels' status word (after the stream has drained).  Bits 1 and 2 are errors;
-    // bit 4 (a hit list overflowed) is returned as true: the caller redoes the affected shots inline.
-    bool check_status() {
+    // Queues the kernels' status word for take_status() (after the launches it speaks for, before the wait for them, so that
+    // one wait serves both).
+    void publish_status() {
         ck(gfs::launch_publish_words((const uint32_t *)d_status.p, h_words_dev, 1, stream), "status publish");
-        ck(cudaStreamSynchronize(stream), "status read");
+    }
+
+    // Reads and clears the published status word, once the stream has drained.  Bits 1 and 2 are errors; bit 4 (a hit list
+    // overflowed) is returned as true: the caller redoes the affected shots inline.
+    bool take_status() {
         const uint32_t st = *(volatile uint32_t *)h_words;
         if (st) {
             ck(cudaMemsetAsync(d_status.p, 0, 4, stream), "status clear");
@@ -761,6 +772,12 @@ struct gfs_sampler {
             return true;
         }
         return false;
+    }
+
+    bool check_status() {
+        publish_status();
+        ck(cudaStreamSynchronize(stream), "status read");
+        return take_status();
     }
 
     // Times the frame kernel for each candidate launch shape on whole waves of at least `trial_shots` shots and
@@ -951,6 +968,9 @@ struct gfs_sampler {
             issue_copy(prev);
         }
         ck(cudaEventRecord(ev[1], copy_stream), "event");
+        if (!symptoms) {
+            publish_status();
+        }
         for (int slot = 0; slot < 2; slot++) {
             if (used[slot]) {
                 account(slot);
@@ -960,7 +980,7 @@ struct gfs_sampler {
         ck(cudaEventSynchronize(ev[1]), "sample");
         t_total = elapsed(0, 1);
         t_copy = std::max(0.0, t_total - t_frame - t_noise - t_transpose);
-        if (!symptoms && check_status()) {
+        if (!symptoms && take_status()) {
             // A hit list overflowed somewhere: redo the whole request with inline noise (same results).
             next_block = first_block;
             force_inline = true;
@@ -1091,10 +1111,11 @@ struct gfs_sampler {
             transpose_detections(flags, cs, dets ? dets + done * dstride : nullptr, dstride,
                                  obs ? obs + done * ostride : nullptr, ostride, dets != nullptr, obs != nullptr);
             ck(cudaEventRecord(ev[3], stream), "event");
+            publish_status();
             ck(cudaStreamSynchronize(stream), "sample");
             t_frame += elapsed(1, 2) - account_noise(-1);
             t_transpose += elapsed(2, 3);
-            if (check_status()) {
+            if (take_status()) {
                 // The chunk's hit list overflowed: redo it with inline noise (same results).
                 force_inline = true;
                 try {
@@ -1147,9 +1168,10 @@ struct gfs_sampler {
                 run_frame(nblk, next_block);
                 transpose((const uint4 *)meas_tmp.p, M, nullptr, 0, nullptr, 0, dref, cs, out + done * stride, stride,
                           packed);
+                publish_status();
                 ck(cudaStreamSynchronize(stream), "sample");
                 account_noise(-1);
-                const bool overflow = check_status();
+                const bool overflow = take_status();
                 force_inline = false;
                 if (!overflow) {
                     break;
