@@ -59,6 +59,7 @@ void init_symptoms(gfs_dem *d) {
     std::vector<std::vector<uint32_t>> seg(GFS_DEM_SEG_UNITS);
     std::vector<uint32_t> all, part;
     constexpr uint32_t kSpread = 2048;
+    double hits = 0;  // expected per 128-shot block
     for (uint32_t g = 0; g < (uint32_t)L.groups.size(); g++) {
         const gfs::DemGroup &G = L.groups[g];
         gfs::DevChan ch{};
@@ -72,6 +73,7 @@ void init_symptoms(gfs_dem *d) {
         if (!(G.flags & 1u)) {
             continue;
         }
+        hits += m.p[L.units[G.first]] * G.n * GFS_BLOCK_SHOTS;
         for (uint32_t u0 = 0; u0 < G.n; u0 += GFS_DEM_SEG_UNITS) {
             const uint32_t n = std::min(GFS_DEM_SEG_UNITS, G.n - u0);
             for (uint32_t u = 0; u < n; u++) {
@@ -159,6 +161,9 @@ void init_symptoms(gfs_dem *d) {
                     }
                     return gfs::plan_stages(spans, D, O, words, plan);
                 });
+    // Screening draws the first gap of a segment with a hit twice.  d=25 at 0.04 / 0.18 / 0.9 / 1.8 hits a segment, screened
+    // and not: 176 / 221 / 410 / 615 and 317 / 345 / 524 / 744 us; small models at 2.6 245 / 269, at 5.2 290 / 273.
+    d->sym.args.screen = hits < 2.0 * (double)items.size() ? 1 : 0;
 }
 
 void create(gfs_dem *d, const char *text, size_t len, uint64_t seed, int device) {

@@ -138,6 +138,7 @@ struct SymArgs {
     uint64_t dets_stride, obs_stride;
     int packed, append;
     int host;  // the rows lie in host memory: plain stores only
+    int screen;  // few segments have a hit: draw their first gap alone, and the rest only of those that have one
 };
 size_t symptom_smem_bytes(uint32_t stride, uint32_t log_blocks);
 cudaError_t launch_symptoms(const SymArgs &args, cudaStream_t stream);

@@ -8,7 +8,7 @@
 // One iteration of a warp draws 32 segments: one Philox call and two gap draws a lane, up to two hits (gap, choice, gap,
 // choice for a channel that draws its Pauli; a channel that does not uses two of the four draws as gaps).  Segments with
 // draws left wait in a queue of the warp until they fill an iteration, so every iteration but a stage's last few is
-// full.  Hits go to a second queue and are applied 32 at a time, one per lane, each list loaded one step before it is
+// full; where few segments have a hit (error models), the first gap decides which are drawn at all.  Hits go to a second queue and are applied 32 at a time, one per lane, each list loaded one step before it is
 // applied.
 //
 // What bounds it: instruction issue (d=25: 210 K warp instructions per block, a quarter of them Philox and gap
@@ -106,8 +106,15 @@ __device__ __forceinline__ void flip_outputs(const SymArgs &a, uint32_t *row, ui
     }
 }
 
+// The screening variant (error models of large codes: 82,000 segments a block, one in seven with a hit) has work for more
+// warps: d=25, 268 blocks, 256 / 384 / 512 threads 277 / 227 / 221 us, 345 without screening.
+constexpr uint32_t kScreenThreads = 512;
 constexpr uint32_t kThreads = 256;  // per CTA (d=25: 320 threads 1.98 ms for 2.04, but d=11 0.64 for 0.58)
 constexpr uint32_t kQueue = 64;     // hits, and segments with draws left, a warp can hold: under 32 left over, 32 more
+
+__host__ __device__ constexpr uint32_t threads(bool screen) {
+    return screen ? kScreenThreads : kThreads;
+}
 
 struct WarpQueues {
     uint2 hits[kQueue];  // output list; shot row << 16 | column of relative code 0
@@ -116,7 +123,7 @@ struct WarpQueues {
 
 // Draws the stage's items: work index j is item item0 + j / blocks of the CTA's block j % blocks; the warps take 32
 // consecutive indices in turn (from a shared counter instead: 2.12 ms for 2.04).
-template <bool PACKED>
+template <bool PACKED, bool SCREEN>
 __device__ __forceinline__ void draw_stage(const SymArgs &a, const SymStage &st, uint32_t *win, WarpQueues &q,
                                            uint32_t block0, uint32_t nblk, uint32_t dst0) {
     const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
@@ -173,7 +180,7 @@ __device__ __forceinline__ void draw_stage(const SymArgs &a, const SymStage &st,
             act = lane < take;
             const uint2 c = q.cont[cn + min(lane, take - 1)];
             j = c.x;
-            pos = (int32_t)(c.y & 0xFFFFu);
+            pos = (int32_t)(int16_t)(c.y & 0xFFFFu);  // -1: nothing of the segment is drawn yet
             draw = c.y >> 16;
             lo = __ldg(items + 2 * (j >> lb));
             hi = __ldg(items + 2 * (j >> lb) + 1);
@@ -183,8 +190,25 @@ __device__ __forceinline__ void draw_stage(const SymArgs &a, const SymStage &st,
             act = j < total && (j & bmask) < nblk;
             lo = flo;
             hi = fhi;
-            cur += kThreads;
+            cur += threads(SCREEN);
             fetch();
+            if (SCREEN) {
+                // Most segments have no hit and end here, after their first gap; those with one are queued and drawn whole, by
+                // full warps (in one pass the few hits of 32 segments took every warp through the second gap and both pushes).
+                bool any = false;
+                if (act) {
+                    const gfs_u32x4 r = gfs_philox(k0, k1, block0 + (j & bmask), lo.x, lo.y, lo.z);
+                    const int32_t trials = (int32_t)(hi.x >> 16);
+                    any = gap_step(r.v[0], a, hi.w, __uint_as_float(hi.z), -1, trials) < trials;
+                }
+                const uint32_t mask = __ballot_sync(0xFFFFFFFFu, any);
+                if (any) {
+                    q.cont[cn + __popc(mask & lt)] = make_uint2(j, 0xFFFFu);
+                }
+                cn += __popc(mask);
+                __syncwarp();
+                continue;
+            }
         } else {
             break;
         }
@@ -326,10 +350,11 @@ __device__ __forceinline__ void write_words(const SymArgs &a, const uint32_t *wi
 
 // Between stages: the words after the written piece move to the front of their row, the rest is cleared.  In 16-byte
 // units, eight lanes a row.
+template <uint32_t THREADS>
 __device__ __forceinline__ void next_window(const SymArgs &a, const SymStage &st, uint32_t *win, uint32_t rows) {
     const uint32_t n = (st.flush1 - st.flush0) / kSymAlign, keep = st.keep / (kSymAlign / 32);  // units
     const uint32_t l = threadIdx.x & 7u;
-    for (uint32_t r = threadIdx.x >> 3; r < rows; r += kThreads >> 3) {  // rows is a multiple of 128
+    for (uint32_t r = threadIdx.x >> 3; r < rows; r += THREADS >> 3) {  // rows is a multiple of 128
         uint4 *const row = reinterpret_cast<uint4 *>(win + (size_t)r * a.stride);
         for (uint32_t i0 = 0; i0 < keep; i0 += 8) {  // a pass reads ahead of what it and earlier ones write
             const uint32_t i = i0 + l;
@@ -347,10 +372,10 @@ __device__ __forceinline__ void next_window(const SymArgs &a, const SymStage &st
 }
 
 // Samples CTA `cta`'s blocks from the circuit's start to its end.
-template <bool PACKED>
+template <bool PACKED, bool SCREEN>
 __device__ __forceinline__ void sample_blocks(const SymArgs &a, uint32_t cta) {
     extern __shared__ __align__(16) uint32_t win[];  // [shot][stride]: detector words, then observable words
-    __shared__ WarpQueues queue[kThreads / 32];
+    __shared__ WarpQueues queue[threads(SCREEN) / 32];
     const uint32_t tid = threadIdx.x, nt = blockDim.x;
     const uint32_t rows = GFS_BLOCK_SHOTS << a.log_blocks;
     const uint64_t blk0 = (uint64_t)cta << a.log_blocks, shot0 = blk0 * GFS_BLOCK_SHOTS;
@@ -363,7 +388,7 @@ __device__ __forceinline__ void sample_blocks(const SymArgs &a, uint32_t cta) {
     __syncthreads();
     for (uint32_t k = 0; k < a.nstages; k++) {
         const SymStage st = a.stages[k];
-        draw_stage<PACKED>(a, st, win, queue[tid >> 5], (uint32_t)(a.block0 + blk0), nblk, dst0);
+        draw_stage<PACKED, SCREEN>(a, st, win, queue[tid >> 5], (uint32_t)(a.block0 + blk0), nblk, dst0);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the rows will be read by bulk copies
         __syncthreads();
         const bool last = k + 1 == a.nstages;
@@ -389,7 +414,7 @@ __device__ __forceinline__ void sample_blocks(const SymArgs &a, uint32_t cta) {
         }
         if (!last) {
             __syncthreads();
-            next_window(a, st, win, rows);
+            next_window<threads(SCREEN)>(a, st, win, rows);
             __syncthreads();
         }
     }
@@ -402,9 +427,9 @@ __device__ __forceinline__ void sample_blocks(const SymArgs &a, uint32_t cta) {
     }
 }
 
-template <bool PACKED>
-__global__ void __launch_bounds__(kThreads) symptom_kernel(const SymArgs a) {
-    sample_blocks<PACKED>(a, blockIdx.x);
+template <bool PACKED, bool SCREEN>
+__global__ void __launch_bounds__(threads(SCREEN)) symptom_kernel(const SymArgs a) {
+    sample_blocks<PACKED, SCREEN>(a, blockIdx.x);
 }
 
 template <bool PACKED>
@@ -426,16 +451,17 @@ __global__ void __launch_bounds__(kThreads)
         reinterpret_cast<uint32_t *>(&a)[threadIdx.x] = __ldg(reinterpret_cast<const uint32_t *>(entries + lo) + threadIdx.x);
     }
     __syncthreads();
-    sample_blocks<PACKED>(a, blockIdx.x - __ldg(prefix + lo));
+    sample_blocks<PACKED, false>(a, blockIdx.x - __ldg(prefix + lo));
 }
 
-template <bool PACKED>
+template <bool PACKED, bool SCREEN>
 cudaError_t launch_packed(const SymArgs &args, uint32_t grid, size_t smem, cudaStream_t stream) {
-    cudaError_t e = cudaFuncSetAttribute(symptom_kernel<PACKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e =
+        cudaFuncSetAttribute(symptom_kernel<PACKED, SCREEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) {
         return e;
     }
-    symptom_kernel<PACKED><<<grid, kThreads, smem, stream>>>(args);
+    symptom_kernel<PACKED, SCREEN><<<grid, threads(SCREEN), smem, stream>>>(args);
     return cudaGetLastError();
 }
 
@@ -467,8 +493,12 @@ cudaError_t launch_symptoms(const SymArgs &args, cudaStream_t stream) {
     if (grid > 0x7FFFFFFFull) {
         return cudaErrorInvalidValue;
     }
-    return args.packed ? launch_packed<true>(args, (uint32_t)grid, smem, stream)
-                       : launch_packed<false>(args, (uint32_t)grid, smem, stream);
+    if (args.screen) {
+        return args.packed ? launch_packed<true, true>(args, (uint32_t)grid, smem, stream)
+                           : launch_packed<false, true>(args, (uint32_t)grid, smem, stream);
+    }
+    return args.packed ? launch_packed<true, false>(args, (uint32_t)grid, smem, stream)
+                       : launch_packed<false, false>(args, (uint32_t)grid, smem, stream);
 }
 
 cudaError_t launch_batch_symptoms(const SymArgs *entries, const uint32_t *prefix, uint32_t n, uint32_t grid, size_t smem,

@@ -144,6 +144,20 @@ def test_error_models(name):
             np.testing.assert_array_equal(o, wo)
 
 
+@pytest.mark.parametrize("hits", [0.02, 1.98, 2.02])
+@pytest.mark.parametrize("mechanisms", [1, 4, 125, 4 * 16 * 32 + 3, 9001])
+def test_error_models_screened(hits, mechanisms):
+    # Below two hits a segment (4 mechanisms, 512 trials) a segment's first gap is drawn alone first; around that line, with
+    # fewer and more segments than a warp or a CTA has lanes.
+    p = hits / 512
+    text = "".join(f"error({p!r}) D{k // 2} D{k // 2 + 1}\n" for k in range(mechanisms)) + "logical_observable L0\n"
+    a, b = (stim_gb300.DetectorErrorModel(text).compile_sampler(seed=8) for _ in range(2))
+    for shots in (1, 129, 20001):
+        d, _, _ = a.sample(shots, bit_packed=True)
+        wd, _, _ = b.sample(shots, bit_packed=True, return_errors=True)
+        np.testing.assert_array_equal(d, wd)
+
+
 @pytest.mark.parametrize("qubits,shots", [(2, 1), (64, 129), (65, 1000), (128, 513), (130, 300), (300, 140)])
 def test_short_phases_around_two_items_a_thread(qubits, shots):
     # The lean frame kernel that works two phases ahead, against the generic one: circuits whose phases have fewer and more
