@@ -129,7 +129,9 @@ struct gfs_batch {
         for (const auto &g : eng.groups) {
             key.insert(key.end(), {(uint64_t)(uintptr_t)g.d_args.p, (uint64_t)(uintptr_t)g.d_prefix.p, g.args.size(), g.smem});
         }
-        for (const auto &e : es) {
+        for (size_t j = 0; j < es.size(); j++) {
+            const auto &e = es[j];
+            key.push_back(eng.by_symptoms[j]);  // a sampler's settings may have changed its route since
             key.push_back(e.shots);
             key.push_back((uint64_t)(uintptr_t)e.dets);
             key.push_back(e.dstride);

@@ -119,6 +119,20 @@ def test_batch_mixes_symptom_and_frame_entries():
             np.testing.assert_array_equal(r.result(), want)
 
 
+def test_batch_follows_settings_between_calls():
+    # Two samplers that trade routes between calls: as many entries each way as before, but not the same ones.
+    text = texts()["surface_code_d5"]
+    want = [stim_gb300.Circuit(text).compile_detector_sampler(seed=k).sample(900, bit_packed=True) for k in range(2)]
+    many = [stim_gb300.Circuit(text).compile_detector_sampler(seed=k) for k in range(2)]
+    batch = stim_gb300.BatchSampler(many)
+    for modes in ((1, -1), (-1, 1), (-1, -1), (1, 1), (-1, 1)):
+        for s, mode in zip(many, modes):
+            s.set_stream_position(0)
+            s.set_noise_mode(mode)
+        for got, w in zip(batch.sample([900, 900], bit_packed=True), want):
+            np.testing.assert_array_equal(got, w)
+
+
 def dem_text(name):
     if name == "surface_rz_d25":
         return workloads.dem_d25_text()
