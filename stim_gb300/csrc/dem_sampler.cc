@@ -226,7 +226,14 @@ void sample(gfs_dem *d, uint64_t shots, uint32_t flags, uint8_t *dets, uint64_t 
     }
     ck(cudaSetDevice(d->device), "cudaSetDevice");
     const bool want_errs = errs != nullptr && !replay;
-    const bool symptoms = d->sym.ready && !want_errs && !replay;
+    // A few blocks of a large model leave most SMs idle, one CTA drawing all segments of a block, while the kernels that go
+    // mechanism by mechanism spread them (host arrays, us, those and symptom sampling; 82 K segments: packed 1 block 86 and
+    // 172, 64 blocks 229 and 261, 96 blocks 308 and 304; unpacked 200 blocks 2,416 and 2,506, 256 blocks 3,068 and 3,110;
+    // 41 K segments: packed 8 blocks 90 and 94, 16 blocks 97 and 95, unpacked 96 blocks 646 and 677, 128 blocks 828 and
+    // 846; 20 K segments: symptom sampling throughout).
+    const uint64_t segments = d->sym.nitems, sample_blocks = (shots + 127) / 128;
+    const bool few_blocks = packed ? 512 * sample_blocks + (32u << 10) < segments : 192 * sample_blocks + (24u << 10) < segments;
+    const bool symptoms = d->sym.ready && !want_errs && !replay && !few_blocks;
     if (symptoms && d->writes_host && shots &&
         gfs_rt::write_in_place({{dets, shots * dstride}, {obs, shots * ostride}}, true, packed)) {
         gfs::SymArgs a = d->sym.call(shots, d->next_block, flags & GFS_BIT_PACKED, drow ? dets : nullptr, dstride,

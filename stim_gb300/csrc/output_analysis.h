@@ -4,7 +4,7 @@
 #pragma once
 
 #include <algorithm>
-#include <iterator>
+#include <cstring>
 
 #include "frame_rules.h"
 #include "gfs_contract.h"
@@ -15,7 +15,8 @@ namespace gfs {
 using Set = std::vector<uint32_t>;  // sorted outputs: detectors by index, then observables as kSymObs | index
 
 constexpr uint64_t kWorkLimit = 400000000ull;
-constexpr uint32_t kProbes = 12;              // iterations of a loop checked for a steady state
+constexpr uint32_t kProbes = 12;   // iterations of a loop checked for a steady state
+constexpr uint32_t kPeriods = 3;   // of one, two or three iterations (colour codes measure X, Y, Z in turn)
 constexpr size_t kMaxEntries = (size_t)1 << 22;   // output lists (16 bytes each) kept per program
 constexpr size_t kMaxLongs = (size_t)1 << 24;
 
@@ -25,8 +26,8 @@ constexpr size_t kMaxLongs = (size_t)1 << 24;
 // measurement result the outputs that read it.  A randomized row whose set is empty has coefficient zero in every
 // output, so writing zeros instead of random bits leaves every output unchanged for every noise realisation; and the
 // sets at a noise occurrence are the outputs its hits flip.  One iteration of a loop maps the state to itself with
-// detectors shifted by the body's count, whatever the iteration: once an iteration leaves the state it found (shifted),
-// all earlier ones do too, so the rest of the loop is filled in by shifting.  The pass gives up (marks nothing) past a
+// detectors shifted by the body's count, whatever the iteration: once a few iterations leave the state that they found
+// (shifted), all earlier ones do too, so the rest of the loop is filled in by shifting.  The pass gives up (marks nothing) past a
 // work limit.
 class OutputAnalysis {
    public:
@@ -83,8 +84,15 @@ class OutputAnalysis {
     bool record = false;  // output lists are being kept
     bool failed = false;
     std::vector<uint8_t> ok;
+    struct Flip {
+        uint32_t id, gens;
+    };
     Set tmp;
     std::vector<uint32_t> pattern;
+    std::vector<Flip> flips, merged;
+    static constexpr uint32_t kUnitCodes = 32;
+    uint32_t num_codes = 0, obs_parity = 0, code_parity[kUnitCodes];
+    uint16_t codes[kUnitCodes], obs_code = 0;
 
     void drop() {
         record = false;
@@ -95,8 +103,8 @@ class OutputAnalysis {
         if (b.empty()) {
             return;
         }
-        tmp.clear();
-        std::set_symmetric_difference(a.begin(), a.end(), b.begin(), b.end(), std::back_inserter(tmp));
+        tmp.resize(a.size() + b.size());
+        tmp.resize(merge(a.data(), a.size(), b.data(), b.size(), tmp.data()));
         a.swap(tmp);
         work += a.size() + b.size();
     }
@@ -111,17 +119,43 @@ class OutputAnalysis {
         work += 1 + a.size() / 8;
     }
 
-    // S_before[k] = XOR of S_after[i] over the outputs i of the forward map that input k reaches.
-    void transpose(uint32_t nv, const uint32_t image[4], Set *after[4]) {
-        Set before[4];
-        for (uint32_t k = 0; k < nv; k++) {
-            for (uint32_t i = 0; i < nv; i++) {
-                if ((image[k] >> i) & 1u) {
-                    sdiff(before[k], *after[i]);
+    // S_before[k] = XOR of S_after[i] over the outputs i of the forward map that input k reaches: by exchanging sets where
+    // each input reaches one output, in place where every set that is added stays as it is, else through copies.
+    struct Map {
+        uint32_t nv, image[4];
+        bool permutes = true, in_place = true;
+
+        void classify() {
+            for (uint32_t k = 0; k < nv; k++) {
+                permutes &= (image[k] & (image[k] - 1)) == 0;
+                in_place &= ((image[k] >> k) & 1u) != 0;
+                for (uint32_t i = 0; i < nv; i++) {
+                    in_place &= i == k || !((image[k] >> i) & 1u) || image[i] == 1u << i;
                 }
             }
         }
-        for (uint32_t k = 0; k < nv; k++) {
+    };
+
+    void transpose(const Map &m, Set *after[4]) {
+        if (m.in_place) {
+            for (uint32_t k = 0; k < m.nv; k++) {
+                for (uint32_t rest = m.image[k] & ~(1u << k); rest; rest &= rest - 1) {
+                    sdiff(*after[k], *after[__builtin_ctz(rest)]);
+                }
+            }
+            return;
+        }
+        Set before[4];
+        for (uint32_t k = 0; k < m.nv; k++) {
+            if (m.permutes) {
+                before[k].swap(*after[__builtin_ctz(m.image[k])]);
+                continue;
+            }
+            for (uint32_t rest = m.image[k]; rest; rest &= rest - 1) {
+                sdiff(before[k], *after[__builtin_ctz(rest)]);
+            }
+        }
+        for (uint32_t k = 0; k < m.nv; k++) {
             after[k]->swap(before[k]);
         }
     }
@@ -226,26 +260,99 @@ class OutputAnalysis {
             l.hi = hi;
             l.base = lo;
         }
-        size_t flips = 0;
+        size_t at = t.lists.entries.size(), count = 0;
+        t.lists.entries.resize(at + 4 * (size_t)n * l.per_unit);
         for (uint32_t u = 0; u < n; u++) {
-            size_t most = 0;
+            // The unit's outputs, each with the set of generators that flip it; pattern b flips those of odd overlap.
+            flips.clear();
             for (uint32_t g = 0; g < gens; g++) {
-                most += gen(u, g).size();
+                add_generator(gen(u, g), 1u << g);
             }
-            pattern.resize(std::max(pattern.size(), most << gens));
-            size_t len[16] = {0};
-            for (uint32_t b = 1; b < (1u << gens); b++) {  // pattern b = pattern without its lowest bit, XOR that bit's
-                const Set &g = gen(u, (uint32_t)__builtin_ctz(b));
-                const uint32_t c = b & (b - 1);
-                len[b] = merge(pattern.data() + c * most, len[c], g.data(), g.size(), pattern.data() + b * most);
-                if (!fixed || b == fixed) {
-                    t.lists.add(pattern.data() + b * most, len[b], l.base);
-                    flips += len[b];
+            const uint32_t first = fixed ? fixed : 1, past = fixed ? fixed + 1 : 1u << gens;
+            const bool small = code_unit(l.base);
+            for (uint32_t b = first; b < past; b++, at += 4) {
+                size_t len = 0;
+                if (small) {
+                    uint16_t h[kUnitCodes + 8];
+                    for (uint32_t k = 0; k < num_codes; k++) {
+                        h[len] = codes[k];
+                        len += (code_parity[k] >> b) & 1u;
+                    }
+                    if (len <= 7) {
+                        std::fill(h + len, h + 8, (uint16_t)kSymNone);
+                        if (obs_parity >> b & 1u) {
+                            h[7] = obs_code;
+                            len++;
+                        }
+                        std::memcpy(t.lists.entries.data() + at, h, 16);
+                        count += len;
+                        continue;
+                    }
+                    len = 0;
                 }
+                pattern.resize(flips.size());
+                for (const Flip &f : flips) {
+                    pattern[len] = f.id;
+                    len += (size_t)__builtin_parity(f.gens & b);
+                }
+                t.lists.put(at, pattern.data(), len, l.base);
+                count += len;
             }
         }
-        work += flips;
-        l.mean = (double)flips / std::max<uint32_t>(1, n * l.per_unit);
+        work += count;
+        l.mean = (double)count / std::max<uint32_t>(1, n * l.per_unit);
+    }
+
+    // The unit's flips as entry halfwords and one observable at most, each with the set of patterns of odd overlap; false
+    // where they are too many or too far apart for that.
+    bool code_unit(uint32_t base) {
+        num_codes = 0;
+        obs_parity = 0;
+        for (size_t k = 0; k < flips.size(); k++) {
+            uint32_t parity = 0;  // bit b: the overlap of pattern b
+            for (uint32_t g = 0; g < 4; g++) {
+                constexpr uint32_t kWith[4] = {0xAAAA, 0xCCCC, 0xF0F0, 0xFF00};  // patterns with generator g
+                parity ^= (flips[k].gens >> g) & 1u ? kWith[g] : 0;
+            }
+            const uint32_t id = flips[k].id;
+            if (id & kSymObs) {
+                if (k + 1 < flips.size() || (id & ~kSymObs) >= kSymLong) {
+                    return false;
+                }
+                obs_code = (uint16_t)id;
+                obs_parity = parity;
+            } else {
+                if (num_codes == kUnitCodes || id - base >= kSymLong) {
+                    return false;
+                }
+                codes[num_codes] = (uint16_t)(id - base);
+                code_parity[num_codes++] = parity;
+            }
+        }
+        return true;
+    }
+
+    // flips gains the outputs of a generator (bit `bit`).
+    void add_generator(const Set &s, uint32_t bit) {
+        if (s.empty()) {
+            return;
+        }
+        merged.resize(flips.size() + s.size());
+        size_t i = 0, j = 0, k = 0;
+        while (i < flips.size() && j < s.size()) {
+            const uint32_t a = flips[i].id, b = s[j];
+            merged[k++] = a < b ? flips[i] : Flip{b, a == b ? flips[i].gens | bit : bit};
+            i += a <= b;
+            j += b <= a;
+        }
+        for (; i < flips.size(); i++) {
+            merged[k++] = flips[i];
+        }
+        for (; j < s.size(); j++) {
+            merged[k++] = Flip{s[j], bit};
+        }
+        merged.resize(k);
+        flips.swap(merged);
     }
 
     // Noise word w fused into gate `op` (program.h), on the gate's instruction-order list.
@@ -283,8 +390,8 @@ class OutputAnalysis {
 
     struct State {
         std::vector<Set> xs, zs, pend;
-        uint64_t meas, det;
-        size_t occ;
+        uint64_t meas = 0, det = 0;
+        size_t occ = 0;
     };
 
     uint64_t slot(uint64_t count, uint64_t j) const {  // pend index of the j-th last of `count` results
@@ -306,7 +413,7 @@ class OutputAnalysis {
         return true;
     }
 
-    // `left` more iterations like the one that took state `b` to the present one.
+    // `left` more times the iterations that took state `b` to the present one.
     void repeat(const State &b, uint64_t left) {
         const uint64_t dmeas = b.meas - meas, ddet = b.det - det;
         const size_t docc = b.occ - occ;
@@ -342,16 +449,24 @@ class OutputAnalysis {
     }
 
     void loop(uint32_t lo, uint32_t hi, uint64_t reps) {
+        std::vector<State> before;  // of the last kPeriods iterations, the latest first
         for (uint64_t r = 0; r < reps && !failed; r++) {
             if (r >= kProbes || r + 1 == reps) {
                 walk(lo, hi);
                 continue;
             }
-            const State before{xs, zs, pend, meas, det, occ};
+            before.insert(before.begin(), State{xs, zs, pend, meas, det, occ});
+            before.resize(std::min<size_t>(before.size(), kPeriods), State());
             walk(lo, hi);
-            if (!failed && steady(before)) {
-                repeat(before, reps - 1 - r);
-                return;
+            for (size_t p = 0; p < before.size() && !failed; p++) {
+                const uint64_t left = reps - 1 - r, times = left / (p + 1);
+                if (times && steady(before[p])) {
+                    repeat(before[p], times);
+                    for (uint64_t k = times * (p + 1); k < left; k++) {
+                        walk(lo, hi);
+                    }
+                    return;
+                }
             }
         }
     }
@@ -379,30 +494,32 @@ class OutputAnalysis {
                     break;
                 }
                 case OP_1Q: {
-                    uint32_t image[4];
+                    Map m{2, {}};
                     for (uint32_t k = 0; k < 2; k++) {
                         uint32_t x = k == 0, z = k == 1;
                         rule1w(sub, x, z);
-                        image[k] = (x & 1u) | ((z & 1u) << 1);
+                        m.image[k] = (x & 1u) | ((z & 1u) << 1);
                     }
+                    m.classify();
                     for (uint32_t u = 0; u < n; u++) {
                         const uint32_t r = prog.pool[list + u];
                         Set *after[4] = {&xs[r], &zs[r], nullptr, nullptr};
-                        transpose(2, image, after);
+                        transpose(m, after);
                     }
                     break;
                 }
                 case OP_2Q: {
-                    uint32_t image[4];
+                    Map m{4, {}};
                     for (uint32_t k = 0; k < 4; k++) {
                         uint32_t v[4] = {k == 0, k == 1, k == 2, k == 3};
                         rule2(sub, v[0], v[1], v[2], v[3]);
-                        image[k] = (v[0] & 1u) | ((v[1] & 1u) << 1) | ((v[2] & 1u) << 2) | ((v[3] & 1u) << 3);
+                        m.image[k] = (v[0] & 1u) | ((v[1] & 1u) << 1) | ((v[2] & 1u) << 2) | ((v[3] & 1u) << 3);
                     }
+                    m.classify();
                     for (uint32_t u = 0; u < n; u++) {
                         const uint32_t r1 = prog.pool[list + 2 * u], r2 = prog.pool[list + 2 * u + 1];
                         Set *after[4] = {&xs[r1], &zs[r1], &xs[r2], &zs[r2]};
-                        transpose(4, image, after);
+                        transpose(m, after);
                     }
                     break;
                 }

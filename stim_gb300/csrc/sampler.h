@@ -139,7 +139,7 @@ inline bool write_in_place(std::initializer_list<std::pair<void *, uint64_t>> pa
 
 // Symptom sampling's tables on the device and the arguments that no call changes (symptoms.h).
 struct SymptomDevice {
-    DevBuf entries, longs, items, stages;
+    DevBuf data;  // items, stages, entries and long lists, one after another
     gfs::SymArgs args{};
     size_t nitems = 0;  // segments of a 128-shot block
     bool ready = false;
@@ -167,26 +167,33 @@ struct SymptomDevice {
         if (!planned || gfs::symptom_smem_bytes(stride, 0) > (size_t)200 << 10) {
             return;
         }
+        const size_t at_stages = plan.items.size() * sizeof(gfs::SymItem);
+        const size_t at_entries = at_stages + plan.stages.size() * sizeof(gfs::SymStage);
+        const size_t at_longs = at_entries + 4 * lists.entries.size();
         try {
-            upload(entries, lists.entries, device, stream);
-            upload(longs, lists.longs, device, stream);
-            upload(items, plan.items, device, stream);
-            upload(stages, plan.stages, device, stream);
-            ck(cudaStreamSynchronize(stream), "upload sync");
+            data.ensure(at_longs + 4 * lists.longs.size(), device);
         } catch (const CudaError &e) {
             if (e.code != cudaErrorMemoryAllocation) {
                 throw;
             }
             cudaGetLastError();
-            for (DevBuf *b : {&entries, &longs, &items, &stages}) {
-                b->release();
-            }
             return;
         }
-        args.entries = (const uint4 *)entries.p;
-        args.longs = (const uint32_t *)longs.p;
-        args.items = (const gfs::SymItem *)items.p;
-        args.stages = (const gfs::SymStage *)stages.p;
+        uint8_t *const base = (uint8_t *)data.p;
+        auto put = [&](size_t at, const void *src, size_t bytes) {
+            if (bytes) {
+                ck(cudaMemcpyAsync(base + at, src, bytes, cudaMemcpyHostToDevice, stream), "upload");
+            }
+        };
+        put(0, plan.items.data(), at_stages);
+        put(at_stages, plan.stages.data(), at_entries - at_stages);
+        put(at_entries, lists.entries.data(), at_longs - at_entries);
+        put(at_longs, lists.longs.data(), 4 * lists.longs.size());
+        ck(cudaStreamSynchronize(stream), "upload sync");
+        args.items = (const gfs::SymItem *)base;
+        args.stages = (const gfs::SymStage *)(base + at_stages);
+        args.entries = (const uint4 *)(base + at_entries);
+        args.longs = (const uint32_t *)(base + at_longs);
         args.nstages = (uint32_t)plan.stages.size();
         args.tables = (const uint32_t *)tables;
         args.chans = (const gfs::DevChan *)chans;

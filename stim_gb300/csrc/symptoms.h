@@ -55,28 +55,33 @@ struct SymLists {
 
     // Appends the sorted list s[0..n) of detectors (at least `base`) and kSymObs | observables.
     void add(const uint32_t *s, size_t n, uint32_t base) {
+        entries.resize(entries.size() + 4);
+        put(entries.size() - 4, s, n, base);
+    }
+
+    // The same as entries[at..at + 4).
+    void put(size_t at, const uint32_t *s, size_t n, uint32_t base) {
         uint32_t h[8] = {kSymNone, kSymNone, kSymNone, kSymNone, kSymNone, kSymNone, kSymNone, kSymNone};
-        size_t nd = 0, no = 0;
-        bool fits = true;
-        for (size_t j = 0; j < n; j++) {
-            const uint32_t id = s[j];
-            if (id & kSymObs) {
-                fits &= no++ == 0 && (id & ~kSymObs) < kSymLong;
-                h[7] = id & ~kSymObs;
-            } else {
-                fits &= nd < 7 && id - base < kSymLong;
-                h[nd < 7 ? nd++ : 6] = id - base;
-            }
-        }
+        const bool obs = n && (s[n - 1] & kSymObs);
+        const size_t nd = n - obs;
+        bool fits = nd <= 7 && !(nd && ((s[nd - 1] & kSymObs) || s[nd - 1] - base >= kSymLong));
+        fits &= !obs || (s[nd] & ~kSymObs) < kSymLong;
         if (fits) {
-            const size_t at = entries.size();
-            entries.resize(at + 4);
+            for (size_t j = 0; j < nd; j++) {
+                h[j] = s[j] - base;
+            }
+            if (obs) {
+                h[7] = s[nd] & ~kSymObs;
+            }
             for (int j = 0; j < 4; j++) {
                 entries[at + j] = h[2 * j] | (h[2 * j + 1] << 16);
             }
             return;
         }
-        entries.insert(entries.end(), {kSymLong, (uint32_t)longs.size(), (uint32_t)n, 0u});
+        entries[at] = kSymLong;
+        entries[at + 1] = (uint32_t)longs.size();
+        entries[at + 2] = (uint32_t)n;
+        entries[at + 3] = 0;
         for (size_t j = 0; j < n; j++) {
             longs.push_back(s[j] & kSymObs ? s[j] : s[j] - base);
         }

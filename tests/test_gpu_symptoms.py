@@ -172,6 +172,16 @@ def test_error_models_screened(hits, mechanisms):
         np.testing.assert_array_equal(d, wd)
 
 
+def test_few_and_many_blocks_of_a_large_error_model():
+    # The d=25 model (82 K segments a block) changes kernels between 96 and 97 blocks; one stream through either.
+    a, b = (stim_gb300.DetectorErrorModel(dem_text("surface_rz_d25")).compile_sampler(seed=3) for _ in range(2))
+    for shots in (96 * 128, 96 * 128 + 1):
+        d, o, _ = a.sample(shots, bit_packed=True)
+        parts = [b.sample(n, bit_packed=True) for n in (50 * 128, shots - 50 * 128)]
+        np.testing.assert_array_equal(d, np.concatenate([p[0] for p in parts]))
+        np.testing.assert_array_equal(o, np.concatenate([p[1] for p in parts]))
+
+
 @pytest.mark.parametrize("qubits,shots", [(2, 1), (64, 129), (65, 1000), (128, 513), (130, 300), (300, 140)])
 def test_short_phases_around_two_items_a_thread(qubits, shots):
     # The lean frame kernel that works two phases ahead, against the generic one: circuits whose phases have fewer and more

@@ -34,6 +34,14 @@ HAND = {
     "far_apart": "R 0\n" + "R 1\nX_ERROR(0.01) 0\nM 1\nDETECTOR rec[-1]\n" * 400 + "M 0\nDETECTOR rec[-1]\n",
     "quiet_stretch": "R 0 1\nX_ERROR(0.1) 0\nM 0\nDETECTOR rec[-1]\nREPEAT 9000 {\n M 1\n DETECTOR rec[-1]\n}\n"
                      "X_ERROR(0.1) 1\nM 1\nDETECTOR rec[-1]\n",
+    # Bodies that give back the state after two and after three iterations, with one and two iterations left over.
+    "period_two": "R 0 1\nREPEAT 30 {\n X_ERROR(0.1) 0\n Z_ERROR(0.2) 1\n SWAP 0 1\n H 1\n M(0.1) 0\n}\nR 0 1\n"
+                  "REPEAT 21 {\n X_ERROR(0.1) 0 1\n SWAP 0 1\n MR 0\n DETECTOR rec[-1]\n DEPOLARIZE2(0.1) 0 1\n}\n"
+                  "M 1\nOBSERVABLE_INCLUDE(1) rec[-1]\n",
+    "period_three": "R 0 1 2\nM 0\nREPEAT 40 {\n DEPOLARIZE1(0.1) 0 1 2\n SWAP 0 1 1 2\n MR(0.2) 0\n DETECTOR rec[-1] rec[-2]\n}\n"
+                    "M 1 2\nOBSERVABLE_INCLUDE(0) rec[-1] rec[-2]\n",
+    "period_five": "R 0 1 2 3 4\nREPEAT 33 {\n DEPOLARIZE1(0.1) 0 1 2 3 4\n SWAP 0 1 1 2 2 3 3 4\n M(0.2) 0\n"
+                   " DETECTOR rec[-1]\n}\nM 1 2\nOBSERVABLE_INCLUDE(0) rec[-1] rec[-2]\n",
     "noiseless": "R 0\nM 0\nDETECTOR rec[-1]\n",
 }
 
