@@ -335,16 +335,20 @@ void sample(gfs_dem *d, uint64_t shots, uint32_t flags, uint8_t *dets, uint64_t 
             tr((const uint4 *)d->err_buf[k].p, E, eout, erow);
         }
     };
+    HostPages pages(d->writes_host, {dets, shots * dstride}, {obs, shots * ostride}, {errs, shots * estride});
     auto copy_out = [&](int k, uint64_t done, uint64_t cs) {
         cudaStream_t st = d->streams[k];
         uint8_t *dout = (uint8_t *)d->out_buf[k].p, *oout = dout + chunk * drow, *eout = oout + chunk * orow;
         if (dets && drow) {
+            pages.before_copy(dets + done * dstride, (cs - 1) * dstride + drow);
             copy2d(dets + done * dstride, dstride, dout, drow, drow, cs, cudaMemcpyDeviceToHost, st, "copy dets");
         }
         if (obs && orow) {
+            pages.before_copy(obs + done * ostride, (cs - 1) * ostride + orow);
             copy2d(obs + done * ostride, ostride, oout, orow, orow, cs, cudaMemcpyDeviceToHost, st, "copy obs");
         }
         if (want_errs && erow) {
+            pages.before_copy(errs + done * estride, (cs - 1) * estride + erow);
             copy2d(errs + done * estride, estride, eout, erow, erow, cs, cudaMemcpyDeviceToHost, st, "copy errs");
         }
     };

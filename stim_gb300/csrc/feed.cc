@@ -100,6 +100,7 @@ void sample_for_decoder(gfs_sampler *s, uint64_t shots, const uint8_t *mask, uin
     // counts of chunk n - 1, whose kept rows leave on the copy stream (with page-locked destinations beside chunk n's
     // kernels), so the device always has a chunk to work on.  A slot is reused once its copy has ended.
     uint64_t kept_total = 0, dropped = 0, events = 0;
+    HostPages pages(s->writes_host, {dets, shots * dstride}, {obs, shots * ostride});
     bool copying[2] = {false, false};
     auto finish = [&](int k) {
         const gfs::FeedArgs &a = args[k];
@@ -112,10 +113,10 @@ void sample_for_decoder(gfs_sampler *s, uint64_t shots, const uint8_t *mask, uin
         const uint8_t *src = nmask ? a.cdets : a.dets;
         const uint8_t *osrc = nmask ? a.cobs : a.obs;
         if (dets && drow && kept) {
-            s->copy_rows(dets + kept_total * dstride, dstride, src, drow, drow, kept, "copy dets");
+            s->copy_rows(dets + kept_total * dstride, dstride, src, drow, drow, kept, pages, "copy dets");
         }
         if (obs && orow && kept) {
-            s->copy_rows(obs + kept_total * ostride, ostride, osrc, orow, orow, kept, "copy obs");
+            s->copy_rows(obs + kept_total * ostride, ostride, osrc, orow, orow, kept, pages, "copy obs");
         }
         ck(cudaEventRecord(s->pev[k][3], s->copy_stream), "event");
         copying[k] = true;

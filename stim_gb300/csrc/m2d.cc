@@ -30,7 +30,7 @@ struct gfs_m2d {
     std::vector<uint8_t> expect;
     DevBuf d_off, d_idx, d_expect, d_lists, sweep_in, sweep_rows;
     bool small = false;  // every measurement index fits the short lists of launch_convert
-    bool reads_host = false;  // the device reads pageable host memory through the host's page tables
+    bool reads_host = false;  // the device reads and writes pageable host memory through the host's page tables
     // Three pipeline slots: chunk k runs on slot k % 3 (its own stream and buffers), so chunk k's device->host
     // copy overlaps chunk k + 1's host->device copy and kernels, and chunk k + 2's copy in need not wait for it.
     static constexpr int kSlots = 3;
@@ -243,7 +243,7 @@ void convert(gfs_m2d *m, uint64_t shots, const uint8_t *meas, uint64_t meas_stri
     // copies, 468 without).  From page-locked memory the copy engine is the faster one, except for small calls, which a
     // copy only delays (d=3, 1,024 shots: 31 us).
     const bool direct = fused && m->reads_host && meas_stride == mrow && ((uintptr_t)meas & 15) == 0 &&
-                        (shots * mrow <= (1u << 20) || !gfs_sampler::page_locked({meas}));
+                        (shots * mrow <= (1u << 20) || !page_locked({meas}));
     // Chunks of up to 2^16 shots, fewer when a circuit's rows are large (about 1 GiB of device buffers).
     const uint64_t per_block = (M + D + O) * 16 + 128 * (mrow + drow + orow);
     uint64_t cb = std::max<uint64_t>(1, std::min<uint64_t>(512, ((uint64_t)1 << 30) / std::max<uint64_t>(1, per_block)));
@@ -276,7 +276,9 @@ void convert(gfs_m2d *m, uint64_t shots, const uint8_t *meas, uint64_t meas_stri
     auto compute = [&](int k, uint64_t done, uint64_t cs, const uint4 *base_dets, const uint4 *base_obs) {
         cudaStream_t st = m->streams[k];
         const uint64_t nblk = (cs + 127) / 128;
-        if (!direct) {
+        if (direct) {
+            populate(meas + done * mrow, cs * mrow, false);
+        } else {
             copy2d(m->in_buf[k].p, mrow, meas + done * meas_stride, meas_stride, mrow, cs, cudaMemcpyHostToDevice, st,
                    "copy measurements");
         }
@@ -335,13 +337,16 @@ void convert(gfs_m2d *m, uint64_t shots, const uint8_t *meas, uint64_t meas_stri
             tr(ot, O, nullptr, 0, oout, orow);
         }
     };
+    HostPages pages(m->reads_host, {dets, shots * dstride}, {obs, shots * ostride});
     auto copy_out = [&](int k, uint64_t done, uint64_t cs) {
         cudaStream_t st = m->streams[k];
         uint8_t *dout = (uint8_t *)m->out_buf[k].p, *oout = dout + chunk * drow;
         if (dets && drow) {
+            pages.before_copy(dets + done * dstride, (cs - 1) * dstride + drow);
             copy2d(dets + done * dstride, dstride, dout, drow, drow, cs, cudaMemcpyDeviceToHost, st, "copy dets");
         }
         if (obs && orow) {
+            pages.before_copy(obs + done * ostride, (cs - 1) * ostride + orow);
             copy2d(obs + done * ostride, ostride, oout, orow, orow, cs, cudaMemcpyDeviceToHost, st, "copy obs");
         }
     };

@@ -111,12 +111,104 @@ inline bool device_shares_host_memory(int device) {
     return access != 0 && tables != 0;
 }
 
+// The pages of [p, p + bytes) in pieces of up to 1,024: f(address, pages, bytes a page, a byte for each page whose bit 0 is
+// set where it has memory), until f returns false.  Nothing where the system cannot tell.
+template <typename F>
+inline void each_page_piece(const void *p, uint64_t bytes, F f) {
+    static const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+    const uintptr_t end = ((uintptr_t)p + bytes + page - 1) & ~(page - 1);
+    unsigned char there[1024];
+    for (uintptr_t lo = (uintptr_t)p & ~(page - 1); lo < end;) {
+        const uintptr_t n = std::min<uintptr_t>(1024, (end - lo) / page);
+        if (mincore((void *)lo, n * page, there) != 0 || !f(lo, n, page, there)) {
+            return;
+        }
+        lo += n * page;
+    }
+}
+
+// Gives pageable host memory that the device is about to write (or read) the pages that it lacks.  Pages that nothing has
+// touched yet would fault one by one, from the device or the copy engine (64 KiB: 21 us each, 3 here; 322 MB into new
+// arrays: 68-128 ms, 14 populated).
+inline void populate(const void *p, uint64_t bytes, bool write = true) {
+#ifdef MADV_POPULATE_WRITE
+    if (!p || bytes <= 16384) {
+        return;
+    }
+    each_page_piece(p, bytes, [&](uintptr_t lo, uintptr_t n, uintptr_t page, const unsigned char *there) {
+        uintptr_t first = 0, past = n;
+        while (first < n && (there[first] & 1)) {
+            first++;
+        }
+        while (past > first && (there[past - 1] & 1)) {
+            past--;
+        }
+        if (past > first) {  // advice: errors do not matter
+            madvise((void *)(lo + first * page), (past - first) * page, write ? MADV_POPULATE_WRITE : MADV_POPULATE_READ);
+        }
+        return true;
+    });
+#endif
+}
+
+// Whether every non-null host destination is page-locked.
+inline bool page_locked(std::initializer_list<const void *> ptrs) {
+    for (const void *p : ptrs) {
+        if (!p) {
+            continue;
+        }
+        cudaPointerAttributes at{};
+        if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (at.type != cudaMemoryTypeHost) {
+            return false;
+        }
+    }
+    return true;
+}
+
+// A call's host destinations (address and bytes; null: none), populated piece by piece before copies into them.  Whether
+// any page is missing is asked once, before the first copy, beside the first chunks' kernels (10 ns a page: per chunk it
+// delayed every copy, d=25 error model 1.63 -> 1.67 ms per 2^17 shots).
+class HostPages {
+   public:
+    using Part = std::pair<const void *, uint64_t>;
+    HostPages(bool shared, Part a, Part b = {}, Part c = {})
+        : parts{a, b, c}, missing(shared && !page_locked({a.first, b.first, c.first})) {
+    }
+
+    void before_copy(const void *p, uint64_t bytes) {
+        if (missing && !asked) {
+            asked = true;
+            missing = false;
+            for (const Part &d : parts) {
+                if (d.first) {
+                    each_page_piece(d.first, d.second, [&](uintptr_t, uintptr_t n, uintptr_t, const unsigned char *there) {
+                        for (uintptr_t k = 0; k < n; k++) {
+                            missing |= !(there[k] & 1);
+                        }
+                        return !missing;
+                    });
+                }
+            }
+        }
+        if (missing) {
+            populate(p, bytes);
+        }
+    }
+
+   private:
+    Part parts[3];
+    bool missing, asked = false;
+};
+
 // Whether a call's results (address and bytes; null: none) are small enough for its last kernel to write them straight to
 // host memory instead of staging and copying them: each copy costs more latency than a small call's kernels (1,024 shots
 // of d=3: 56 us, 28 without).  Symptom sampling writes 4 MiB so (d=11, 2.6 MB: 68 us, 61 in place; 10.8 MB: 115 and 184),
 // unpacked rows, whose bytes are mostly expansion, 8 (d=25 repetition code, 6.3 MB: 104 and 87); other kernels 64 KiB (their
-// transposes write rows in 2-byte units; 6.6 MB of d=9 records: 253 and 322).  Pages that nothing has touched yet are
-// populated first: the device would fault on them one by one (21 us each, 3 here).
+// transposes write rows in 2-byte units; 6.6 MB of d=9 records: 253 and 322).
 inline bool write_in_place(std::initializer_list<std::pair<void *, uint64_t>> parts, bool symptoms, bool packed) {
     uint64_t bytes = 0;
     for (const auto &p : parts) {
@@ -125,13 +217,9 @@ inline bool write_in_place(std::initializer_list<std::pair<void *, uint64_t>> pa
     if (bytes > (symptoms ? (packed ? (uint64_t)4 << 20 : (uint64_t)8 << 20) : (uint64_t)64 << 10)) {
         return false;
     }
-    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
     for (const auto &p : parts) {
-        if (p.first && p.second > 16384) {
-            const uintptr_t lo = (uintptr_t)p.first & ~(page - 1);
-#ifdef MADV_POPULATE_WRITE
-            madvise((void *)lo, (uintptr_t)p.first + p.second - lo, MADV_POPULATE_WRITE);  // advice: errors do not matter
-#endif
+        if (p.first) {
+            populate(p.first, p.second);
         }
     }
     return true;
@@ -867,7 +955,8 @@ struct gfs_sampler {
     // Device->host copy of `rows` rows of `width` bytes on copy_stream: one linear copy when both sides are
     // contiguous (a strided copy of narrow rows moves them one by one).
     void copy_rows(uint8_t *dst, uint64_t dpitch, const uint8_t *src, uint64_t spitch, uint64_t width, uint64_t rows,
-                   const char *what) {
+                   HostPages &pages, const char *what) {
+        pages.before_copy(dst, (rows - 1) * dpitch + width);
         if (dpitch == width && spitch == width) {
             ck(cudaMemcpyAsync(dst, src, width * rows, cudaMemcpyDeviceToHost, copy_stream), what);
         } else {
@@ -879,25 +968,8 @@ struct gfs_sampler {
     // staging buffer; its device->host copy runs on `copy_stream` while chunk k + 1's kernels run.  The
     // copy of chunk k is issued only after chunk k + 1's kernels are queued, because a copy into pageable
     // memory may hold the calling thread until it completes.
-    // Whether every non-null host destination is page-locked: then a chunk's copy can be queued as soon as its
-    // kernels are, because cudaMemcpyAsync into page-locked memory returns at once.
-    static bool page_locked(std::initializer_list<const void *> ptrs) {
-        for (const void *p : ptrs) {
-            if (!p) {
-                continue;
-            }
-            cudaPointerAttributes at{};
-            if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-                cudaGetLastError();
-                return false;
-            }
-            if (at.type != cudaMemoryTypeHost) {
-                return false;
-            }
-        }
-        return true;
-    }
-
+    // Page-locked destinations (`eager`): a chunk's copy is queued as soon as its kernels are, because the call returns at
+    // once.
     template <typename Produce, typename Copy>
     void host_pipeline(uint64_t shots, uint64_t slot_row_bytes, Produce produce, Copy copy, bool eager = false,
                        bool symptoms = false) {
@@ -1074,6 +1146,7 @@ struct gfs_sampler {
         const bool direct = !device_out && writes_host &&
                             gfs_rt::write_in_place({{dets, shots * dstride}, {obs, shots * ostride}}, symptoms, packed);
         if (!device_out && !direct) {
+            HostPages pages(writes_host, {dets, shots * dstride}, {obs, shots * ostride});
             // Staging rows use the caller's stride when its rows are contiguous, so that each chunk leaves in
             // one linear copy; otherwise they are padded to 32 bytes and copied row by row.
             const uint64_t ds = dstride == drow ? drow : pad32(drow), os = ostride == orow ? orow : pad32(orow);
@@ -1088,10 +1161,10 @@ struct gfs_sampler {
                 },
                 [&](uint64_t done, uint64_t cs, uint8_t *buf) {
                     if (dets && drow) {
-                        copy_rows(dets + done * dstride, dstride, buf, ds, drow, cs, "copy dets");
+                        copy_rows(dets + done * dstride, dstride, buf, ds, drow, cs, pages, "copy dets");
                     }
                     if (obs && orow) {
-                        copy_rows(obs + done * ostride, ostride, buf + cs * ds, os, orow, cs, "copy obs");
+                        copy_rows(obs + done * ostride, ostride, buf + cs * ds, os, orow, cs, pages, "copy obs");
                     }
                 },
                 page_locked({dets, obs}), symptoms);
@@ -1216,6 +1289,7 @@ struct gfs_sampler {
             return;
         }
         const uint64_t rs = stride == row ? row : pad32(row);
+        HostPages pages(writes_host, {out, shots * stride});
         host_pipeline(
             shots, rs,
             [&](uint64_t, uint64_t cs, uint8_t *buf) {
@@ -1223,7 +1297,7 @@ struct gfs_sampler {
             },
             [&](uint64_t done, uint64_t cs, uint8_t *buf) {
                 if (row) {
-                    copy_rows(out + done * stride, stride, buf, rs, row, cs, "copy meas");
+                    copy_rows(out + done * stride, stride, buf, rs, row, cs, pages, "copy meas");
                 }
             },
             page_locked({out}));
