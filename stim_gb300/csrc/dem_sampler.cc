@@ -235,7 +235,7 @@ void sample(gfs_dem *d, uint64_t shots, uint32_t flags, uint8_t *dets, uint64_t 
     const bool few_blocks = packed ? 512 * sample_blocks + (32u << 10) < segments : 192 * sample_blocks + (24u << 10) < segments;
     const bool symptoms = d->sym.ready && !want_errs && !replay && !few_blocks;
     if (symptoms && d->writes_host && shots &&
-        gfs_rt::write_in_place({{dets, shots * dstride}, {obs, shots * ostride}}, true, packed)) {
+        gfs_rt::write_in_place({{dets, shots * dstride}, {obs, shots * ostride}}, d->sym.in_place(packed, drow, dstride))) {
         gfs::SymArgs a = d->sym.call(shots, d->next_block, flags & GFS_BIT_PACKED, drow ? dets : nullptr, dstride,
                                      orow ? obs : nullptr, ostride, (shots + 127) / 128, d->num_sms);
         a.host = 1;

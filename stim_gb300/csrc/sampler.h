@@ -206,15 +206,14 @@ class HostPages {
 
 // Whether a call's results (address and bytes; null: none) are small enough for its last kernel to write them straight to
 // host memory instead of staging and copying them: each copy costs more latency than a small call's kernels (1,024 shots
-// of d=3: 56 us, 28 without).  Symptom sampling writes 4 MiB so (d=11, 2.6 MB: 68 us, 61 in place; 10.8 MB: 115 and 184),
-// unpacked rows, whose bytes are mostly expansion, 8 (d=25 repetition code, 6.3 MB: 104 and 87); other kernels 64 KiB (their
-// transposes write rows in 2-byte units; 6.6 MB of d=9 records: 253 and 322).
-inline bool write_in_place(std::initializer_list<std::pair<void *, uint64_t>> parts, bool symptoms, bool packed) {
+// of d=3: 56 us, 28 without): up to SymptomDevice::in_place, other kernels 64 KiB (their transposes write rows in 2-byte units;
+// 6.6 MB of d=9 records: 253 us copied, 322 in place).
+inline bool write_in_place(std::initializer_list<std::pair<void *, uint64_t>> parts, uint64_t most = (uint64_t)64 << 10) {
     uint64_t bytes = 0;
     for (const auto &p : parts) {
         bytes += p.first ? p.second : 0;
     }
-    if (bytes > (symptoms ? (packed ? (uint64_t)4 << 20 : (uint64_t)8 << 20) : (uint64_t)64 << 10)) {
+    if (bytes > most) {
         return false;
     }
     for (const auto &p : parts) {
@@ -292,6 +291,14 @@ struct SymptomDevice {
         args.stride = stride;
         nitems = plan.items.size();
         ready = true;
+    }
+
+    // Bytes up to which results are written in place (write_in_place): 4 MiB of packed rows (d=11, 2.6 MB: 68 us copied, 61 in
+    // place; 10.8 MB: 115 and 184), 16 of short ones, which the kernel writes across rows (d=7, 5.6 MB: 103 and 67; d=5, 16.8 MB:
+    // 186 and 142), 8 of unpacked rows, whose bytes are mostly expansion (d=25 repetition code, 6.3 MB: 104 and 87).
+    uint64_t in_place(bool packed, uint64_t row, uint64_t stride) const {
+        const bool across = args.nstages == 1 && stride == row && row <= 127;
+        return (uint64_t)(packed ? (across ? 16 : 4) : 8) << 20;
     }
 
     // Kernel arguments for `cs` shots from stream block `block0` on into device rows.  `launch_blocks`: 128-shot blocks
@@ -1144,7 +1151,8 @@ struct gfs_sampler {
         reset_timings();
         const bool symptoms = symptoms_active(flags);
         const bool direct = !device_out && writes_host &&
-                            gfs_rt::write_in_place({{dets, shots * dstride}, {obs, shots * ostride}}, symptoms, packed);
+                            gfs_rt::write_in_place({{dets, shots * dstride}, {obs, shots * ostride}},
+                                                   symptoms ? sym.in_place(packed, drow, dstride) : (uint64_t)64 << 10);
         if (!device_out && !direct) {
             HostPages pages(writes_host, {dets, shots * dstride}, {obs, shots * ostride});
             // Staging rows use the caller's stride when its rows are contiguous, so that each chunk leaves in
@@ -1284,7 +1292,7 @@ struct gfs_sampler {
             ck(cudaMemcpyAsync(ref_bits.p, ref, (M + 7) / 8, cudaMemcpyHostToDevice, stream), "ref upload");
             dref = (const uint8_t *)ref_bits.p;
         }
-        if (writes_host && gfs_rt::write_in_place({{out, shots * stride}}, false, packed)) {
+        if (writes_host && gfs_rt::write_in_place({{out, shots * stride}})) {
             measurements_device(shots, flags, ref, out, stride);
             return;
         }

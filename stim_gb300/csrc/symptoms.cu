@@ -116,6 +116,12 @@ __host__ __device__ constexpr uint32_t threads(bool screen) {
     return screen ? kScreenThreads : kThreads;
 }
 
+// Packed rows up to these lengths are written across rows, in device memory (longer: bulk copies) and in host memory, where
+// partial words cost most (us, one row after another and across: d=3, 3 bytes, 2^20 shots, device 47 and 31, in place 322 and
+// 62; 10 bytes, 2^18 shots in place 271 and 63; 78 bytes, 2^15 shots in place 62 and 42; 42 bytes, 2^20 shots, device 100 and
+// 111).
+constexpr uint32_t kFlatDevice = 16, kFlatHost = 127;
+
 struct WarpQueues {
     uint2 hits[kQueue];  // output list; shot row << 16 | column of relative code 0
     uint2 cont[kQueue];  // work index; position of the last hit | iterations done << 16
@@ -304,6 +310,39 @@ __device__ __forceinline__ void write_packed(const SymArgs &a, const SymStage &s
     asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the rows may be changed
 }
 
+// Short packed rows one after another (`rb` bytes each, all outputs in the window): consecutive lanes write consecutive
+// aligned words of the CTA's rows, whichever rows those are, so that a warp's store is 128 whole bytes.
+__device__ __forceinline__ void write_flat(const SymArgs &a, const uint32_t *win, uint32_t rb, uint64_t shot0,
+                                           uint32_t nvalid, uint32_t dst0) {
+    uint8_t *const d = a.dets + shot0 * rb;
+    const int32_t mis = (int32_t)(dst0 & 3u), total = (int32_t)(nvalid * rb);
+    for (int32_t q = (int32_t)threadIdx.x; 4 * q < mis + total; q += (int32_t)blockDim.x) {
+        const int32_t o = 4 * q - mis;  // first byte of this word
+        uint32_t r = (uint32_t)max(o, 0) / rb, b = (uint32_t)max(o, 0) - r * rb;
+        const uint8_t *row = reinterpret_cast<const uint8_t *>(win + (size_t)r * a.stride) + (row_shift<true>(a, dst0, r) >> 3);
+        uint32_t v = 0;
+        if (o >= 0 && b + 4 <= rb) {
+            v = *reinterpret_cast<const uint32_t *>(row + b);  // a row's words are its destination's
+        } else {
+            for (int32_t k = max(-o, 0); k < 4 && o + k < total; k++) {
+                v |= (uint32_t)row[b] << (8 * k);
+                if (++b == rb) {
+                    b = 0;
+                    r++;
+                    row = reinterpret_cast<const uint8_t *>(win + (size_t)r * a.stride) + (row_shift<true>(a, dst0, r) >> 3);
+                }
+            }
+        }
+        if (o >= 0 && o + 4 <= total) {
+            *reinterpret_cast<uint32_t *>(d + o) = v;
+        } else {
+            for (int32_t k = max(-o, 0); k < 4 && o + k < total; k++) {
+                d[o + k] = (uint8_t)(v >> (8 * k));
+            }
+        }
+    }
+}
+
 // Unpacked rows, and rows of any kind in host memory (columns [c0, c1) of every shot): one warp per row, consecutive lanes
 // writing consecutive aligned 32-bit words, of four expanded bits or (a packed row's words are its destination's) as they
 // are; the partial words at the ends byte by byte.
@@ -406,7 +445,10 @@ __device__ __forceinline__ void sample_blocks(const SymArgs &a, uint32_t cta) {
             __syncthreads();
         }
         if (a.dets) {
-            if (PACKED && !a.host) {
+            const uint32_t rb = (c1 + 7) / 8;
+            if (PACKED && a.nstages == 1 && a.dets_stride == rb && rb <= (a.host ? kFlatHost : kFlatDevice)) {
+                write_flat(a, win, rb, shot0, nvalid, dst0);
+            } else if (PACKED && !a.host) {
                 write_packed(a, st, win, c1, shot0, nvalid, dst0, last);
             } else {
                 write_words<PACKED>(a, win, st.flush0, c1, shot0, nvalid, dst0, last);

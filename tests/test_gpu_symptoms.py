@@ -67,6 +67,32 @@ def test_destinations_at_any_alignment(name, packed):
         assert (got[offset + shots * (row + pad):] == 0xA5).all()
 
 
+@pytest.mark.parametrize("row", [1, 3, 15, 16, 17, 126, 127, 128])
+def test_short_rows_at_any_address(row):
+    # Rows around the lengths up to which the kernel writes across rows (16 bytes on the device, 127 in host memory), at
+    # addresses of every kind, with nothing written around them.
+    torch = pytest.importorskip("torch")
+    bits = 8 * row - 3
+    qs = " ".join(str(q) for q in range(bits))
+    c = stim_gb300.Circuit(f"R {qs}\nX_ERROR(0.2) {qs}\nM {qs}\n" + "".join(f"DETECTOR rec[-{k + 1}]\n" for k in range(bits)))
+    a, b = (c.compile_detector_sampler(seed=6) for _ in range(2))
+    b.set_noise_mode(1)
+    for shots, offset in ((1, 1), (127, 2), (129, 7), (1027, 16), (2000, 3)):
+        n = shots * row
+        want = b.sample(shots, bit_packed=True)
+        dev = torch.full((n + 64,), 0xA5, dtype=torch.uint8, device="cuda")
+        host = np.full(n + 64, 0xA5, dtype=np.uint8)
+        torch.cuda.synchronize()
+        position = a.stream_position()
+        _native.check(_native.lib().gfs_sample_detections_device(a._h, shots, _native.BIT_PACKED, dev.data_ptr() + offset, row, None, 0))
+        dev = dev.cpu().numpy()
+        a.set_stream_position(position)
+        a.sample(shots, bit_packed=True, dets_out=host[offset:offset + n].reshape(shots, row))
+        for got in (dev, host):
+            np.testing.assert_array_equal(got[offset:offset + n].reshape(shots, row), want)
+            assert (got[:offset] == 0xA5).all() and (got[offset + n:] == 0xA5).all()
+
+
 @pytest.mark.parametrize("p", [1e-7, 3e-6, 1e-5, 1e-4, 1e-3, 2.6e-3, 2.8e-3, 0.01, 0.05, 0.2, 0.6, 0.95])
 def test_gaps_at_any_probability(p):
     # 40 qubits: two whole segments and a partial one; X flips draw gaps only, depolarizing noise a choice per hit.
