@@ -176,7 +176,7 @@ class HostPages {
    public:
     using Part = std::pair<const void *, uint64_t>;
     HostPages(bool shared, Part a, Part b = {}, Part c = {})
-        : parts{a, b, c}, missing(shared && !page_locked({a.first, b.first, c.first})) {
+        : parts{a, b, c}, missing(shared) {
     }
 
     void before_copy(const void *p, uint64_t bytes) {
@@ -184,7 +184,7 @@ class HostPages {
             asked = true;
             missing = false;
             for (const Part &d : parts) {
-                if (d.first) {
+                if (d.first && d.second > 16384) {
                     each_page_piece(d.first, d.second, [&](uintptr_t, uintptr_t n, uintptr_t, const unsigned char *there) {
                         for (uintptr_t k = 0; k < n; k++) {
                             missing |= !(there[k] & 1);
@@ -193,6 +193,7 @@ class HostPages {
                     });
                 }
             }
+            missing = missing && !page_locked({parts[0].first, parts[1].first, parts[2].first});
         }
         if (missing) {
             populate(p, bytes);
