@@ -594,7 +594,8 @@ def run_gpu(args):
             "scaling": "weak", "vs_baseline": None, "dtype": "u32 bitwise",
             "data": "synthetic (reference-generated circuit, seeded shots)",
             "config": {"workload": "surface_code:rotated_memory_z d=25 r=25 p=1e-3", "shots_per_step": shots,
-                       "detectors": D, "observables": O, "launch_shape": sampler.launch_shape(),
+                       "detectors": D, "observables": O,
+                       "launch_shape": {"kernel": "symptom"} if symptoms else sampler.launch_shape(),
                        "l2": "outputs (2 GB/step) exceed L2; a 256 MiB buffer is also rewritten between steps",
                        "parallelism": f"replicas by shot range x{world}"},
             "p50_ms": statistics.median(step_ms), "p99_ms": sorted(step_ms)[-1],
@@ -944,8 +945,9 @@ def run_batched(args, local):
         "speedup": seq_s / bat_s, "timing": "host wall clock around a completed call, both forms (median)",
         "launch_shape": batch.launch_shape(), "autotune_best_frame_ms": tune_ms,
         "graph_launches": t["graph_launches"], "graph_builds": t["graph_builds"],
-        "note": "device-resident outputs; batched = one persistent frame-kernel launch + per-circuit transposes "
-                "in one CUDA graph; sequential = one gfs_sample_detections_device call per circuit",
+        "note": "device-resident outputs; batched = batched symptom launches (for circuits that need frames one persistent "
+                "frame-kernel launch + per-circuit transposes) in one CUDA graph; sequential = one "
+                "gfs_sample_detections_device call per circuit",
     }
 
 

@@ -185,7 +185,8 @@ gfs_status gfs_sampler_last_timings(const gfs_sampler *s, double *out4, uint64_t
 /*
  * Launch shape: blocks_per_cta in {1, 2, 4} (128-shot blocks held in one CTA's shared memory),
  * threads per CTA (multiple of 32, <= 256), grid CTAs (0 = one full wave of resident CTAs).
- * Fails when the circuit's state does not fit shared memory with that many blocks.
+ * Fails when the circuit's state does not fit shared memory with that many blocks.  A chosen shape also chooses the
+ * frame kernels for detection events that would otherwise be sampled by output lists (gfs_sampler_set_noise_mode).
  */
 gfs_status gfs_sampler_set_shape(gfs_sampler *s, int blocks_per_cta, int threads, int grid);
 gfs_status gfs_sampler_get_shape(const gfs_sampler *s, int *blocks_per_cta, int *threads, int *grid,
@@ -224,15 +225,16 @@ gfs_status gfs_sampler_set_stream_position(gfs_sampler *s, uint64_t shot);
 gfs_status gfs_sampler_get_stream_position(const gfs_sampler *s, uint64_t *shot);
 
 /*
- * Noise generation: 1 (default, -1 = automatic) draws every noise hit of a chunk in a separate kernel
- * into a list that the frame kernel then applies; 0 draws noise inside the frame kernel.  Results are
- * identical either way.  No counterpart in the reference.
+ * Noise generation: -1 (default) samples detection events by output lists where the circuit allows it (each noise hit
+ * flips its precomputed detectors and observables in one kernel, without frames), otherwise as 1; 1 draws every noise
+ * hit of a chunk in a separate kernel into a list that the frame kernel then applies; 0 draws noise inside the frame
+ * kernel.  Results are identical either way.  No counterpart in the reference.
  */
 gfs_status gfs_sampler_set_noise_mode(gfs_sampler *s, int mode);
 /*
- * Frame kernel for hit-list launches: 1 (default, -1 = automatic) the lean kernel when the program has a lean
- * phase list (no correlated errors, heralds or sweep feedback; compact unit lists; at most two loop levels),
- * 0 the generic kernel.  Results are identical either way.  gfs_sampler_get_frame_kernel reports which one the
+ * Frame kernel for hit-list launches (a choice other than -1 also keeps detection events from being sampled by output
+ * lists): 1 (-1 = automatic) the lean kernel when the program has a lean phase list (no correlated errors, heralds or
+ * sweep feedback; compact unit lists; at most two loop levels), 0 the generic kernel.  Results are identical either way.  gfs_sampler_get_frame_kernel reports which one the
  * next hit-list launch uses (1 lean, 0 generic).  No counterpart in the reference.
  */
 gfs_status gfs_sampler_set_frame_kernel(gfs_sampler *s, int kind);

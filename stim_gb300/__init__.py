@@ -212,6 +212,7 @@ class _SamplerBase:
 
     # -- tuning / introspection (no counterpart in the reference) --
     def set_launch_shape(self, blocks_per_cta: int, threads: int = 256, grid: int = 0):
+        """Shape of the frame kernels, which a chosen shape also selects for detection events."""
         check(lib().gfs_sampler_set_shape(self._h, blocks_per_cta, threads, grid))
 
     def launch_shape(self):
@@ -226,7 +227,7 @@ class _SamplerBase:
 
     def set_frame_kernel(self, kind: int):
         """Frame kernel of hit-list launches: -1 automatic, 0 generic, 1 lean when the program has a lean phase
-        list.  Results are identical."""
+        list; a choice also selects the frame kernels for detection events.  Results are identical."""
         check(lib().gfs_sampler_set_frame_kernel(self._h, int(kind)))
 
     def set_ring_placement(self, placement: int):
@@ -254,8 +255,8 @@ class _SamplerBase:
         return ms.value
 
     def set_noise_mode(self, mode: int):
-        """-1 automatic, 0 noise drawn inside the frame kernel, 1 noise drawn into hit lists by a separate
-        kernel.  Results are identical."""
+        """-1 automatic (detection events by output lists where the circuit allows it), 0 noise drawn inside the frame
+        kernel, 1 noise drawn into hit lists by a separate kernel.  Results are identical."""
         check(lib().gfs_sampler_set_noise_mode(self._h, int(mode)))
 
     def last_timings(self):

@@ -1,7 +1,9 @@
 // Batched frame sampling shared by the batch API (batch.cc) and the request server (serve.cc): a list of
 // entries (a lowered program on the device, a seed, a stream position, a shot count, destinations) is
-// planned into one work list of (entry, 128-shot slice) items, sampled by ONE persistent
-// batch_frame_kernel launch, and turned shot-major by one transpose per entry and output.
+// sampled by their output lists in up to four batched symptom launches (per shared-memory class, packed or not), which
+// write the rows as they are; the entries that need frames (or whose sampler chose a frame kernel) are planned into one
+// work list of (entry, 128-shot slice) items, sampled by ONE persistent batch_frame_kernel launch, and turned shot-major
+// by one transpose per entry and output.
 #pragma once
 
 #include <unordered_map>

@@ -4,9 +4,10 @@
 // DetectorErrorModel.compile_sampler(seed=...).sample(shots, bit_packed, return_errors,
 // recorded_errors_to_replay) (src/stim/simulators/dem_sampler.pybind.cc:40-80).  The reference draws every
 // error row with biased_randomize_bits over all shots and XORs it into its symptoms' rows.  Here the model is
-// parsed and grouped by probability once (dem.cc); a sample call runs, per chunk of 128-shot blocks, the
-// sampling kernel (errors walked under the counter-based contract, symptoms XORed into detector rows) and the
-// shot-major transposes.  Replayed errors take the converter's path instead: their rows are transposed in
+// parsed and grouped by probability once (dem.cc); a sample call runs symptom_kernel (symptoms.h: a block's rows in shared
+// memory, errors drawn under the counter-based contract, their symptoms XORed in), or, when the errors themselves are
+// wanted and for a few blocks of a large model, per chunk of 128-shot blocks, dem_sample_kernel (symptoms XORed into
+// detector rows in device memory) and the shot-major transposes.  Replayed errors take the converter's path instead: their rows are transposed in
 // and folded into the outputs (each output the XOR of the mechanisms that list it).
 #include "dem.h"
 #include "gfs_contract.h"

@@ -3,9 +3,9 @@
 // Replaces the sampling half of sinter's _CompiledStimThenDecodeSampler.sample
 // (glue/sample/src/sinter/_decoding/_stim_then_decode_sampler.py:170-190): detection events bit-packed with
 // separate observables (:171-175), the detection-event count (:178-181) and the postselection mask (:183-190).
-// Per chunk of shots: the frame and transpose kernels write dense shot-major rows into device buffers,
-// feed_popcount_kernel counts their set bits, and with a mask feed_flags / feed_scan / feed_compact drop the
-// postselected shots and pack the kept rows in shot order; only the kept rows are copied to the host, on the
+// Per chunk of shots: symptom sampling (or the frame and transpose kernels) writes dense shot-major rows into device
+// buffers, feed_popcount_kernel counts their set bits, and with a mask feed_flags / feed_scan / feed_rank / feed_gather
+// drop the postselected shots and pack the kept rows in shot order; only the kept rows are copied to the host, on the
 // copy stream while the next chunk is sampled into the other slot.
 #include "sampler.h"
 

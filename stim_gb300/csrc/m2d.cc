@@ -5,8 +5,9 @@
 // noiseless circuit once per batch with a frame simulator and XORs each detector's (and observable's)
 // referenced measurement rows, inverting a row when the reference sample's parity of those measurements is
 // 1.  Here the walk happens once, at creation: every output becomes a list of absolute measurement indices
-// plus an expectation bit (the reference sample's parity), uploaded to the device.  A conversion then runs
-// three kernels per chunk of shots: shot-major input bits into 128-shot measurement rows, the XOR fold, and
+// plus an expectation bit (the reference sample's parity), uploaded to the device.  Packed
+// records of circuits whose 128 shots fit shared memory are converted by one kernel (m2d_block.cu); the others go
+// through three per chunk of shots: shot-major input bits into 128-shot measurement rows, the XOR fold, and
 // the usual shot-major output transpose.
 //
 // Sweep bits: the reference's frame simulator turns sweep-controlled Paulis into extra flips of measurement

@@ -4,8 +4,8 @@
 // device: it keeps lowered circuits in a device-resident cache keyed by circuit text, cuts requests into
 // chunks of at most `max_chunk_shots` shots, and admits chunks first come first served into the next
 // batch while the batch's HBM footprint (detector-major scratch plus shot-major staging) stays within
-// its slot budget.  Two slots alternate: while one batch runs (one persistent batch_frame_kernel
-// launch, transposes, device->host copies, all on the slot's stream), the worker forms and launches the
+// its slot budget.  Two slots alternate: while one batch runs (batched symptom launches, and for circuits that need
+// frames one persistent batch_frame_kernel launch and transposes; device->host copies, all on the slot's stream), the worker forms and launches the
 // next one, so requests that arrive while others are on the GPU join as soon as a slot and its memory
 // free up, and the two batches overlap on the device.  A request's result depends only on (circuit,
 // seed, shot index) -- chunk k of a request samples the request's stream from shot k*max_chunk_shots --
