@@ -123,7 +123,6 @@ struct SymArgs {
     const uint32_t *longs;
     const SymItem *items;
     const SymStage *stages;
-    uint32_t nstages;
     const uint32_t *tables;
     const DevChan *chans;
     uint64_t seed;
@@ -133,6 +132,7 @@ struct SymArgs {
     uint32_t words;       // detector words per shot row in shared memory
     uint32_t stride;      // words per shot row, observables included (a multiple of four)
     uint32_t log_blocks;  // 128-shot blocks per CTA, log2
+    uint32_t nstages;
     // Shot-major outputs (null: not wanted); append: the observables follow the detectors in the detector rows.
     uint8_t *dets, *obs;
     uint64_t dets_stride, obs_stride;

@@ -8,25 +8,26 @@
 // One iteration of a warp draws 32 segments: one Philox call and two gap draws a lane, up to two hits (gap, choice, gap,
 // choice for a channel that draws its Pauli; a channel that does not uses two of the four draws as gaps).  Segments with
 // draws left wait in a queue of the warp until they fill an iteration, so every iteration but a stage's last few is
-// full; where few segments have a hit (error models), the first gap decides which are drawn at all.  Hits go to a second queue and are applied 32 at a time, one per lane, each list loaded one step before it is
-// applied.
+// full; where few segments have a hit (error models), the first gap decides which are drawn at all.  Hits go to a second
+// queue and are applied 32 at a time, one per lane, each list loaded one step before it is applied.
 //
-// What bounds it: instruction issue (d=25: 210 K warp instructions per block, a quarter of them Philox and gap
+// What bounds it: instruction issue (d=25: 203 K warp instructions per block, a quarter of them Philox and gap
 // arithmetic that the contract asks for; 0.55 of the issue slots used, the rest fixed latencies and barriers).  The output
 // alone would take 0.31 ms at d=25 (2.05 GB per 2^20 shots at 6.7 TB/s), the contract's Philox calls 0.18 ms (580 G
-// calls/s).  d=25, p=1e-3, 2^20 shots: 2.04 ms where noise, frame and transpose kernels took 7.81; d=11, p=5e-3: 0.58 ms
-// (2.22); d=13 colour code, p=1e-2, 200,001 shots: 0.25 ms (0.97).  On the way at d=25: hits applied as each lane draws
+// calls/s).  d=25, p=1e-3, 2^20 shots: 1.97 ms where noise, frame and transpose kernels took 7.81; d=11, p=5e-3: 0.56 ms
+// (2.22); d=13 colour code, p=1e-2, 200,001 shots: 0.24 ms (0.97).  On the way at d=25: hits applied as each lane draws
 // them, with the gap table for every draw, 5.2 ms; the float estimate of the gap instead of the table and prefetched
 // descriptors 3.7; the hit queue 2.9; rows written by bulk copies instead of word stores 2.46; queued segments instead of
 // lanes that refill one by one 2.36; hits queued behind the next items' loads 2.19; fewer gap instructions 2.12; items in
-// turn 2.04.
+// turn 2.04; nine warps a CTA instead of eight 1.97.
 #include "frame_device.cuh"
 
 namespace gfs {
 
 namespace {
 
-// The position a gap draw leads to (as gfs_hit_after_draw; `trials` or more: past the segment), without the gap table where the float estimate decides.
+// The position a gap draw leads to (as gfs_hit_after_draw; `trials` or more: past the segment), without the gap table
+// where the float estimate decides.
 // e = log2(u / 2^32) / log2(1 - p) has G(u) = floor(e) unless e is close to an integer.  With c = -1 / log2(1 - p), the
 // error of e is below 3.6e-7 e (__log2f outside (0.5, 2): 2 ulp; the factor c and the product: one rounding each) plus
 // 4.3e-7 c (the conversion of u: 2^-24 relative; __log2f inside (0.5, 2): 2^-22; for u >= 2^24 the table's rounding to
@@ -109,8 +110,12 @@ __device__ __forceinline__ void flip_outputs(const SymArgs &a, uint32_t *row, ui
 // The screening variant (error models of large codes: 82,000 segments a block, one in seven with a hit) has work for more
 // warps: d=25, 268 blocks, 256 / 384 / 512 threads 277 / 227 / 221 us, 345 without screening.
 constexpr uint32_t kScreenThreads = 512;
-constexpr uint32_t kThreads = 256;  // per CTA (d=25: 320 threads 1.98 ms for 2.04, but d=11 0.64 for 0.58)
-constexpr uint32_t kQueue = 64;     // hits, and segments with draws left, a warp can hold: under 32 left over, 32 more
+// Nine warps: three CTAs with a 124-word window and nine warps' queues fill an SM's shared memory to the byte (us, 2^19 shots,
+// 256 / 288 / 320 / 352 threads: d=25 1,043 / 1,005 / 1,157 / 1,274, d=19, p=5e-3 1,498 / 1,418 / 1,615 / 1,720, d=13, whole
+// rows, 162 / 157 / 171 / 181; 320 with 116 words: d=25 1,015, d=19 1,486).
+constexpr uint32_t kThreads = 288;
+constexpr uint32_t kBatchThreads = 256;  // small codes among large ones (32 codes: 543 us, 555 with 288)
+constexpr uint32_t kQueue = 63;  // hits, and segments with draws left, a warp can hold: 31 left over, 32 more
 
 __host__ __device__ constexpr uint32_t threads(bool screen) {
     return screen ? kScreenThreads : kThreads;
@@ -129,7 +134,7 @@ struct WarpQueues {
 
 // Draws the stage's items: work index j is item item0 + j / blocks of the CTA's block j % blocks; the warps take 32
 // consecutive indices in turn (from a shared counter instead: 2.12 ms for 2.04).
-template <bool PACKED, bool SCREEN>
+template <bool PACKED, bool SCREEN, uint32_t THREADS>
 __device__ __forceinline__ void draw_stage(const SymArgs &a, const SymStage &st, uint32_t *win, WarpQueues &q,
                                            uint32_t block0, uint32_t nblk, uint32_t dst0) {
     const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
@@ -196,7 +201,7 @@ __device__ __forceinline__ void draw_stage(const SymArgs &a, const SymStage &st,
             act = j < total && (j & bmask) < nblk;
             lo = flo;
             hi = fhi;
-            cur += threads(SCREEN);
+            cur += THREADS;
             fetch();
             if (SCREEN) {
                 // Most segments have no hit and end here, after their first gap; those with one are queued and drawn whole, by
@@ -411,10 +416,10 @@ __device__ __forceinline__ void next_window(const SymArgs &a, const SymStage &st
 }
 
 // Samples CTA `cta`'s blocks from the circuit's start to its end.
-template <bool PACKED, bool SCREEN>
+template <bool PACKED, bool SCREEN, uint32_t THREADS>
 __device__ __forceinline__ void sample_blocks(const SymArgs &a, uint32_t cta) {
     extern __shared__ __align__(16) uint32_t win[];  // [shot][stride]: detector words, then observable words
-    __shared__ WarpQueues queue[threads(SCREEN) / 32];
+    __shared__ WarpQueues queue[THREADS / 32];
     const uint32_t tid = threadIdx.x, nt = blockDim.x;
     const uint32_t rows = GFS_BLOCK_SHOTS << a.log_blocks;
     const uint64_t blk0 = (uint64_t)cta << a.log_blocks, shot0 = blk0 * GFS_BLOCK_SHOTS;
@@ -427,7 +432,7 @@ __device__ __forceinline__ void sample_blocks(const SymArgs &a, uint32_t cta) {
     __syncthreads();
     for (uint32_t k = 0; k < a.nstages; k++) {
         const SymStage st = a.stages[k];
-        draw_stage<PACKED, SCREEN>(a, st, win, queue[tid >> 5], (uint32_t)(a.block0 + blk0), nblk, dst0);
+        draw_stage<PACKED, SCREEN, THREADS>(a, st, win, queue[tid >> 5], (uint32_t)(a.block0 + blk0), nblk, dst0);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the rows will be read by bulk copies
         __syncthreads();
         const bool last = k + 1 == a.nstages;
@@ -456,7 +461,7 @@ __device__ __forceinline__ void sample_blocks(const SymArgs &a, uint32_t cta) {
         }
         if (!last) {
             __syncthreads();
-            next_window<threads(SCREEN)>(a, st, win, rows);
+            next_window<THREADS>(a, st, win, rows);
             __syncthreads();
         }
     }
@@ -471,11 +476,11 @@ __device__ __forceinline__ void sample_blocks(const SymArgs &a, uint32_t cta) {
 
 template <bool PACKED, bool SCREEN>
 __global__ void __launch_bounds__(threads(SCREEN)) symptom_kernel(const SymArgs a) {
-    sample_blocks<PACKED, SCREEN>(a, blockIdx.x);
+    sample_blocks<PACKED, SCREEN, threads(SCREEN)>(a, blockIdx.x);
 }
 
 template <bool PACKED>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kBatchThreads)
     batch_symptom_kernel(const SymArgs *entries, const uint32_t *prefix, uint32_t n) {
     __shared__ SymArgs a;
     uint32_t lo = 0, hi = n;  // last j with prefix[j] <= blockIdx.x
@@ -493,7 +498,7 @@ __global__ void __launch_bounds__(kThreads)
         reinterpret_cast<uint32_t *>(&a)[threadIdx.x] = __ldg(reinterpret_cast<const uint32_t *>(entries + lo) + threadIdx.x);
     }
     __syncthreads();
-    sample_blocks<PACKED, false>(a, blockIdx.x - __ldg(prefix + lo));
+    sample_blocks<PACKED, false, kBatchThreads>(a, blockIdx.x - __ldg(prefix + lo));
 }
 
 template <bool PACKED, bool SCREEN>
@@ -515,7 +520,7 @@ cudaError_t launch_batch(const SymArgs *entries, const uint32_t *prefix, uint32_
     if (e != cudaSuccess) {
         return e;
     }
-    batch_symptom_kernel<PACKED><<<grid, kThreads, smem, stream>>>(entries, prefix, n);
+    batch_symptom_kernel<PACKED><<<grid, kBatchThreads, smem, stream>>>(entries, prefix, n);
     return cudaGetLastError();
 }
 
