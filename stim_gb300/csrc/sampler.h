@@ -176,7 +176,7 @@ class HostPages {
    public:
     using Part = std::pair<const void *, uint64_t>;
     HostPages(bool shared, Part a, Part b = {}, Part c = {})
-        : parts{a, b, c}, missing(shared) {
+        : parts{a, b, c}, missing(shared && (a.first ? a.second : 0) + (b.first ? b.second : 0) + (c.first ? c.second : 0) > kAsk) {
     }
 
     void before_copy(const void *p, uint64_t bytes) {
@@ -201,6 +201,7 @@ class HostPages {
     }
 
    private:
+    static constexpr uint64_t kAsk = (uint64_t)4 << 20;  // asking costs 4 us, which shows in smaller calls (87 to 91 us)
     Part parts[3];
     bool missing, asked = false;
 };
@@ -315,7 +316,7 @@ struct SymptomDevice {
         a.obs_stride = os;
         a.packed = flags & GFS_BIT_PACKED ? 1 : 0;
         a.append = flags & GFS_APPEND_OBSERVABLES ? 1 : 0;
-        // Several blocks per CTA while a block has few segments for its 256 lanes and the grid still covers every SM
+        // Several blocks per CTA while a block has few segments for its 288 lanes and the grid still covers every SM
         // twice (d=3, 30 segments, 2^20 shots: 72 us with one block per CTA, 41 with eight; d=9, 395 segments, 2^18
         // shots: 57 and 48 with two; few blocks: 2^16 shots of d=3 take 12 us with one, 16 with eight).
         uint32_t lb = 0;
