@@ -3,6 +3,7 @@
 // 64-bit hit-record format written by noise_kernel.
 #pragma once
 
+#include <atomic>
 #include <cstdint>
 
 #include "frame_rules.h"
@@ -10,6 +11,35 @@
 #include "kernels.h"
 
 namespace gfs {
+
+// Lets launches of KERNEL on the current device take up to `smem` bytes of dynamic shared memory.  The limit belongs to the
+// function, whoever launches it: set to each launch's own size it could be lowered by another thread between one thread's
+// setting and its launch, which then failed.  So it is raised once per device, to all that a CTA may have beside the
+// kernel's static shared memory, and never lowered; how many CTAs an SM holds follows from the launch's own size.
+template <auto KERNEL>
+cudaError_t allow_smem(size_t smem) {
+    constexpr int kDevices = 64;
+    static std::atomic<int> limits[kDevices];  // 0: not raised yet (threads that meet here set the same value)
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    int limit = e == cudaSuccess && device < kDevices ? limits[device].load(std::memory_order_acquire) : 0;
+    if (e == cudaSuccess && limit == 0) {
+        cudaFuncAttributes at{};
+        int most = 0;
+        e = cudaFuncGetAttributes(&at, KERNEL);
+        if (e == cudaSuccess) {
+            e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+        }
+        limit = most - (int)at.sharedSizeBytes;
+        if (e == cudaSuccess) {
+            e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
+        }
+        if (e == cudaSuccess && device < kDevices) {
+            limits[device].store(limit, std::memory_order_release);
+        }
+    }
+    return e != cudaSuccess ? e : smem <= (size_t)limit ? cudaSuccess : cudaErrorInvalidValue;
+}
 
 __device__ __forceinline__ uint4 x4(uint4 a, uint4 b) {
     return make_uint4(a.x ^ b.x, a.y ^ b.y, a.z ^ b.z, a.w ^ b.w);

@@ -555,8 +555,7 @@ __global__ void __maxnreg__(96) batch_frame_kernel_lean(const BatchArgs b) {
 
 template <int B>
 cudaError_t lean_batch_launch_b(const BatchArgs &args, const LaunchShape &s, cudaStream_t stream) {
-    cudaError_t e =
-        cudaFuncSetAttribute(batch_frame_kernel_lean<B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
+    cudaError_t e = allow_smem<batch_frame_kernel_lean<B>>(s.smem);
     if (e != cudaSuccess) {
         return e;
     }
@@ -570,8 +569,7 @@ cudaError_t lean_batch_launch_b(const BatchArgs &args, const LaunchShape &s, cud
 
 template <int B>
 cudaError_t lean_batch_occ_b(const LaunchShape &s, int *out) {
-    cudaError_t e =
-        cudaFuncSetAttribute(batch_frame_kernel_lean<B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
+    cudaError_t e = allow_smem<batch_frame_kernel_lean<B>>(s.smem);
     if (e != cudaSuccess) {
         return e;
     }
@@ -580,8 +578,7 @@ cudaError_t lean_batch_occ_b(const LaunchShape &s, int *out) {
 
 template <int B, int J>
 cudaError_t lean_launch_j(const KernelArgs &args, const LaunchShape &s, cudaStream_t stream) {
-    cudaError_t e =
-        cudaFuncSetAttribute(frame_kernel_lean<B, J>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
+    cudaError_t e = allow_smem<frame_kernel_lean<B, J>>(s.smem);
     if (e != cudaSuccess) {
         return e;
     }
@@ -596,8 +593,7 @@ cudaError_t lean_launch_b(const KernelArgs &args, const LaunchShape &s, cudaStre
 
 template <int B, int J>
 cudaError_t lean_occ_j(const LaunchShape &s, int *out) {
-    cudaError_t e =
-        cudaFuncSetAttribute(frame_kernel_lean<B, J>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
+    cudaError_t e = allow_smem<frame_kernel_lean<B, J>>(s.smem);
     if (e != cudaSuccess) {
         return e;
     }

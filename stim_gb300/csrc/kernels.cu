@@ -1240,8 +1240,7 @@ size_t frame_smem_bytes(uint32_t nrows, uint32_t ring, uint32_t nobs, int blocks
 
 template <int B, bool H>
 static cudaError_t launch_b(const KernelArgs &args, const LaunchShape &s, cudaStream_t stream) {
-    cudaError_t e =
-        cudaFuncSetAttribute(frame_kernel<B, H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
+    cudaError_t e = allow_smem<frame_kernel<B, H>>(s.smem);
     if (e != cudaSuccess) {
         return e;
     }
@@ -1251,8 +1250,7 @@ static cudaError_t launch_b(const KernelArgs &args, const LaunchShape &s, cudaSt
 
 template <bool H>
 static cudaError_t launch_global_frames(const KernelArgs &args, const LaunchShape &s, cudaStream_t stream) {
-    cudaError_t e =
-        cudaFuncSetAttribute(frame_kernel_global<H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
+    cudaError_t e = allow_smem<frame_kernel_global<H>>(s.smem);
     if (e != cudaSuccess) {
         return e;
     }
@@ -1325,8 +1323,7 @@ cudaError_t launch_noise_kernel(const KernelArgs &args, int blocks_per_cta, cuda
 
 template <int B, bool H>
 static cudaError_t launch_batch_b(const BatchArgs &args, const LaunchShape &s, cudaStream_t stream) {
-    cudaError_t e = cudaFuncSetAttribute(batch_frame_kernel<B, H>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)s.smem);
+    cudaError_t e = allow_smem<batch_frame_kernel<B, H>>(s.smem);
     if (e != cudaSuccess) {
         return e;
     }
@@ -1389,8 +1386,7 @@ cudaError_t launch_batch_frame_kernel(const BatchArgs &args, const LaunchShape &
 
 template <int B, bool H>
 static cudaError_t occ_batch_b(const LaunchShape &s, int *out) {
-    cudaError_t e = cudaFuncSetAttribute(batch_frame_kernel<B, H>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)s.smem);
+    cudaError_t e = allow_smem<batch_frame_kernel<B, H>>(s.smem);
     if (e != cudaSuccess) {
         return e;
     }
@@ -1413,8 +1409,7 @@ cudaError_t batch_frame_kernel_max_ctas_per_sm(const LaunchShape &shape, int *ou
 
 template <int B, bool H>
 static cudaError_t occ_b(const LaunchShape &s, int *out) {
-    cudaError_t e =
-        cudaFuncSetAttribute(frame_kernel<B, H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
+    cudaError_t e = allow_smem<frame_kernel<B, H>>(s.smem);
     if (e != cudaSuccess) {
         return e;
     }
@@ -1423,8 +1418,7 @@ static cudaError_t occ_b(const LaunchShape &s, int *out) {
 
 template <bool H>
 static cudaError_t occ_global_frames(const LaunchShape &s, int *out) {
-    cudaError_t e =
-        cudaFuncSetAttribute(frame_kernel_global<H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
+    cudaError_t e = allow_smem<frame_kernel_global<H>>(s.smem);
     if (e != cudaSuccess) {
         return e;
     }

@@ -168,7 +168,7 @@ cudaError_t launch_convert(const ConvertArgs &args, cudaStream_t stream) {
     uint32_t r, s;
     regions(args.M, args.D, args.O, args.append != 0, &r, &s);
     const size_t smem = ((size_t)r + s) * sizeof(uint4);
-    cudaError_t e = cudaFuncSetAttribute(convert_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem<convert_kernel>(smem);
     if (e != cudaSuccess) {
         return e;
     }

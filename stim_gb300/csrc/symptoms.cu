@@ -503,8 +503,7 @@ __global__ void __launch_bounds__(kBatchThreads)
 
 template <bool PACKED, bool SCREEN>
 cudaError_t launch_packed(const SymArgs &args, uint32_t grid, size_t smem, cudaStream_t stream) {
-    cudaError_t e =
-        cudaFuncSetAttribute(symptom_kernel<PACKED, SCREEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem<symptom_kernel<PACKED, SCREEN>>(smem);
     if (e != cudaSuccess) {
         return e;
     }
@@ -515,8 +514,7 @@ cudaError_t launch_packed(const SymArgs &args, uint32_t grid, size_t smem, cudaS
 template <bool PACKED>
 cudaError_t launch_batch(const SymArgs *entries, const uint32_t *prefix, uint32_t n, uint32_t grid, size_t smem,
                          cudaStream_t stream) {
-    cudaError_t e =
-        cudaFuncSetAttribute(batch_symptom_kernel<PACKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem<batch_symptom_kernel<PACKED>>(smem);
     if (e != cudaSuccess) {
         return e;
     }
