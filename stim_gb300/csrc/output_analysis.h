@@ -15,7 +15,7 @@ namespace gfs {
 using Set = std::vector<uint32_t>;  // sorted outputs: detectors by index, then observables as kSymObs | index
 
 constexpr uint64_t kWorkLimit = 400000000ull;
-constexpr uint32_t kProbes = 12;   // iterations of a loop checked for a steady state
+constexpr uint32_t kProbes = 12;   // iterations of a loop checked for a steady state, at most
 constexpr uint32_t kPeriods = 3;   // of one, two or three iterations (colour codes measure X, Y, Z in turn)
 constexpr size_t kMaxEntries = (size_t)1 << 22;   // output lists (16 bytes each) kept per program
 constexpr size_t kMaxLongs = (size_t)1 << 24;
@@ -448,10 +448,29 @@ class OutputAnalysis {
         det -= left * ddet;
     }
 
+    // Units that one pass over ops [lo, hi) works on.
+    double units(uint32_t lo, uint32_t hi) const {
+        double n = 0;
+        for (uint32_t pc = lo; pc < hi; pc++) {
+            const DevOp &op = prog.ops[pc];
+            if ((op.code & 0xFFu) == OP_LOOP_BEGIN) {
+                n += (double)((uint64_t)op.a | ((uint64_t)op.b << 32)) * units(pc + 1, pc + 1 + op.n);
+                pc += op.n;
+            } else {
+                n += op.n;
+            }
+        }
+        return n;
+    }
+
+    // A probe copies and compares the whole state, so a loop gets as many as together touch at most half of the sets that its
+    // iterations do (2,000 loops of two iterations over one of 5,000 qubits: 1.1 s with a probe each, 12 ms without).
     void loop(uint32_t lo, uint32_t hi, uint64_t reps) {
+        const double worth = (double)reps * units(lo, hi) / (2.0 * (double)(xs.size() + zs.size() + R));
+        const uint64_t probes = worth < kProbes ? (uint64_t)worth : kProbes;
         std::vector<State> before;  // of the last kPeriods iterations, the latest first
         for (uint64_t r = 0; r < reps && !failed; r++) {
-            if (r >= kProbes || r + 1 == reps) {
+            if (r >= probes || r + 1 == reps) {
                 walk(lo, hi);
                 continue;
             }
