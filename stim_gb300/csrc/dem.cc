@@ -1,6 +1,7 @@
 // Detector error model parsing and lowering (dem.h).
 #include "dem.h"
 
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <map>
@@ -427,6 +428,155 @@ DemLayout layout_dem(const DemModel &m) {
         }
     }
     return L;
+}
+
+DemSymptoms list_symptoms(const DemModel &m, const DemLayout &L) {
+    const uint64_t D = m.num_detectors, O = m.num_observables;
+    DemSymptoms t;
+    if (D + O == 0 || D >= kSymObs || O >= kSymObs) {
+        return t;
+    }
+    std::vector<SymItem> items;
+    std::vector<SymSpan> at;  // detectors of items[k]
+    std::vector<std::vector<uint32_t>> seg(GFS_DEM_SEG_UNITS);
+    std::vector<uint32_t> all, part;
+    constexpr uint32_t kSpread = 2048;
+    for (uint32_t g = 0; g < (uint32_t)L.groups.size(); g++) {
+        const DemGroup &G = L.groups[g];
+        DevChan ch{};
+        ch.table = G.table;
+        ch.active = G.flags & 1u;
+        ch.inv_c = G.inv_c;
+        t.chans.push_back(ch);
+        if (G.flags & 2u) {
+            return t;  // p >= 1: every trial hits
+        }
+        if (!(G.flags & 1u)) {
+            continue;
+        }
+        const double unit_hits = m.p[L.units[G.first]] * GFS_BLOCK_SHOTS;
+        t.cost.hits += unit_hits * G.n;
+        for (uint32_t u0 = 0; u0 < G.n; u0 += kDemChunkUnits) {
+            const double n = std::min(kDemChunkUnits, G.n - u0);
+            t.cost.chunks += 1;
+            t.cost.rounds += unit_hits * n / std::min(32.0, std::ceil(n / GFS_DEM_SEG_UNITS));
+        }
+        t.cost.chunk_hits = std::max(t.cost.chunk_hits, unit_hits * std::min(G.n, kDemChunkUnits));
+        for (uint32_t u0 = 0; u0 < G.n; u0 += GFS_DEM_SEG_UNITS) {
+            const uint32_t n = std::min(GFS_DEM_SEG_UNITS, G.n - u0);
+            t.cost.segments += 1;
+            for (uint32_t u = 0; u < n; u++) {
+                const uint32_t e = L.units[G.first + u0 + u];
+                std::vector<uint32_t> &v = seg[u];
+                v.assign(m.sym.begin() + m.sym_off[e], m.sym.begin() + m.sym_off[e + 1]);
+                for (uint32_t &o : v) {
+                    o = o < D ? o : kSymObs | (uint32_t)(o - D);
+                }
+                std::sort(v.begin(), v.end());
+                size_t k = 0;
+                for (size_t j = 0; j < v.size();) {  // a symptom listed twice cancels
+                    if (j + 1 < v.size() && v[j] == v[j + 1]) {
+                        j += 2;
+                    } else {
+                        v[k++] = v[j++];
+                    }
+                }
+                v.resize(k);
+            }
+            // Mechanisms of a rare probability can lie anywhere in the model: a segment whose detectors spread over more
+            // than kSpread is drawn once per cluster of them, each time with its lists cut down to that cluster (the
+            // observables with the first).  d=25: 9 of 81,743 segments.
+            all.clear();
+            for (uint32_t u = 0; u < n; u++) {
+                for (uint32_t o : seg[u]) {
+                    if (!(o & kSymObs)) {
+                        all.push_back(o);
+                    }
+                }
+            }
+            std::sort(all.begin(), all.end());
+            for (size_t k = 0; k < all.size() || k == 0;) {
+                SymSpan s{0, 1, 0};
+                const size_t k0 = k;
+                while (k < all.size() && all[k] - all[k0] < kSpread) {
+                    k++;
+                }
+                if (k > k0) {
+                    s.lo = all[k0];
+                    s.hi = all[k - 1];
+                }
+                SymItem it{};
+                it.c1 = u0 / GFS_DEM_SEG_UNITS;
+                it.c2 = g;
+                it.c3 = gfs_c3(GFS_P_DEM, g, 0);
+                it.entry = (uint32_t)(t.lists.entries.size() / 4);
+                it.kind = KN_FLIP | 1u << 8 | (n * GFS_BLOCK_SHOTS) << 16;
+                it.base = s.lo <= s.hi ? s.lo : 0;
+                it.inv_c = G.inv_c;
+                it.chan = g;
+                for (uint32_t u = 0; u < n; u++) {
+                    part.clear();
+                    for (uint32_t o : seg[u]) {
+                        if (o & kSymObs ? k0 == 0 : o >= s.lo && o <= s.hi) {
+                            part.push_back(o);
+                        }
+                    }
+                    t.lists.add(part.data(), part.size(), it.base);
+                }
+                items.push_back(it);
+                at.push_back(s);
+                t.cost.drawn += unit_hits * n;
+                if (all.empty()) {
+                    break;
+                }
+            }
+        }
+    }
+    std::vector<uint32_t> order(items.size());
+    for (uint32_t k = 0; k < order.size(); k++) {
+        order[k] = k;
+    }
+    std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return at[a].lo < at[b].lo; });
+    for (uint32_t k : order) {
+        t.items.push_back(items[k]);
+        t.spans.push_back({(uint32_t)t.items.size(), at[k].lo, at[k].hi});
+    }
+    if (t.chans.empty()) {
+        t.chans.resize(1);
+    }
+    t.cost.items = (double)items.size();
+    t.ok = true;
+    return t;
+}
+
+bool symptoms_pay(const DemCost &c, uint64_t shots, uint64_t num_detectors, uint64_t row_bytes, bool packed) {
+    constexpr double kLink = 193e3;  // bytes a us to the host
+    const double blocks = (double)((shots + GFS_BLOCK_SHOTS - 1) / GFS_BLOCK_SHOTS), D = (double)num_detectors;
+    const double row = (double)std::max<uint64_t>(1, row_bytes);
+    const double block_bytes = (double)std::min<uint64_t>(shots, GFS_BLOCK_SHOTS) * row;
+    const double all_bytes = blocks * block_bytes, link = all_bytes / kLink;
+    auto chunk_of = [&](double bytes, double most) { return std::max(1.0, std::min({blocks, most, std::floor(bytes)})); };
+
+    // symptom_kernel: one CTA draws a block's items and hits and writes its rows, window by window; about 210 CTAs' worth of
+    // that goes on at a time.  64 MiB of rows a launch; small results leave while they are drawn.
+    const double cta = (c.stages > 1 ? 3.5 * c.stages : 0) + 1.1e-3 * c.segments + 2.2e-3 * (c.items - c.segments) +
+                       2.4e-3 * c.drawn + block_bytes / 20e3;
+    const double n = chunk_of((double)(64 << 20) / (128.0 * row), 1e18);
+    const double first = cta * std::max(1.0, n / 210);
+    const bool in_place = all_bytes <= (packed ? 4 : 8) * 1048576.0;
+    const double symptoms = 22 + (in_place ? std::max(first, link)
+                                           : first + std::max(link, (blocks - n) * cta / 210) +
+                                                 30 * (std::ceil(blocks / n) - 1));
+
+    // dem_sample_kernel: warps spread over chunks of mechanisms and blocks, so that few blocks take as long as the busiest
+    // chunk; then the transposes.  Up to 512 blocks or 1 GiB of buffers a launch.
+    const double block = 0.65e-5 * c.segments + 3e-4 * c.chunks + 6e-4 * c.rounds + (packed ? 2e-5 : 6e-5) * D;
+    const double busiest = 0.08 * std::min(c.chunk_hits, 300.0) + 0.042 * std::max(0.0, c.chunk_hits - 300);
+    const double m = chunk_of((double)(1 << 30) / (16 * D + 128.0 * row), 512);
+    const double mechanisms = 41 + std::max(busiest, m * block) +
+                              (c.chunk_hits > 300 ? 0.4 : 1.0) * std::min(busiest, m * block) +
+                              std::max(link, (blocks - m) * block);
+    return symptoms <= 0.97 * mechanisms;
 }
 
 }  // namespace gfs

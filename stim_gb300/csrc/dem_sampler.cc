@@ -6,7 +6,7 @@
 // error row with biased_randomize_bits over all shots and XORs it into its symptoms' rows.  Here the model is
 // parsed and grouped by probability once (dem.cc); a sample call runs symptom_kernel (symptoms.h: a block's rows in shared
 // memory, errors drawn under the counter-based contract, their symptoms XORed in), or, when the errors themselves are
-// wanted and for a few blocks of a large model, per chunk of 128-shot blocks, dem_sample_kernel (symptoms XORed into
+// wanted and where it is the faster way (symptoms_pay), per chunk of 128-shot blocks, dem_sample_kernel (symptoms XORed into
 // detector rows in device memory) and the shot-major transposes.  Replayed errors take the converter's path instead: their rows are transposed in
 // and folded into the outputs (each output the XOR of the mechanisms that list it).
 #include "dem.h"
@@ -29,6 +29,7 @@ struct gfs_dem {
     // Symptom sampling (symptoms.h) of calls that do not return errors: the mechanisms' symptoms are the output lists.
     DevBuf d_chans;
     gfs_rt::SymptomDevice sym;
+    gfs::DemCost cost;
     int num_sms = 0;
     bool writes_host = false;
 
@@ -44,127 +45,25 @@ struct gfs_dem {
 
 namespace {
 
-// The segments of every group as symptom items, in order of their lowest detector, with the symptoms of their
-// mechanisms as output lists.
+// Uploads the mechanisms' symptoms as output lists.
 void init_symptoms(gfs_dem *d) {
-    const gfs::DemModel &m = d->model;
-    const gfs::DemLayout &L = d->lay;
-    const uint64_t D = m.num_detectors, O = m.num_observables;
-    if (D + O == 0 || D >= gfs::kSymObs || O >= gfs::kSymObs) {
+    const uint64_t D = d->model.num_detectors, O = d->model.num_observables;
+    gfs::DemSymptoms t = gfs::list_symptoms(d->model, d->lay);
+    if (!t.ok) {
         return;
     }
-    std::vector<gfs::DevChan> chans;
-    std::vector<gfs::SymItem> items;
-    std::vector<gfs::SymSpan> at;  // detectors of items[k]
-    gfs::SymLists lists;
-    std::vector<std::vector<uint32_t>> seg(GFS_DEM_SEG_UNITS);
-    std::vector<uint32_t> all, part;
-    constexpr uint32_t kSpread = 2048;
-    double hits = 0;  // expected per 128-shot block
-    for (uint32_t g = 0; g < (uint32_t)L.groups.size(); g++) {
-        const gfs::DemGroup &G = L.groups[g];
-        gfs::DevChan ch{};
-        ch.table = G.table;
-        ch.active = G.flags & 1u;
-        ch.inv_c = G.inv_c;
-        chans.push_back(ch);
-        if (G.flags & 2u) {
-            return;  // p >= 1: every trial hits
-        }
-        if (!(G.flags & 1u)) {
-            continue;
-        }
-        hits += m.p[L.units[G.first]] * G.n * GFS_BLOCK_SHOTS;
-        for (uint32_t u0 = 0; u0 < G.n; u0 += GFS_DEM_SEG_UNITS) {
-            const uint32_t n = std::min(GFS_DEM_SEG_UNITS, G.n - u0);
-            for (uint32_t u = 0; u < n; u++) {
-                const uint32_t e = L.units[G.first + u0 + u];
-                std::vector<uint32_t> &v = seg[u];
-                v.assign(m.sym.begin() + m.sym_off[e], m.sym.begin() + m.sym_off[e + 1]);
-                for (uint32_t &o : v) {
-                    o = o < D ? o : gfs::kSymObs | (uint32_t)(o - D);
-                }
-                std::sort(v.begin(), v.end());
-                size_t k = 0;
-                for (size_t j = 0; j < v.size();) {  // a symptom listed twice cancels
-                    if (j + 1 < v.size() && v[j] == v[j + 1]) {
-                        j += 2;
-                    } else {
-                        v[k++] = v[j++];
-                    }
-                }
-                v.resize(k);
-            }
-            // Mechanisms of a rare probability can lie anywhere in the model: a segment whose detectors spread over more
-            // than kSpread is drawn once per cluster of them, each time with its lists cut down to that cluster (the
-            // observables with the first).  d=25: 9 of 81,743 segments.
-            all.clear();
-            for (uint32_t u = 0; u < n; u++) {
-                for (uint32_t o : seg[u]) {
-                    if (!(o & gfs::kSymObs)) {
-                        all.push_back(o);
-                    }
-                }
-            }
-            std::sort(all.begin(), all.end());
-            for (size_t k = 0; k < all.size() || k == 0;) {
-                gfs::SymSpan s{0, 1, 0};
-                const size_t k0 = k;
-                while (k < all.size() && all[k] - all[k0] < kSpread) {
-                    k++;
-                }
-                if (k > k0) {
-                    s.lo = all[k0];
-                    s.hi = all[k - 1];
-                }
-                gfs::SymItem it{};
-                it.c1 = u0 / GFS_DEM_SEG_UNITS;
-                it.c2 = g;
-                it.c3 = gfs_c3(GFS_P_DEM, g, 0);
-                it.entry = (uint32_t)(lists.entries.size() / 4);
-                it.kind = gfs::KN_FLIP | 1u << 8 | (n * GFS_BLOCK_SHOTS) << 16;
-                it.base = s.lo <= s.hi ? s.lo : 0;
-                it.inv_c = G.inv_c;
-                it.chan = g;
-                for (uint32_t u = 0; u < n; u++) {
-                    part.clear();
-                    for (uint32_t o : seg[u]) {
-                        if (o & gfs::kSymObs ? k0 == 0 : o >= s.lo && o <= s.hi) {
-                            part.push_back(o);
-                        }
-                    }
-                    lists.add(part.data(), part.size(), it.base);
-                }
-                items.push_back(it);
-                at.push_back(s);
-                if (all.empty()) {
-                    break;
-                }
-            }
-        }
-    }
-    std::vector<uint32_t> order(items.size());
-    for (uint32_t k = 0; k < order.size(); k++) {
-        order[k] = k;
-    }
-    std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return at[a].lo < at[b].lo; });
-    if (chans.empty()) {
-        chans.resize(1);
-    }
-    upload(d->d_chans, chans, d->device, d->stream);
-    d->sym.init(d->device, d->stream, lists, D, O, d->seed, d->d_tables.p, d->d_chans.p,
+    upload(d->d_chans, t.chans, d->device, d->stream);
+    d->sym.init(d->device, d->stream, t.lists, D, O, d->seed, d->d_tables.p, d->d_chans.p,
                 [&](uint32_t words, gfs::SymptomPlan &plan) {
                     plan = gfs::SymptomPlan();
-                    std::vector<gfs::SymSpan> spans;
-                    for (uint32_t k : order) {
-                        plan.items.push_back(items[k]);
-                        spans.push_back({(uint32_t)plan.items.size(), at[k].lo, at[k].hi});
-                    }
-                    return gfs::plan_stages(spans, D, O, words, plan);
+                    plan.items = t.items;
+                    return gfs::plan_stages(t.spans, D, O, words, plan);
                 });
+    d->cost = t.cost;
+    d->cost.stages = d->sym.args.nstages;
     // Screening draws the first gap of a segment with a hit twice.  d=25 at 0.04 / 0.18 / 0.9 / 1.8 hits a segment, screened
     // and not: 176 / 221 / 410 / 615 and 317 / 345 / 524 / 744 us; small models at 2.6 245 / 269, at 5.2 290 / 273.
-    d->sym.args.screen = hits < 2.0 * (double)items.size() ? 1 : 0;
+    d->sym.args.screen = t.cost.hits < 2.0 * t.cost.items ? 1 : 0;
 }
 
 void create(gfs_dem *d, const char *text, size_t len, uint64_t seed, int device) {
@@ -227,14 +126,8 @@ void sample(gfs_dem *d, uint64_t shots, uint32_t flags, uint8_t *dets, uint64_t 
     }
     ck(cudaSetDevice(d->device), "cudaSetDevice");
     const bool want_errs = errs != nullptr && !replay;
-    // A few blocks of a large model leave most SMs idle, one CTA drawing all segments of a block, while the kernels that go
-    // mechanism by mechanism spread them (host arrays, us, those and symptom sampling; 82 K segments: packed 1 block 86 and
-    // 172, 64 blocks 229 and 261, 96 blocks 308 and 304; unpacked 200 blocks 2,416 and 2,506, 256 blocks 3,068 and 3,110;
-    // 41 K segments: packed 8 blocks 90 and 94, 16 blocks 97 and 95, unpacked 96 blocks 646 and 677, 128 blocks 828 and
-    // 846; 20 K segments: symptom sampling throughout).
-    const uint64_t segments = d->sym.nitems, sample_blocks = (shots + 127) / 128;
-    const bool few_blocks = packed ? 512 * sample_blocks + (32u << 10) < segments : 192 * sample_blocks + (24u << 10) < segments;
-    const bool symptoms = d->sym.ready && !want_errs && !replay && !few_blocks;
+    const bool symptoms = d->sym.ready && !want_errs && !replay &&
+                          gfs::symptoms_pay(d->cost, shots, D, (dets ? drow : 0) + (obs ? orow : 0), packed);
     if (symptoms && d->writes_host && shots &&
         gfs_rt::write_in_place({{dets, shots * dstride}, {obs, shots * ostride}}, d->sym.in_place(packed, drow, dstride))) {
         gfs::SymArgs a = d->sym.call(shots, d->next_block, flags & GFS_BIT_PACKED, drow ? dets : nullptr, dstride,
