@@ -48,6 +48,12 @@ struct Program {
     std::vector<OccXform> occ_xform;  // transforms of the hit occurrences the lean plan moved (NoiseOcc.xform)
     bool lean_ok = false;
     SymptomTable symptoms;  // outputs flipped by each noise hit (detection sampling; symptoms.h)
+
+    // Output flips a block up to which flipping one by one costs less than walking the frames: `work` counts the frame rows
+    // that a block touches, and a hit costs a frame kernel about four of them (d=25: 40 K flips against 537 K rows).
+    double symptoms_worth() const {
+        return work + 4 * hits_per_block;
+    }
 };
 
 struct LowerOptions {

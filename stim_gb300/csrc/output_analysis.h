@@ -82,6 +82,7 @@ class OutputAnalysis {
     uint64_t R = 1, meas = 0, det = 0, work = 0;
     size_t occ = 0;       // noise occurrences before this point
     bool record = false;  // output lists are being kept
+    double flips_per_block = 0;  // of the occurrences listed so far, loops filled in by shifting once
     bool failed = false;
     std::vector<uint8_t> ok;
     struct Flip {
@@ -205,7 +206,8 @@ class OutputAnalysis {
             return;
         }
         SymptomTable &t = prog.symptoms;
-        SymList &l = t.occ[--occ];
+        const size_t k = --occ;
+        SymList &l = t.occ[k];
         l = SymList();
         if (!prog.chans[ch].active) {
             return;
@@ -238,7 +240,7 @@ class OutputAnalysis {
         }
         l.per_unit = fixed ? 1u : (1u << gens) - 1;
         l.entry = (uint32_t)(t.lists.entries.size() / 4);
-        if (t.lists.entries.size() / 4 + (size_t)n * l.per_unit > kMaxEntries || t.lists.longs.size() > kMaxLongs) {
+        if (t.lists.entries.size() / 4 + (size_t)n * l.per_unit > kMaxEntries) {
             drop();
             return;
         }
@@ -263,6 +265,10 @@ class OutputAnalysis {
         size_t at = t.lists.entries.size(), count = 0;
         t.lists.entries.resize(at + 4 * (size_t)n * l.per_unit);
         for (uint32_t u = 0; u < n; u++) {
+            if (t.lists.longs.size() > kMaxLongs) {
+                drop();
+                return;
+            }
             // The unit's outputs, each with the set of generators that flip it; pattern b flips those of odd overlap.
             flips.clear();
             for (uint32_t g = 0; g < gens; g++) {
@@ -299,8 +305,13 @@ class OutputAnalysis {
                 count += len;
             }
         }
-        work += count;
         l.mean = (double)count / std::max<uint32_t>(1, n * l.per_unit);
+        // Lists too long to pay (200 qubits measured 200 times without resets, every result a detector: 66 flips a hit) are
+        // given up as soon as that shows: listing them all took 0.16 s, 10 times as long as the pass alone.
+        flips_per_block += prog.occ_hits_per_block[k] * l.mean;
+        if (flips_per_block > prog.symptoms_worth()) {
+            drop();
+        }
     }
 
     // The unit's flips as entry halfwords and one observable at most, each with the set of patterns of odd overlap; false

@@ -663,10 +663,7 @@ struct gfs_sampler {
     void init_symptoms() {
         gfs::SymptomTable &t = prog.symptoms;
         const uint64_t D = prog.num_detectors, O = prog.num_observables;
-        // Lists so long that flipping outputs one by one costs more than walking the frames (prog.work: the frame rows
-        // a block touches; a hit costs a frame kernel about four of them) stay with the frame kernels.  No circuit of the
-        // test set or the benchmark comes near this line (d=25: 40 K flips against 537 K rows).
-        if (!t.ok || D + O == 0 || t.flips_per_block > prog.work + 4 * prog.hits_per_block) {
+        if (!t.ok || D + O == 0 || t.flips_per_block > prog.symptoms_worth()) {
             return;
         }
         sym.init(device, stream, t.lists, D, O, seed, d_tables.p, d_chans.p,

@@ -24,3 +24,14 @@ def test_many_short_loops_over_many_qubits():
     looped = seconds(f"R {q}\n" + ("REPEAT 2 {\n" + body + "}\n") * 1000 + end)
     flat = seconds(f"R {q}\n" + (body + body) * 1000 + end)
     assert looped < 10 * flat + 0.05
+
+
+def test_lists_too_long_to_pay():
+    # No resets, every result a detector: a hit flips all later results of its qubit.  Listing them took ten times as long as
+    # lowering, and the sampler then kept its frames.
+    q = " ".join(map(str, range(200)))
+
+    def raw(noise):
+        return (f"R {q}\nREPEAT 200 {{\n{noise}M {q}\n" + "".join(f"DETECTOR rec[-{k + 1}]\n" for k in range(200)) + "}\n")
+
+    assert seconds(raw(f"DEPOLARIZE1(0.01) {q}\n")) < 4 * seconds(raw("")) + 0.02
