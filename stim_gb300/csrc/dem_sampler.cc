@@ -129,7 +129,7 @@ void sample(gfs_dem *d, uint64_t shots, uint32_t flags, uint8_t *dets, uint64_t 
     const bool symptoms = d->sym.ready && !want_errs && !replay &&
                           gfs::symptoms_pay(d->cost, shots, D, (dets ? drow : 0) + (obs ? orow : 0), packed);
     if (symptoms && d->writes_host && shots &&
-        gfs_rt::write_in_place({{dets, shots * dstride}, {obs, shots * ostride}}, d->sym.in_place(packed, drow, dstride))) {
+        gfs_rt::write_in_place({{dets, shots, drow, dstride}, {obs, shots, orow, ostride}}, d->sym.in_place(packed, drow, dstride))) {
         gfs::SymArgs a = d->sym.call(shots, d->next_block, flags & GFS_BIT_PACKED, drow ? dets : nullptr, dstride,
                                      orow ? obs : nullptr, ostride, (shots + 127) / 128, d->num_sms);
         a.host = 1;
@@ -229,20 +229,20 @@ void sample(gfs_dem *d, uint64_t shots, uint32_t flags, uint8_t *dets, uint64_t 
             tr((const uint4 *)d->err_buf[k].p, E, eout, erow);
         }
     };
-    HostPages pages(d->writes_host, {dets, shots * dstride}, {obs, shots * ostride}, {errs, shots * estride});
+    HostPages pages(d->writes_host, {dets, shots, drow, dstride}, {obs, shots, orow, ostride}, {errs, shots, erow, estride});
     auto copy_out = [&](int k, uint64_t done, uint64_t cs) {
         cudaStream_t st = d->streams[k];
         uint8_t *dout = (uint8_t *)d->out_buf[k].p, *oout = dout + chunk * drow, *eout = oout + chunk * orow;
         if (dets && drow) {
-            pages.before_copy(dets + done * dstride, (cs - 1) * dstride + drow);
+            pages.before_copy({dets + done * dstride, cs, drow, dstride});
             copy2d(dets + done * dstride, dstride, dout, drow, drow, cs, cudaMemcpyDeviceToHost, st, "copy dets");
         }
         if (obs && orow) {
-            pages.before_copy(obs + done * ostride, (cs - 1) * ostride + orow);
+            pages.before_copy({obs + done * ostride, cs, orow, ostride});
             copy2d(obs + done * ostride, ostride, oout, orow, orow, cs, cudaMemcpyDeviceToHost, st, "copy obs");
         }
         if (want_errs && erow) {
-            pages.before_copy(errs + done * estride, (cs - 1) * estride + erow);
+            pages.before_copy({errs + done * estride, cs, erow, estride});
             copy2d(errs + done * estride, estride, eout, erow, erow, cs, cudaMemcpyDeviceToHost, st, "copy errs");
         }
     };

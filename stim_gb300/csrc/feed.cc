@@ -100,7 +100,7 @@ void sample_for_decoder(gfs_sampler *s, uint64_t shots, const uint8_t *mask, uin
     // counts of chunk n - 1, whose kept rows leave on the copy stream (with page-locked destinations beside chunk n's
     // kernels), so the device always has a chunk to work on.  A slot is reused once its copy has ended.
     uint64_t kept_total = 0, dropped = 0, events = 0;
-    HostPages pages(s->writes_host, {dets, shots * dstride}, {obs, shots * ostride});
+    HostPages pages(s->writes_host, {dets, shots, drow, dstride}, {obs, shots, orow, ostride});
     bool copying[2] = {false, false};
     auto finish = [&](int k) {
         const gfs::FeedArgs &a = args[k];

@@ -338,16 +338,16 @@ void convert(gfs_m2d *m, uint64_t shots, const uint8_t *meas, uint64_t meas_stri
             tr(ot, O, nullptr, 0, oout, orow);
         }
     };
-    HostPages pages(m->reads_host, {dets, shots * dstride}, {obs, shots * ostride});
+    HostPages pages(m->reads_host, {dets, shots, drow, dstride}, {obs, shots, orow, ostride});
     auto copy_out = [&](int k, uint64_t done, uint64_t cs) {
         cudaStream_t st = m->streams[k];
         uint8_t *dout = (uint8_t *)m->out_buf[k].p, *oout = dout + chunk * drow;
         if (dets && drow) {
-            pages.before_copy(dets + done * dstride, (cs - 1) * dstride + drow);
+            pages.before_copy({dets + done * dstride, cs, drow, dstride});
             copy2d(dets + done * dstride, dstride, dout, drow, drow, cs, cudaMemcpyDeviceToHost, st, "copy dets");
         }
         if (obs && orow) {
-            pages.before_copy(obs + done * ostride, (cs - 1) * ostride + orow);
+            pages.before_copy({obs + done * ostride, cs, orow, ostride});
             copy2d(obs + done * ostride, ostride, oout, orow, orow, cs, cudaMemcpyDeviceToHost, st, "copy obs");
         }
     };

@@ -169,23 +169,38 @@ inline bool page_locked(std::initializer_list<const void *> ptrs) {
     return true;
 }
 
-// A call's host destinations (address and bytes; null: none), populated piece by piece before copies into them.  Whether
+// A call's result in host memory: rows of `width` bytes, `pitch` apart (p null: not wanted).
+struct HostRows {
+    const void *p = nullptr;
+    uint64_t rows = 0, width = 0, pitch = 0;
+
+    // First byte to last, the gaps between rows included, nothing after the last row.
+    uint64_t bytes() const {
+        return p && rows && width ? (rows - 1) * pitch + width : 0;
+    }
+    // Whether every page of that holds part of a row.  Rows further apart (a few columns of a wide array) share no pages, and
+    // the pages in between, which may never have been touched, are not this call's to ask for.
+    bool dense() const {
+        return rows <= 1 || pitch < width + (uint64_t)sysconf(_SC_PAGESIZE);
+    }
+};
+
+// A call's host destinations, populated piece by piece before copies into them.  Whether
 // any page is missing is asked once, before the first copy, beside the first chunks' kernels (10 ns a page: per chunk it
 // delayed every copy, d=25 error model 1.63 -> 1.67 ms per 2^17 shots).
 class HostPages {
    public:
-    using Part = std::pair<const void *, uint64_t>;
-    HostPages(bool shared, Part a, Part b = {}, Part c = {})
-        : parts{a, b, c}, missing(shared && (a.first ? a.second : 0) + (b.first ? b.second : 0) + (c.first ? c.second : 0) > kAsk) {
+    HostPages(bool shared, HostRows a, HostRows b = {}, HostRows c = {})
+        : parts{a, b, c}, missing(shared && a.bytes() + b.bytes() + c.bytes() > kAsk) {
     }
 
-    void before_copy(const void *p, uint64_t bytes) {
+    void before_copy(const HostRows &to) {
         if (missing && !asked) {
             asked = true;
             missing = false;
-            for (const Part &d : parts) {
-                if (d.first && d.second > 16384) {
-                    each_page_piece(d.first, d.second, [&](uintptr_t, uintptr_t n, uintptr_t, const unsigned char *there) {
+            for (const HostRows &d : parts) {
+                if (d.dense() && d.bytes() > 16384) {
+                    each_page_piece(d.p, d.bytes(), [&](uintptr_t, uintptr_t n, uintptr_t, const unsigned char *there) {
                         for (uintptr_t k = 0; k < n; k++) {
                             missing |= !(there[k] & 1);
                         }
@@ -193,35 +208,36 @@ class HostPages {
                     });
                 }
             }
-            missing = missing && !page_locked({parts[0].first, parts[1].first, parts[2].first});
+            missing = missing && !page_locked({parts[0].p, parts[1].p, parts[2].p});
         }
-        if (missing) {
-            populate(p, bytes);
+        if (missing && to.dense()) {
+            populate(to.p, to.bytes());
         }
     }
 
    private:
     static constexpr uint64_t kAsk = (uint64_t)4 << 20;  // asking costs 4 us, which shows in smaller calls (87 to 91 us)
-    Part parts[3];
+    HostRows parts[3];
     bool missing, asked = false;
 };
 
-// Whether a call's results (address and bytes; null: none) are small enough for its last kernel to write them straight to
+// Whether a call's results are small enough for its last kernel to write them straight to
 // host memory instead of staging and copying them: each copy costs more latency than a small call's kernels (1,024 shots
 // of d=3: 56 us, 28 without): up to SymptomDevice::in_place, other kernels 64 KiB (their transposes write rows in 2-byte units;
 // 6.6 MB of d=9 records: 253 us copied, 322 in place).
-inline bool write_in_place(std::initializer_list<std::pair<void *, uint64_t>> parts, uint64_t most = (uint64_t)64 << 10) {
+inline bool write_in_place(std::initializer_list<HostRows> parts, uint64_t most = (uint64_t)64 << 10) {
     uint64_t bytes = 0;
-    for (const auto &p : parts) {
-        bytes += p.first ? p.second : 0;
+    for (const HostRows &d : parts) {
+        bytes += d.bytes();
+        if (d.bytes() && !d.dense()) {
+            return false;
+        }
     }
     if (bytes > most) {
         return false;
     }
-    for (const auto &p : parts) {
-        if (p.first) {
-            populate(p.first, p.second);
-        }
+    for (const HostRows &d : parts) {
+        populate(d.p, d.bytes());
     }
     return true;
 }
@@ -962,7 +978,7 @@ struct gfs_sampler {
     // contiguous (a strided copy of narrow rows moves them one by one).
     void copy_rows(uint8_t *dst, uint64_t dpitch, const uint8_t *src, uint64_t spitch, uint64_t width, uint64_t rows,
                    HostPages &pages, const char *what) {
-        pages.before_copy(dst, (rows - 1) * dpitch + width);
+        pages.before_copy({dst, rows, width, dpitch});
         if (dpitch == width && spitch == width) {
             ck(cudaMemcpyAsync(dst, src, width * rows, cudaMemcpyDeviceToHost, copy_stream), what);
         } else {
@@ -1150,10 +1166,10 @@ struct gfs_sampler {
         reset_timings();
         const bool symptoms = symptoms_active(flags);
         const bool direct = !device_out && writes_host &&
-                            gfs_rt::write_in_place({{dets, shots * dstride}, {obs, shots * ostride}},
+                            gfs_rt::write_in_place({{dets, shots, drow, dstride}, {obs, shots, orow, ostride}},
                                                    symptoms ? sym.in_place(packed, drow, dstride) : (uint64_t)64 << 10);
         if (!device_out && !direct) {
-            HostPages pages(writes_host, {dets, shots * dstride}, {obs, shots * ostride});
+            HostPages pages(writes_host, {dets, shots, drow, dstride}, {obs, shots, orow, ostride});
             // Staging rows use the caller's stride when its rows are contiguous, so that each chunk leaves in
             // one linear copy; otherwise they are padded to 32 bytes and copied row by row.
             const uint64_t ds = dstride == drow ? drow : pad32(drow), os = ostride == orow ? orow : pad32(orow);
@@ -1291,12 +1307,12 @@ struct gfs_sampler {
             ck(cudaMemcpyAsync(ref_bits.p, ref, (M + 7) / 8, cudaMemcpyHostToDevice, stream), "ref upload");
             dref = (const uint8_t *)ref_bits.p;
         }
-        if (writes_host && gfs_rt::write_in_place({{out, shots * stride}})) {
+        if (writes_host && gfs_rt::write_in_place({{out, shots, row, stride}})) {
             measurements_device(shots, flags, ref, out, stride);
             return;
         }
         const uint64_t rs = stride == row ? row : pad32(row);
-        HostPages pages(writes_host, {out, shots * stride});
+        HostPages pages(writes_host, {out, shots, row, stride});
         host_pipeline(
             shots, rs,
             [&](uint64_t, uint64_t cs, uint8_t *buf) {
