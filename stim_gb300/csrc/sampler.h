@@ -127,10 +127,9 @@ inline void each_page_piece(const void *p, uint64_t bytes, F f) {
     }
 }
 
-// Gives pageable host memory that the device is about to write (or read) the pages that it lacks.  Pages that nothing has
-// touched yet would fault one by one, from the device or the copy engine (64 KiB: 21 us each, 3 here; 322 MB into new
-// arrays: 68-128 ms, 14 populated).
-inline void populate(const void *p, uint64_t bytes, bool write = true) {
+// Gives pageable host memory that the copy engine is about to write the pages that it lacks.  Pages that nothing has touched
+// yet would fault one by one (64 KiB: 21 us each, 3 here; 322 MB into new arrays: 68-128 ms, 14 populated).
+inline void populate(const void *p, uint64_t bytes) {
 #ifdef MADV_POPULATE_WRITE
     if (!p || bytes <= 16384) {
         return;
@@ -144,7 +143,7 @@ inline void populate(const void *p, uint64_t bytes, bool write = true) {
             past--;
         }
         if (past > first) {  // advice: errors do not matter
-            madvise((void *)(lo + first * page), (past - first) * page, write ? MADV_POPULATE_WRITE : MADV_POPULATE_READ);
+            madvise((void *)(lo + first * page), (past - first) * page, MADV_POPULATE_WRITE);
         }
         return true;
     });
@@ -167,6 +166,34 @@ inline bool page_locked(std::initializer_list<const void *> ptrs) {
         }
     }
     return true;
+}
+
+// Whether the device may read or write host memory where it lies.  Memory that this process may not touch (a read-only or
+// inaccessible mapping, a file's pages past its end) must not reach a kernel, whose access would be a GPU fault: a few pages are
+// touched by the host itself, which faults as in any copy, more are asked for at once (present pages cost 30 ns each), and
+// where the system refuses, the caller copies.  It refuses driver mappings too, of which page-locked memory is accessible.
+inline bool device_may_access(const void *p, uint64_t bytes, bool write) {
+    if (!p || !bytes) {
+        return true;
+    }
+    static const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+    const uintptr_t lo = (uintptr_t)p & ~(page - 1), past = (uintptr_t)p + bytes;
+    if (past - lo <= 8 * page) {
+        for (uintptr_t at = (uintptr_t)p; at < past; at = (at & ~(page - 1)) + page) {
+            if (write) {
+                __atomic_fetch_or((uint8_t *)at, (uint8_t)0, __ATOMIC_RELAXED);
+            } else {
+                (void)*(const volatile uint8_t *)at;
+            }
+        }
+        return true;
+    }
+#ifdef MADV_POPULATE_WRITE
+    if (madvise((void *)lo, past - lo, write ? MADV_POPULATE_WRITE : MADV_POPULATE_READ) == 0) {
+        return true;
+    }
+#endif
+    return page_locked({p});
 }
 
 // A call's result in host memory: rows of `width` bytes, `pitch` apart (p null: not wanted).
@@ -237,7 +264,9 @@ inline bool write_in_place(std::initializer_list<HostRows> parts, uint64_t most 
         return false;
     }
     for (const HostRows &d : parts) {
-        populate(d.p, d.bytes());
+        if (!device_may_access(d.p, d.bytes(), true)) {
+            return false;
+        }
     }
     return true;
 }

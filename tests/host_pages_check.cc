@@ -1,6 +1,8 @@
 // Checks what a call does to the pages of its host memory (stim_gb300/csrc/sampler.h: HostRows, HostPages, write_in_place),
 // on the CPU.  Usage: host_pages_check CASE  ->  prints "ok", or what is wrong, exit 1.
 // Test infrastructure (tests/test_host_pages.py compiles it); the product never uses it.
+#include <csetjmp>
+#include <csignal>
 #include <sys/mman.h>
 
 #include <cstdio>
@@ -29,6 +31,25 @@ size_t resident(const uint8_t *p, size_t bytes) {
         n += c & 1;
     }
     return n;
+}
+
+sigjmp_buf back;
+void on_fault(int) {
+    siglongjmp(back, 1);
+}
+
+// Whether f takes a memory fault on the host.
+template <typename F>
+int faults(F f) {
+    struct sigaction a {};
+    a.sa_handler = on_fault;
+    sigaction(SIGSEGV, &a, nullptr);
+    sigaction(SIGBUS, &a, nullptr);
+    if (sigsetjmp(back, 1)) {
+        return 1;
+    }
+    f();
+    return 0;
 }
 
 int expect(const char *what, size_t got, size_t want) {
@@ -65,6 +86,24 @@ int main(int argc, char **argv) {
         bad |= expect("pages after rows in place", resident(p, size), 1508);
         bad |= expect("too large for in place", write_in_place({{p + 1508 * kPage, 9, kPage, kPage}}, 8 * kPage), 0);
         bad |= expect("pages after rows too large", resident(p, size), 1508);
+    } else if (c == "read_only") {  // what the process may not write, no kernel gets to write
+        std::memset(p, 1, 100 * kPage);
+        mprotect(p, 100 * kPage, PROT_READ);
+        bad |= expect("many read-only pages in place", write_in_place({{p, 100, kPage, kPage}}, size), 0);
+        bad |= expect("one read-only page among many in place", write_in_place({{p + 99 * kPage, 100, kPage, kPage}}, size), 0);
+        bad |= expect("read-only pages may be read", device_may_access(p, 100 * kPage, false), 1);
+        bad |= expect("a read-only page: the host faults", faults([&] { write_in_place({{p + kPage, 3, 1, 1}}, size); }), 1);
+        bad |= expect("a writable page", faults([&] { bad |= expect("in place", write_in_place({{p + 100 * kPage, 3, 1, 1}}, size), 1); }), 0);
+        bad |= expect("its bytes", p[100 * kPage] + p[100 * kPage + 1], 0);
+    } else if (c == "inaccessible") {
+        mprotect(p, 100 * kPage, PROT_NONE);
+        bad |= expect("pages without access may be read", device_may_access(p, 100 * kPage, false), 0);
+        bad |= expect("a page without access: the host faults", faults([&] { device_may_access(p, 8, false); }), 1);
+        FILE *f = std::tmpfile();
+        bad |= ftruncate(fileno(f), kPage + 5);
+        void *m = mmap(nullptr, 100 * kPage, PROT_READ, MAP_SHARED, fileno(f), 0);
+        bad |= expect("a file's pages up to its end", device_may_access(m, 2 * kPage, false), 1);
+        bad |= expect("a file's pages past its end", device_may_access(m, 100 * kPage, false), 0);
     } else {
         std::printf("unknown case\n");
         return 2;

@@ -32,3 +32,9 @@ def run(checker, case):
 def test_only_pages_of_rows_are_asked_for(checker, case):
     out = run(checker, case)
     assert (out.returncode, out.stdout) == (0, "ok\n"), out.stdout + out.stderr
+
+
+@pytest.mark.parametrize("case", ["read_only", "inaccessible"])
+def test_memory_that_the_process_may_not_touch_reaches_no_kernel(checker, case):
+    out = run(checker, case)
+    assert (out.returncode, out.stdout) == (0, "ok\n"), out.stdout + out.stderr
