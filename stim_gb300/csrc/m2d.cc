@@ -377,6 +377,18 @@ void convert(gfs_m2d *m, uint64_t shots, const uint8_t *meas, uint64_t meas_stri
         }
         return;
     }
+    // Where a step fails, nothing of the call may stay in flight: the kernels may be reading the caller's records, and the
+    // copies write its arrays.
+    struct Drain {
+        gfs_m2d *m;
+        ~Drain() {
+            if (m) {
+                for (cudaStream_t st : m->streams) {
+                    cudaStreamSynchronize(st);
+                }
+            }
+        }
+    } drain{m};
     // Chunk k's copy out is issued after chunk k + 1's copy in and kernels are queued (a copy to or from
     // pageable memory may hold the calling thread until it completes); a slot is reused once its previous
     // chunk has left.
@@ -408,6 +420,7 @@ void convert(gfs_m2d *m, uint64_t shots, const uint8_t *meas, uint64_t meas_stri
     for (cudaStream_t st : m->streams) {
         ck(cudaStreamSynchronize(st), "convert");
     }
+    drain.m = nullptr;
 }
 
 // Files opened like the reference's RaiiFile (src/stim/io/raii_file.cc:44-66): no path, no file.
