@@ -1194,7 +1194,7 @@ struct gfs_sampler {
         ck(cudaSetDevice(device), "cudaSetDevice");
         reset_timings();
         const bool symptoms = symptoms_active(flags);
-        const bool direct = !device_out && writes_host &&
+        const bool direct = !device_out && writes_host && !chunk_shots &&  // a chosen chunk size is kept
                             gfs_rt::write_in_place({{dets, shots, drow, dstride}, {obs, shots, orow, ostride}},
                                                    symptoms ? sym.in_place(packed, drow, dstride) : (uint64_t)64 << 10);
         if (!device_out && !direct) {
@@ -1336,7 +1336,7 @@ struct gfs_sampler {
             ck(cudaMemcpyAsync(ref_bits.p, ref, (M + 7) / 8, cudaMemcpyHostToDevice, stream), "ref upload");
             dref = (const uint8_t *)ref_bits.p;
         }
-        if (writes_host && gfs_rt::write_in_place({{out, shots, row, stride}})) {
+        if (writes_host && !chunk_shots && gfs_rt::write_in_place({{out, shots, row, stride}})) {
             measurements_device(shots, flags, ref, out, stride);
             return;
         }
