@@ -277,15 +277,15 @@ void convert(gfs_m2d *m, uint64_t shots, const uint8_t *meas, uint64_t meas_stri
     auto compute = [&](int k, uint64_t done, uint64_t cs, const uint4 *base_dets, const uint4 *base_obs) {
         cudaStream_t st = m->streams[k];
         const uint64_t nblk = (cs + 127) / 128;
-        const bool in_place = direct && device_may_access(meas + done * mrow, cs * mrow, false);
-        if (!in_place) {
-            m->in_buf[k].ensure(std::max<uint64_t>(16, chunk * mrow), m->device);
+        if (direct) {
+            touch_pages({meas + done * mrow, cs, mrow, mrow}, false);
+        } else {
             copy2d(m->in_buf[k].p, mrow, meas + done * meas_stride, meas_stride, mrow, cs, cudaMemcpyHostToDevice, st,
                    "copy measurements");
         }
         if (fused) {
             gfs::ConvertArgs ca{};
-            ca.in = in_place ? meas + done * mrow : (const uint8_t *)m->in_buf[k].p;
+            ca.in = direct ? meas + done * mrow : (const uint8_t *)m->in_buf[k].p;
             ca.nshots = cs;
             ca.M = (uint32_t)M;
             ca.D = (uint32_t)D;

@@ -7,6 +7,7 @@
 #include <unistd.h>
 
 #include <algorithm>
+#include <chrono>
 #include <cstdio>
 #include <cstring>
 #include <initializer_list>
@@ -168,35 +169,7 @@ inline bool page_locked(std::initializer_list<const void *> ptrs) {
     return true;
 }
 
-// Whether the device may read or write host memory where it lies.  Memory that this process may not touch (a read-only or
-// inaccessible mapping, a file's pages past its end) must not reach a kernel, whose access would be a GPU fault: a few pages are
-// touched by the host itself, which faults as in any copy, more are asked for at once (present pages cost 30 ns each), and
-// where the system refuses, the caller copies.  It refuses driver mappings too, of which page-locked memory is accessible.
-inline bool device_may_access(const void *p, uint64_t bytes, bool write) {
-    if (!p || !bytes) {
-        return true;
-    }
-    static const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
-    const uintptr_t lo = (uintptr_t)p & ~(page - 1), past = (uintptr_t)p + bytes;
-    if (past - lo <= 8 * page) {
-        for (uintptr_t at = (uintptr_t)p; at < past; at = (at & ~(page - 1)) + page) {
-            if (write) {
-                __atomic_fetch_or((uint8_t *)at, (uint8_t)0, __ATOMIC_RELAXED);
-            } else {
-                (void)*(const volatile uint8_t *)at;
-            }
-        }
-        return true;
-    }
-#ifdef MADV_POPULATE_WRITE
-    if (madvise((void *)lo, past - lo, write ? MADV_POPULATE_WRITE : MADV_POPULATE_READ) == 0) {
-        return true;
-    }
-#endif
-    return page_locked({p});
-}
-
-// A call's result in host memory: rows of `width` bytes, `pitch` apart (p null: not wanted).
+// Rows of a call in host memory: `width` bytes each, `pitch` apart (p null: none).
 struct HostRows {
     const void *p = nullptr;
     uint64_t rows = 0, width = 0, pitch = 0;
@@ -211,6 +184,38 @@ struct HostRows {
         return rows <= 1 || pitch < width + (uint64_t)sysconf(_SC_PAGESIZE);
     }
 };
+
+// Touches every page of (dense) rows that a kernel is about to read or write where they lie, at a byte of a row.  Memory that
+// this process may not touch (a read-only or inaccessible mapping, a file's pages past its end) so faults here, on the host, and
+// not in the kernel, whose access would be a GPU fault; and pages that nothing has touched yet get their memory (from the
+// device they would fault one by one, 21 us each).  A present page takes 40 ns; eight that take more than a microsecond each
+// were missing, and the rest is asked for at once (64 KiB pages: 3 us each).
+inline void touch_pages(const HostRows &d, bool write) {
+    static const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+    const uintptr_t p = (uintptr_t)d.p, past = p + d.bytes();
+    bool asked = false;
+    for (uintptr_t at = p; at < past;) {
+        const auto start = std::chrono::steady_clock::now();
+        for (int k = 0; k < 8 && at < past; k++, at = (at & ~(page - 1)) + page) {
+            const uintptr_t in_row = (at - p) % d.pitch;
+            const uintptr_t own = in_row < d.width ? at : at + (d.pitch - in_row);  // a gap's bytes are not the call's
+            if (own >= past) {
+                break;
+            }
+            volatile uint8_t *const byte = (volatile uint8_t *)own;
+            const uint8_t value = *byte;
+            if (write) {
+                *byte = value;
+            }
+        }
+#ifdef MADV_POPULATE_WRITE
+        if (!asked && at < past && std::chrono::steady_clock::now() - start > std::chrono::microseconds(8)) {
+            asked = true;  // advice: a page that stays missing faults when it is touched
+            madvise((void *)(at & ~(page - 1)), past - (at & ~(page - 1)), write ? MADV_POPULATE_WRITE : MADV_POPULATE_READ);
+        }
+#endif
+    }
+}
 
 // A call's host destinations, populated piece by piece before copies into them.  Whether
 // any page is missing is asked once, before the first copy, beside the first chunks' kernels (10 ns a page: per chunk it
@@ -264,9 +269,7 @@ inline bool write_in_place(std::initializer_list<HostRows> parts, uint64_t most 
         return false;
     }
     for (const HostRows &d : parts) {
-        if (!device_may_access(d.p, d.bytes(), true)) {
-            return false;
-        }
+        touch_pages(d, true);
     }
     return true;
 }

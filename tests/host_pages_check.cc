@@ -86,24 +86,36 @@ int main(int argc, char **argv) {
         bad |= expect("pages after rows in place", resident(p, size), 1508);
         bad |= expect("too large for in place", write_in_place({{p + 1508 * kPage, 9, kPage, kPage}}, 8 * kPage), 0);
         bad |= expect("pages after rows too large", resident(p, size), 1508);
-    } else if (c == "read_only") {  // what the process may not write, no kernel gets to write
+    } else if (c == "read_only") {  // what the process may not write faults on the host
         std::memset(p, 1, 100 * kPage);
-        mprotect(p, 100 * kPage, PROT_READ);
-        bad |= expect("many read-only pages in place", write_in_place({{p, 100, kPage, kPage}}, size), 0);
-        bad |= expect("one read-only page among many in place", write_in_place({{p + 99 * kPage, 100, kPage, kPage}}, size), 0);
-        bad |= expect("read-only pages may be read", device_may_access(p, 100 * kPage, false), 1);
-        bad |= expect("a read-only page: the host faults", faults([&] { write_in_place({{p + kPage, 3, 1, 1}}, size); }), 1);
-        bad |= expect("a writable page", faults([&] { bad |= expect("in place", write_in_place({{p + 100 * kPage, 3, 1, 1}}, size), 1); }), 0);
-        bad |= expect("its bytes", p[100 * kPage] + p[100 * kPage + 1], 0);
+        mprotect(p + kPage, 99 * kPage, PROT_READ);
+        bad |= expect("read-only pages may be read: a fault", faults([&] { touch_pages({p, 100, kPage, kPage}, false); }), 0);
+        for (size_t n : {3 * kPage, 99 * kPage, 100 * kPage}) {
+            bad |= expect("read-only pages in place: a fault", faults([&] { write_in_place({{p, n, 1, 1}}, size); }), 1);
+        }
+        bad |= expect("writable bytes beside them: a fault", faults([&] { write_in_place({{p, kPage, 1, 1}}, size); }), 0);
+        bad |= expect("a writable byte", p[kPage - 1], 1);
+        bad |= expect("read-only pages among writable ones: a fault",
+                      faults([&] { write_in_place({{p + 99 * kPage, 100, kPage, kPage}}, size); }), 1);
+    } else if (c == "gaps") {  // the bytes between rows belong to others: pages are touched at bytes of rows
+        std::memset(p, 1, 64 * kPage);
+        mprotect(p + kPage, kPage, PROT_READ);
+        // The second row's first byte is the last of page 1.
+        bad |= expect("a read-only page with one byte of a row: a fault",
+                      faults([&] { write_in_place({{p + kPage - 8, 2, 8, kPage + 7}}, size); }), 1);
+        bad |= expect("a read-only page after the last row: a fault",
+                      faults([&] { write_in_place({{p + kPage / 2, 2, kPage / 4, kPage / 4}}, size); }), 0);
+        bad |= expect("many rows across a read-only page: a fault",
+                      faults([&] { write_in_place({{p, 30, 100, 3 * kPage / 4}}, size); }), 1);
     } else if (c == "inaccessible") {
-        mprotect(p, 100 * kPage, PROT_NONE);
-        bad |= expect("pages without access may be read", device_may_access(p, 100 * kPage, false), 0);
-        bad |= expect("a page without access: the host faults", faults([&] { device_may_access(p, 8, false); }), 1);
+        mprotect(p + 100 * kPage, kPage, PROT_NONE);
+        bad |= expect("pages before one without access: a fault", faults([&] { touch_pages({p, 100, kPage, kPage}, false); }), 0);
+        bad |= expect("pages up to one without access: a fault", faults([&] { touch_pages({p, 100 * kPage + 1, 1, 1}, false); }), 1);
         FILE *f = std::tmpfile();
         bad |= ftruncate(fileno(f), kPage + 5);
         void *m = mmap(nullptr, 100 * kPage, PROT_READ, MAP_SHARED, fileno(f), 0);
-        bad |= expect("a file's pages up to its end", device_may_access(m, 2 * kPage, false), 1);
-        bad |= expect("a file's pages past its end", device_may_access(m, 100 * kPage, false), 0);
+        bad |= expect("a file's pages up to its end: a fault", faults([&] { touch_pages({m, 2, kPage, kPage}, false); }), 0);
+        bad |= expect("a file's pages past its end: a fault", faults([&] { touch_pages({m, 100, kPage, kPage}, false); }), 1);
     } else {
         std::printf("unknown case\n");
         return 2;

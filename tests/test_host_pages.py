@@ -34,7 +34,7 @@ def test_only_pages_of_rows_are_asked_for(checker, case):
     assert (out.returncode, out.stdout) == (0, "ok\n"), out.stdout + out.stderr
 
 
-@pytest.mark.parametrize("case", ["read_only", "inaccessible"])
-def test_memory_that_the_process_may_not_touch_reaches_no_kernel(checker, case):
+@pytest.mark.parametrize("case", ["read_only", "gaps", "inaccessible"])
+def test_memory_that_the_process_may_not_touch_faults_on_the_host(checker, case):
     out = run(checker, case)
     assert (out.returncode, out.stdout) == (0, "ok\n"), out.stdout + out.stderr
