@@ -250,10 +250,12 @@ gfs_status gfs_sampler_set_hit_capacity(gfs_sampler *s, uint64_t records);
 gfs_status gfs_sampler_last_counts(const gfs_sampler *s, uint64_t *counts4);
 
 /*
- * Launch-shape autotuner: times the frame kernel on `trial_shots` shots (0 = 2^18) for each candidate
- * shape (blocks per CTA x threads x ring placement) that fits and keeps the fastest; *best_ms (may be
- * null) receives its time.  The sampler's stream position does not move and results never depend on the
- * shape.  No counterpart in the reference (its CPU sampler has no launch shape).
+ * Autotuner: times the frame kernel on `trial_shots` shots (0 = 2^18) for each candidate launch shape (blocks per
+ * CTA x threads x ring placement) that fits, and sampling by output lists where the circuit and the other settings
+ * allow it, and keeps the fastest: the frame kernels get the best shape, and detection calls run whichever took less,
+ * whatever gfs_sampler_set_shape chose before.  *best_ms (may be null) receives the time of what was kept.  The
+ * sampler's stream position does not move and results never depend on the choice.  No counterpart in the reference
+ * (its CPU sampler has no launch shape).
  */
 gfs_status gfs_sampler_autotune(gfs_sampler *s, uint64_t trial_shots, double *best_ms);
 
@@ -282,7 +284,8 @@ gfs_status gfs_batch_sample_detections(gfs_batch *b, const uint64_t *shots, uint
 gfs_status gfs_batch_set_shape(gfs_batch *b, int blocks_per_cta, int threads, int ring_placement);
 gfs_status gfs_batch_get_shape(const gfs_batch *b, int *blocks_per_cta, int *threads, int *grid, uint64_t *smem_bytes,
                                int *ring_global);
-/* Times each candidate shape on these shot counts (samplers do not advance) and keeps the fastest. */
+/* Times each candidate shape of the frame kernel, and the launches that sample by output lists, on these shot counts
+ * (samplers do not advance) and keeps the fastest, whatever gfs_batch_set_shape chose before. */
 gfs_status gfs_batch_autotune(gfs_batch *b, const uint64_t *shots, double *best_ms);
 /* out4: frame, transposes, host copies, whole call (ms); counts4: frame launches, transpose launches,
  * graph launches, graph builds (cumulative). */

@@ -248,8 +248,9 @@ class _SamplerBase:
         return v.value
 
     def autotune(self, trial_shots: int = 0) -> float:
-        """Times the frame kernel for each candidate launch shape and keeps the fastest (results never
-        depend on the shape; the stream position does not move).  Returns the best time in ms."""
+        """Times the frame kernel for each candidate launch shape, and sampling by output lists where the circuit and the
+        other settings allow it, and keeps the fastest (results never depend on it; the stream position does not move).
+        Returns the best time in ms."""
         ms = ctypes.c_double()
         check(lib().gfs_sampler_autotune(self._h, int(trial_shots), ctypes.byref(ms)))
         return ms.value
@@ -782,7 +783,8 @@ class BatchSampler:
                 "ring_global": bool(r.value)}
 
     def autotune(self, shots) -> float:
-        """Times each candidate launch shape on these shot counts and keeps the fastest; returns its ms."""
+        """Times each candidate launch shape of the frame kernel, and the launches that sample by output lists, on these
+        shot counts and keeps the fastest; returns its ms."""
         cshots, _ = self._shots(shots)
         ms = ctypes.c_double()
         check(lib().gfs_batch_autotune(self._h, cshots, ctypes.byref(ms)))

@@ -719,10 +719,15 @@ struct gfs_sampler {
         t.lists = gfs::SymLists();  // on the device now
     }
 
+    // Whether nothing but a chosen launch shape keeps detection calls from symptom_kernel.
+    bool symptoms_possible() const {
+        return sym.ready && mode == GFS_MODE_DETECTIONS && hits_pref == -1 && lean_pref == -1 && ring_pref == -1 &&
+               hit_capacity_override == 0;
+    }
+
     // Whether a detection call with these layout flags runs symptom_kernel.
     bool symptoms_active(uint32_t flags) const {
-        return sym.ready && mode == GFS_MODE_DETECTIONS && !frame_chosen && hits_pref == -1 && lean_pref == -1 &&
-               ring_pref == -1 && hit_capacity_override == 0 && !(flags & GFS_PREPEND_OBSERVABLES);
+        return symptoms_possible() && !frame_chosen && !(flags & GFS_PREPEND_OBSERVABLES);
     }
 
     // Enqueues the sampling of `cs` shots from stream block `block0` on into device rows (host: rows in host memory).
@@ -929,8 +934,10 @@ struct gfs_sampler {
         return take_status();
     }
 
-    // Times the frame kernel for each candidate launch shape on whole waves of at least `trial_shots` shots and
-    // keeps the fastest per shot.  The stream position does not move (the trial's results are discarded).
+    // Times the frame kernel for each candidate launch shape on whole waves of at least `trial_shots` shots, and symptom_kernel
+    // where the program allows it, and keeps the fastest per shot: the best shape of the frame kernels, which measurements
+    // and prepended observables use in any case, and the kernel that detection calls run (whatever was chosen before).  The
+    // stream position does not move (the trial's results are discarded).
     double autotune(uint64_t trial_shots) {
         struct Cand {
             int bpc, threads, ring;
@@ -978,6 +985,21 @@ struct gfs_sampler {
         shape_inline = best < 0 ? before_inline : best_inline;
         shape_lean = best < 0 ? before_lean : best_lean;
         lean_ready = best < 0 ? before_lean_ready : best_lean_ready;
+        if (symptoms_possible()) {
+            // Several waves, as above.  The rows stay in shared memory, as the frame kernels' times hold no transpose.
+            const uint64_t nblk = std::max<uint64_t>(want_blk, 16 * (uint64_t)num_sms);
+            float total = 0;
+            for (int rep = 0; rep < 2; rep++) {
+                ck(cudaEventRecord(ev[1], stream), "event");
+                run_symptoms(nblk * 128, next_block, GFS_BIT_PACKED, nullptr, 0, nullptr, 0);
+                ck(cudaEventRecord(ev[2], stream), "event");
+                ck(cudaStreamSynchronize(stream), "autotune");
+                total = (float)elapsed(1, 2);
+            }
+            const double per_block = total / (double)nblk;
+            frame_chosen = best >= 0 && best < per_block;
+            best = frame_chosen ? best : per_block;
+        }
         return best < 0 ? best : best * (double)want_blk;  // ms for the requested trial size
     }
 
