@@ -186,16 +186,19 @@ gfs_status gfs_sampler_last_timings(const gfs_sampler *s, double *out4, uint64_t
  * Launch shape: blocks_per_cta in {1, 2, 4} (128-shot blocks held in one CTA's shared memory),
  * threads per CTA (multiple of 32, <= 256), grid CTAs (0 = one full wave of resident CTAs).
  * Fails when the circuit's state does not fit shared memory with that many blocks.  A chosen shape also chooses the
- * frame kernels for detection events that would otherwise be sampled by output lists (gfs_sampler_set_noise_mode).
+ * frame kernels for detection events that would otherwise be sampled by output lists, until
+ * gfs_sampler_set_noise_mode(s, -1) or gfs_sampler_autotune.
  */
 gfs_status gfs_sampler_set_shape(gfs_sampler *s, int blocks_per_cta, int threads, int grid);
+/* The frame kernels' shape, also while detection calls run by output lists. */
 gfs_status gfs_sampler_get_shape(const gfs_sampler *s, int *blocks_per_cta, int *threads, int *grid,
                                  uint64_t *smem_bytes);
 
 /*
  * Where the measurement record window lives: 0 = shared memory, 1 = a per-CTA region of a global
  * (L2-resident) buffer, which frees shared memory for more resident CTAs; -1 = choose automatically (the
- * default).  Results do not depend on it.
+ * default).  A choice other than -1 also keeps detection events from being sampled by output lists.  Results do
+ * not depend on it.
  */
 gfs_status gfs_sampler_set_ring_placement(gfs_sampler *s, int placement);
 
@@ -226,7 +229,8 @@ gfs_status gfs_sampler_get_stream_position(const gfs_sampler *s, uint64_t *shot)
 
 /*
  * Noise generation: -1 (default) samples detection events by output lists where the circuit allows it (each noise hit
- * flips its precomputed detectors and observables in one kernel, without frames), otherwise as 1; 1 draws every noise
+ * flips its precomputed detectors and observables in one kernel, without frames; also after gfs_sampler_set_shape),
+ * otherwise as 1; 1 draws every noise
  * hit of a chunk in a separate kernel into a list that the frame kernel then applies; 0 draws noise inside the frame
  * kernel.  Results are identical either way.  No counterpart in the reference.
  */
@@ -243,7 +247,8 @@ gfs_status gfs_sampler_get_frame_kernel(const gfs_sampler *s, int *kind);
 gfs_status gfs_sampler_last_noise_ms(const gfs_sampler *s, double *ms);
 /* Hit-list region capacity in records per noise occurrence and slice (0 = automatic: expected hits plus a
  * wide margin).  A chunk whose hits do not fit is redone with inline noise, with identical results; a
- * small capacity exercises that. */
+ * small capacity exercises that.  A capacity other than 0 also keeps detection events from being sampled by output
+ * lists. */
 gfs_status gfs_sampler_set_hit_capacity(gfs_sampler *s, uint64_t records);
 /* Kernel launches of the last sample call: frame, transpose, noise; plus hit-list overflows (chunks redone
  * with inline noise) over the sampler's life. */

@@ -212,7 +212,8 @@ class _SamplerBase:
 
     # -- tuning / introspection (no counterpart in the reference) --
     def set_launch_shape(self, blocks_per_cta: int, threads: int = 256, grid: int = 0):
-        """Shape of the frame kernels, which a chosen shape also selects for detection events."""
+        """Shape of the frame kernels, which a chosen shape also selects for detection events (until set_noise_mode(-1)
+        or autotune)."""
         check(lib().gfs_sampler_set_shape(self._h, blocks_per_cta, threads, grid))
 
     def launch_shape(self):

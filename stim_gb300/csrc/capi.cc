@@ -648,6 +648,7 @@ gfs_status gfs_sampler_set_noise_mode(gfs_sampler *s, int mode) {
         }
         ck(cudaSetDevice(s->device), "cudaSetDevice");
         s->hits_pref = mode;
+        s->frame_chosen &= mode != -1;  // automatic: by output lists again, whatever shape was chosen before
         s->choose_shape(s->shape.blocks_per_cta, s->shape.threads, 0, s->shape.ring_global ? 1 : 0);
     });
 }

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 import stim_gb300
-from stim_gb300 import workloads
+from stim_gb300 import _native, workloads
 
 pytestmark = pytest.mark.gpu
 
@@ -32,6 +32,22 @@ def test_sampler_autotune_keeps_the_fastest(distance, trial):
     s.set_launch_shape(1, 64)
     assert not by_lists(s)
     s.autotune(trial)
+    assert by_lists(s)
+
+
+def test_every_setting_can_be_taken_back():
+    # Choices that keep detection events on the frame kernels, and what leads back to sampling by output lists.
+    s = circuit(5).compile_detector_sampler(seed=1)
+    capacity = lambda n: _native.check(_native.lib().gfs_sampler_set_hit_capacity(s._h, n))  # noqa: E731
+    for choose, back in ((lambda: s.set_launch_shape(1, 64), lambda: s.set_noise_mode(-1)),
+                         (lambda: s.set_noise_mode(1), lambda: s.set_noise_mode(-1)),
+                         (lambda: s.set_frame_kernel(0), lambda: s.set_frame_kernel(-1)),
+                         (lambda: s.set_ring_placement(1), lambda: s.set_ring_placement(-1)),
+                         (lambda: capacity(100), lambda: capacity(0))):
+        assert by_lists(s)
+        choose()
+        assert not by_lists(s)
+        back()
     assert by_lists(s)
 
 
