@@ -109,6 +109,14 @@ struct BatchEngine {
         }
     }
 
+    // Waits for everything this engine has begun, after an error.
+    void drain() {
+        cudaStreamSynchronize(stream);
+        for (cudaStream_t st : side) {
+            cudaStreamSynchronize(st);
+        }
+    }
+
     void init(int dev) {
         device = dev;
         ck(cudaSetDevice(device), "cudaSetDevice");
@@ -285,36 +293,49 @@ struct BatchEngine {
         return ctas;
     }
 
+    // The first group's launch goes on `stream`, the others beside it.  Whatever happens, `stream` waits for those that were
+    // begun, so that nothing outlives what is waited for after an error.
     void enqueue_symptoms() {
-        bool first = true, forked = false;
         int used = 0;
+        bool first = true;
+        struct Join {
+            BatchEngine &e;
+            const int &used;
+            cudaError_t error = cudaSuccess;
+            bool done = false;
+            void now() {
+                done = true;
+                for (int k = 0; k < used; k++) {
+                    cudaError_t r = cudaEventRecord(e.join[k], e.side[k]);
+                    r = r == cudaSuccess ? cudaStreamWaitEvent(e.stream, e.join[k], 0) : r;
+                    error = error == cudaSuccess ? r : error;
+                }
+            }
+            ~Join() {
+                if (!done) {
+                    now();
+                }
+            }
+        } joined{*this, used};
         for (SymGroup &g : groups) {
             if (g.args.empty()) {
                 continue;
             }
             cudaStream_t st = stream;
-            if (!first) {
-                if (!forked) {
-                    throw std::logic_error("symptom launches without a fork");
-                }
+            if (first) {
+                ck(cudaEventRecord(fork, stream), "fork");
+            } else {
                 st = side[used];
                 ck(cudaStreamWaitEvent(st, fork, 0), "fork");
-            } else {
-                ck(cudaEventRecord(fork, stream), "fork");
-                forked = true;
-            }
-            ck(gfs::launch_batch_symptoms((const gfs::SymArgs *)g.d_args.p, (const uint32_t *)g.d_prefix.p,
-                                          (uint32_t)g.args.size(), g.prefix.back(), g.smem, g.args[0].packed != 0, st),
-               "batch symptom kernel launch");
-            if (!first) {
-                ck(cudaEventRecord(join[used], st), "join");
                 used++;
             }
             first = false;
+            ck(gfs::launch_batch_symptoms((const gfs::SymArgs *)g.d_args.p, (const uint32_t *)g.d_prefix.p,
+                                          (uint32_t)g.args.size(), g.prefix.back(), g.smem, g.args[0].packed != 0, st),
+               "batch symptom kernel launch");
         }
-        for (int k = 0; k < used; k++) {
-            ck(cudaStreamWaitEvent(stream, join[k], 0), "join");
-        }
+        joined.now();
+        ck(joined.error, "join");
     }
 
     // Plans the entries (launch order = `order`, or input order when empty), allocates the arenas and

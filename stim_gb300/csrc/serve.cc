@@ -425,7 +425,7 @@ struct gfs_server {
 
     void sync_slot(Slot &slot) {
         for (auto &e : slot.eng) {
-            cudaStreamSynchronize(e.stream);
+            e.drain();
         }
     }
 
