@@ -22,15 +22,18 @@ __host__ __device__ __forceinline__ uint32_t up32(uint32_t n) {
     return (n + 31) & ~31u;
 }
 
-// Output columns [c0, c0 + n) of Q, shot-major, `row` bytes a shot, to `dst` (any alignment).
+// Output columns [c0, c0 + n) of Q, shot-major, `row` bytes a shot, to `dst` (any alignment): `groups` of 32 shots.
 __device__ __forceinline__ void rows_out(const uint4 *Q, uint32_t c0, uint32_t n, uint32_t row, uint8_t *dst,
-                                         const Transpose32 &turn) {
+                                         uint32_t groups, const Transpose32 &turn) {
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     for (uint32_t w = warp; w < (n + 31) / 32; w += kThreads / 32) {
         const uint4 v = 32 * w + lane < n ? Q[c0 + 32 * w + lane] : zero4();
         const uint32_t g[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
         for (uint32_t k = 0; k < 4; k++) {
+            if (k >= groups) {
+                break;
+            }
             const uint32_t x = turn(g[k]);
             uint8_t *const d = dst + (32 * k + lane) * row + 4 * w;
             const uint32_t left = row - 4 * w;  // bytes of this shot's row from here on
@@ -64,6 +67,7 @@ __global__ void __launch_bounds__(kThreads) convert_kernel(const ConvertArgs a, 
     uint4 *const S = sm + first;  // staged records, then output rows
     const uint64_t shot0 = (uint64_t)blockIdx.x * kShots;
     const uint32_t nvalid = a.nshots - shot0 < kShots ? (uint32_t)(a.nshots - shot0) : kShots;
+    const uint32_t groups = (nvalid + 31) / 32;  // of 32 shots; those without a shot are not turned (d=17, one shot: 49 us, now 41)
     {
         // The records may lie in host memory (then this is the copy in): several 16-byte loads a thread in flight.
         const uint4 *const in = reinterpret_cast<const uint4 *>(a.in + shot0 * mrow);  // 128 rows: a multiple of 16 bytes
@@ -88,9 +92,12 @@ __global__ void __launch_bounds__(kThreads) convert_kernel(const ConvertArgs a, 
     const Transpose32 turn(lane);
     const uint32_t *const words = reinterpret_cast<const uint32_t *>(S);
     for (uint32_t w = warp; w < up32(a.M) / 32; w += kThreads / 32) {
-        uint32_t g[4];
+        uint32_t g[4] = {0, 0, 0, 0};
 #pragma unroll
         for (uint32_t k = 0; k < 4; k++) {
+            if (k >= groups) {
+                break;
+            }
             const uint32_t at = (32 * k + lane) * mrow + 4 * w;  // byte offset: two aligned words hold its four bytes
             g[k] = turn(__funnelshift_r(words[at >> 2], words[(at >> 2) + 1], 8 * (at & 3u)));
         }
@@ -125,6 +132,9 @@ __global__ void __launch_bounds__(kThreads) convert_kernel(const ConvertArgs a, 
             const uint32_t g[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
             for (uint32_t k = 0; k < 4; k++) {
+                if (k >= groups) {
+                    break;
+                }
                 const uint32_t x = turn(g[k]), shot = 32 * k + lane;
                 for (uint32_t b = 0; b < 4 && 4 * w + b < orow; b++) {
                     if (shot < nvalid) {
@@ -135,7 +145,7 @@ __global__ void __launch_bounds__(kThreads) convert_kernel(const ConvertArgs a, 
         }
     }
     if (a.dets && drow) {
-        rows_out(S, 0, dcols, drow, reinterpret_cast<uint8_t *>(R), turn);
+        rows_out(S, 0, dcols, drow, reinterpret_cast<uint8_t *>(R), groups, turn);
         __syncthreads();
         store_bytes(a.dets + shot0 * drow, R, nvalid * drow);
     }
