@@ -348,18 +348,25 @@ __device__ __forceinline__ void write_flat(const SymArgs &a, const uint32_t *win
     }
 }
 
-// Sixteen 0 / 1 bytes of the low sixteen bits of v.
+// The low four, or sixteen, bits of v as 0 / 1 bytes (bit k of n to bit 8 k of n * (1 + 2^7 + 2^14 + 2^21)).
+__device__ __forceinline__ uint32_t expand4(uint32_t v) {
+    return (v & 15u) * 0x00204081u & 0x01010101u;
+}
 __device__ __forceinline__ uint4 expand16(uint32_t v) {
-    auto four = [](uint32_t n) { return (n & 15u) * 0x00204081u & 0x01010101u; };  // bit k of n to bit 8 k
-    return make_uint4(four(v), four(v >> 4), four(v >> 8), four(v >> 12));
+    return make_uint4(expand4(v), expand4(v >> 4), expand4(v >> 8), expand4(v >> 12));
 }
 
+// Unpacked rows up to this length are written word by word (us for 6 MB in host memory and 100 MB in device memory, words and
+// units: 24 columns 106 / 342 and 120 / 580, 201 columns 97 / 139 and 90 / 170, 333 columns 81 / 86 and 74 / 96, 400 columns
+// 61 / 78 and 55 / 65, 625 columns 72 / 88 and 68 / 80, 3,001 columns 79 / 64 and 61 / 37).
+constexpr uint32_t kWordRow = 350;
+static_assert(kWordRow >= 16, "longer rows hold a whole unit");
+
 // Unpacked rows, and rows of any kind in host memory (columns [c0, c1) of every shot): one warp per row, consecutive lanes
-// writing consecutive aligned units, and the partial units at the ends byte by byte.  A packed row's words are its
-// destination's, and leave as they are.  An unpacked row leaves in 16-byte units of sixteen expanded bits, four of a lane on
-// their way together: with words of four bits, one after another, a CTA wrote 13 GB/s, which one block of many detectors
-// waited for (48,000 detectors, 129 shots: 644 us, now 277; 10,007 shots of the d=25 repetition code in host memory: 88, now
-// 80).
+// writing consecutive aligned 32-bit words, of four expanded bits or (a packed row's words are its destination's) as they are;
+// the partial words at the ends byte by byte.  Long unpacked rows leave in 16-byte units of sixteen expanded bits, four of a
+// lane on their way together, with words only at their ends: word by word, one load chain after another, a CTA wrote 13 GB/s,
+// which a few blocks of many detectors waited for (48,000 detectors, 129 shots: 644 us, now 277).
 template <bool PACKED>
 __device__ __forceinline__ void write_words(const SymArgs &a, const uint32_t *win, uint32_t c0, uint32_t c1,
                                             uint64_t shot0, uint32_t nvalid, uint32_t dst0, bool last) {
@@ -384,30 +391,53 @@ __device__ __forceinline__ void write_words(const SymArgs &a, const uint32_t *wi
         }
         const uint32_t nbytes = c1 - c0;
         uint8_t *const d = start + c0;
-        const uint32_t head = min((uint32_t)(-(uintptr_t)d & 15u), nbytes);  // bytes before the first whole unit
-        const uint32_t units = (nbytes - head) / 16, tail = head + 16 * units;
-        uint4 *const d16 = reinterpret_cast<uint4 *>(d + head);
-        auto bits = [&](uint32_t q) {
-            const uint32_t c = head + 16 * q;
-            return __funnelshift_r(row[c >> 5], row[(c >> 5) + 1], c & 31u);
-        };
-        if (lane < 16) {
-            if (lane < head) {
-                d[lane] = (uint8_t)out_byte<false>(row, lane);
+        auto bits = [&](uint32_t c) { return __funnelshift_r(row[c >> 5], row[(c >> 5) + 1], c & 31u); };
+        auto bytes = [&](uint32_t c, uint32_t n) {  // fewer than four
+            for (uint32_t b = c; b < c + n; b++) {
+                d[b] = (uint8_t)out_byte<false>(row, b);
             }
-        } else if (tail + lane - 16 < nbytes) {
-            d[tail + lane - 16] = (uint8_t)out_byte<false>(row, tail + lane - 16);
+        };
+        auto word = [&](uint32_t c) { *reinterpret_cast<uint32_t *>(d + c) = expand4(bits(c)); };
+        if (nbytes <= kWordRow) {
+            const int32_t mis = (int32_t)((uintptr_t)d & 3u), n = (int32_t)nbytes;
+            for (int32_t q = (int32_t)lane; 4 * q < mis + n; q += 32) {
+                const int32_t o = 4 * q - mis;  // first byte (column) of this word within the piece
+                if (o >= 0 && o + 4 <= n) {
+                    word((uint32_t)o);
+                } else {
+                    bytes((uint32_t)max(o, 0), (uint32_t)(min(o + 4, n) - max(o, 0)));
+                }
+            }
+            continue;
         }
+        const uint32_t head = (uint32_t)(-(uintptr_t)d & 15u), units = (nbytes - head) / 16, tail = head + 16 * units;
+        if (lane < 4) {  // the words around the units, and the bytes around those
+            const uint32_t odd = head & 3u, c = odd + 4 * lane;
+            if (lane < 3 && c < head) {
+                word(c);
+            } else if (lane == 3) {
+                bytes(0, odd);
+            }
+        } else if (lane < 8) {
+            const uint32_t c = tail + 4 * (lane - 4);
+            if (c + 4 <= nbytes) {
+                word(c);
+            } else if (c < nbytes) {
+                bytes(c, nbytes - c);
+            }
+        }
+        uint4 *const d16 = reinterpret_cast<uint4 *>(d + head);
         uint32_t q = lane;
         for (; q + 96 < units; q += 128) {
-            const uint32_t v0 = bits(q), v1 = bits(q + 32), v2 = bits(q + 64), v3 = bits(q + 96);
+            const uint32_t v0 = bits(head + 16 * q), v1 = bits(head + 16 * (q + 32)), v2 = bits(head + 16 * (q + 64)),
+                           v3 = bits(head + 16 * (q + 96));
             d16[q] = expand16(v0);
             d16[q + 32] = expand16(v1);
             d16[q + 64] = expand16(v2);
             d16[q + 96] = expand16(v3);
         }
         for (; q < units; q += 32) {
-            d16[q] = expand16(bits(q));
+            d16[q] = expand16(bits(head + 16 * q));
         }
     }
 }
