@@ -560,7 +560,7 @@ bool symptoms_pay(const DemCost &c, uint64_t shots, uint64_t num_detectors, uint
     // symptom_kernel: one CTA draws a block's items and hits and writes its rows, window by window; about 210 CTAs' worth of
     // that goes on at a time.  64 MiB of rows a launch; small results leave while they are drawn.
     const double cta = (c.stages > 1 ? 3.5 * c.stages : 0) + 1.1e-3 * c.segments + 2.2e-3 * (c.items - c.segments) +
-                       2.4e-3 * c.drawn + block_bytes / 20e3;
+                       2.4e-3 * c.drawn + block_bytes / (packed ? 20e3 : 60e3);
     const double n = chunk_of((double)(64 << 20) / (128.0 * row), 1e18);
     const double first = cta * std::max(1.0, n / 210);
     const bool in_place = all_bytes <= (packed ? 4 : 8) * 1048576.0;

@@ -68,12 +68,12 @@ DemSymptoms list_symptoms(const DemModel &m, const DemLayout &L);
 // (`row_bytes` bytes) go to the host: an estimate in us of either, its constants fitted to 40 models (100 to 200,000
 // detectors, 100 to 326,000 mechanisms in order, shuffled or scattered, one to 300,000 probabilities from 1e-6 to 0.3; 1 to
 // 131,072 shots, packed and not): of 382 calls timed both ways it takes none for the route that is slower by more than 6%
-// and keeps seven, all below 80 us, on the mechanism kernels that symptom sampling would take 7-15% off.  Symptom sampling is
+// and keeps seven, all below 80 us, on the mechanism kernels that symptom sampling would take 8-23% off.  Symptom sampling is
 // the faster one where all detectors fit one window (d=5: 42 us for 66) and where there are blocks for every SM (d=25, 2^17
 // shots: 1.63 ms for 2.42).  With fewer blocks one CTA's chain bounds it, longer for many items (d=25, one block: 172 us for
-// 86), many hits (10,000 detectors, 20,000 mechanisms of p=0.1, 129 shots: 681 for 610), long unpacked rows (50,000
-// detectors, 129 shots: 380 for 99) and many stages (200,000 detectors, one shot: 207 for 65); and shuffled models draw a
-// segment once for each cluster of its detectors (d=25 shuffled, 65,536 shots: 1,526 for 1,264).
+// 86), many hits (10,000 detectors, 20,000 mechanisms of p=0.1, 129 shots: 666 for 610), long rows (50,000 detectors, 129
+// shots, unpacked: 207 for 99) and many stages (200,000 detectors, one shot: 202 for 65); and shuffled models draw a segment
+// once for each cluster of its detectors (d=25 shuffled, 65,536 shots: 1,533 for 1,264).
 bool symptoms_pay(const DemCost &c, uint64_t shots, uint64_t num_detectors, uint64_t row_bytes, bool packed);
 
 }  // namespace gfs

@@ -54,8 +54,8 @@ CASES = {
     "d25 shuffled": (shuffled_d25, "", "1p 129p 65536p"),
     "one window": (lambda: chain(100, 100, 0.001), "1p 1u 129u 65536p 65536u", ""),
     "one window, many hits": (lambda: chain(1000, 5000, 0.3, 1), "1p 1u 4097p 65536u", ""),
-    "sparse": (lambda: chain(10000, 400, 0.001), "1p 1u 129p 1025p 16384p", "129u 1025u 4097u"),
-    "in order": (lambda: chain(10000, 10000, 0.001), "1p 129p 1025p 16384p", "129u 1025u"),
+    "sparse": (lambda: chain(10000, 400, 0.001), "1p 1u 129p 1025p 16384p", ""),
+    "in order": (lambda: chain(10000, 10000, 0.001), "1p 129p 129u 1025p 16384p", ""),
     "many hits": (lambda: chain(10000, 20000, 0.1, 1), "16384p 65536p", "1u 129u 1025u 4097u"),
     "many hits, p=0.3": (lambda: chain(10000, 20000, 0.3, 1), "16384p 65536p", "1p 129p 129u 4097p"),
     "long rows": (lambda: chain(50000, 2000, 0.001), "", "1u 129p 129u 1025p 1025u"),
