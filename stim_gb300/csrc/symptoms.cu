@@ -357,16 +357,15 @@ __device__ __forceinline__ uint4 expand16(uint32_t v) {
 }
 
 // Unpacked rows up to this length are written word by word (us for 6 MB in host memory and 100 MB in device memory, words and
-// units: 24 columns 106 / 342 and 120 / 580, 201 columns 97 / 139 and 90 / 170, 333 columns 81 / 86 and 74 / 96, 400 columns
-// 61 / 78 and 55 / 65, 625 columns 72 / 88 and 68 / 80, 3,001 columns 79 / 64 and 61 / 37).
-constexpr uint32_t kWordRow = 350;
-static_assert(kWordRow >= 16, "longer rows hold a whole unit");
+// units: 24 columns 99 / 310 and 186 / 453, 100 columns 70 / 98 and 94 / 139, 150 columns 100 / 136 and 80 / 106, 333 columns
+// 82 / 86 and 66 / 58, 625 columns 72 / 88 and 64 / 59, 3,001 columns 79 / 63 and 58 / 35).
+constexpr uint32_t kWordRow = 128;
 
 // Unpacked rows, and rows of any kind in host memory (columns [c0, c1) of every shot): one warp per row, consecutive lanes
 // writing consecutive aligned 32-bit words, of four expanded bits or (a packed row's words are its destination's) as they are;
 // the partial words at the ends byte by byte.  Long unpacked rows leave in 16-byte units of sixteen expanded bits, four of a
-// lane on their way together, with words only at their ends: word by word, one load chain after another, a CTA wrote 13 GB/s,
-// which a few blocks of many detectors waited for (48,000 detectors, 129 shots: 644 us, now 277).
+// lane on their way together, and a byte a lane at their ends: word by word, one load chain after another, a CTA wrote 13
+// GB/s, which a few blocks of many detectors waited for (48,000 detectors, 129 shots: 644 us, now 277).
 template <bool PACKED>
 __device__ __forceinline__ void write_words(const SymArgs &a, const uint32_t *win, uint32_t c0, uint32_t c1,
                                             uint64_t shot0, uint32_t nvalid, uint32_t dst0, bool last) {
@@ -410,21 +409,11 @@ __device__ __forceinline__ void write_words(const SymArgs &a, const uint32_t *wi
             }
             continue;
         }
-        const uint32_t head = (uint32_t)(-(uintptr_t)d & 15u), units = (nbytes - head) / 16, tail = head + 16 * units;
-        if (lane < 4) {  // the words around the units, and the bytes around those
-            const uint32_t odd = head & 3u, c = odd + 4 * lane;
-            if (lane < 3 && c < head) {
-                word(c);
-            } else if (lane == 3) {
-                bytes(0, odd);
-            }
-        } else if (lane < 8) {
-            const uint32_t c = tail + 4 * (lane - 4);
-            if (c + 4 <= nbytes) {
-                word(c);
-            } else if (c < nbytes) {
-                bytes(c, nbytes - c);
-            }
+        const uint32_t head = min((uint32_t)(-(uintptr_t)d & 15u), nbytes), units = (nbytes - head) / 16, tail = head + 16 * units;
+        // The bytes before the first unit and after the last: one of each of two half warps' lanes.
+        const uint32_t edge = lane < 16 ? lane : tail + lane - 16;
+        if (edge < (lane < 16 ? head : nbytes)) {
+            d[edge] = (uint8_t)out_byte<false>(row, edge);
         }
         uint4 *const d16 = reinterpret_cast<uint4 *>(d + head);
         uint32_t q = lane;

@@ -15,8 +15,9 @@ def circuit(detectors):
                               + "OBSERVABLE_INCLUDE(0) rec[-1]\n")
 
 
-# Around one unit, the longest rows written word by word (350), the 32 units of a step, the 128 units of four, and several windows (more than 3,072 detectors).
-@pytest.mark.parametrize("detectors", [1, 2, 15, 16, 17, 33, 48, 349, 350, 351, 361, 511, 530, 2031, 2048, 2065, 2600, 4000, 9001])
+# Around one unit, the longest rows written word by word (128), the 32 units of a step, the 128 units of four, and several
+# windows (more than 3,072 detectors).
+@pytest.mark.parametrize("detectors", [1, 2, 15, 16, 17, 33, 127, 128, 129, 140, 511, 530, 2031, 2048, 2065, 2600, 4000, 9001])
 def test_every_alignment(detectors):
     torch = pytest.importorskip("torch")
     c, shots = circuit(detectors), 137
