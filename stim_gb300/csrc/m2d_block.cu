@@ -22,18 +22,16 @@ __host__ __device__ __forceinline__ uint32_t up32(uint32_t n) {
     return (n + 31) & ~31u;
 }
 
-// Output columns [c0, c0 + n) of Q, shot-major, `row` bytes a shot, to `dst` (any alignment): `groups` of 32 shots.
+// Output columns [c0, c0 + n) of Q, shot-major, `row` bytes a shot, to `dst` (any alignment).
+template <uint32_t GROUPS>
 __device__ __forceinline__ void rows_out(const uint4 *Q, uint32_t c0, uint32_t n, uint32_t row, uint8_t *dst,
-                                         uint32_t groups, const Transpose32 &turn) {
+                                         const Transpose32 &turn) {
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     for (uint32_t w = warp; w < (n + 31) / 32; w += kThreads / 32) {
         const uint4 v = 32 * w + lane < n ? Q[c0 + 32 * w + lane] : zero4();
         const uint32_t g[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (uint32_t k = 0; k < 4; k++) {
-            if (k >= groups) {
-                break;
-            }
+        for (uint32_t k = 0; k < GROUPS; k++) {
             const uint32_t x = turn(g[k]);
             uint8_t *const d = dst + (32 * k + lane) * row + 4 * w;
             const uint32_t left = row - 4 * w;  // bytes of this shot's row from here on
@@ -58,6 +56,9 @@ __device__ __forceinline__ void store_bytes(uint8_t *dst, const uint4 *src, uint
     }
 }
 
+// GROUPS: groups of 32 shots that are turned, all four or, in a call of no more shots than that, one (d=17, one shot: 49 us,
+// now 38; counted in the kernel the turns of whole blocks went out of step: 320 shots of d=3 29 us, then 36).
+template <uint32_t GROUPS>
 __global__ void __launch_bounds__(kThreads) convert_kernel(const ConvertArgs a, uint32_t first) {
     extern __shared__ uint4 sm[];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
@@ -67,7 +68,6 @@ __global__ void __launch_bounds__(kThreads) convert_kernel(const ConvertArgs a, 
     uint4 *const S = sm + first;  // staged records, then output rows
     const uint64_t shot0 = (uint64_t)blockIdx.x * kShots;
     const uint32_t nvalid = a.nshots - shot0 < kShots ? (uint32_t)(a.nshots - shot0) : kShots;
-    const uint32_t groups = (nvalid + 31) / 32;  // of 32 shots; those without a shot are not turned (d=17, one shot: 49 us, now 41)
     {
         // The records may lie in host memory (then this is the copy in): several 16-byte loads a thread in flight.
         const uint4 *const in = reinterpret_cast<const uint4 *>(a.in + shot0 * mrow);  // 128 rows: a multiple of 16 bytes
@@ -94,10 +94,7 @@ __global__ void __launch_bounds__(kThreads) convert_kernel(const ConvertArgs a, 
     for (uint32_t w = warp; w < up32(a.M) / 32; w += kThreads / 32) {
         uint32_t g[4] = {0, 0, 0, 0};
 #pragma unroll
-        for (uint32_t k = 0; k < 4; k++) {
-            if (k >= groups) {
-                break;
-            }
+        for (uint32_t k = 0; k < GROUPS; k++) {
             const uint32_t at = (32 * k + lane) * mrow + 4 * w;  // byte offset: two aligned words hold its four bytes
             g[k] = turn(__funnelshift_r(words[at >> 2], words[(at >> 2) + 1], 8 * (at & 3u)));
         }
@@ -131,10 +128,7 @@ __global__ void __launch_bounds__(kThreads) convert_kernel(const ConvertArgs a, 
             const uint4 v = 32 * w + lane < a.O ? S[a.D + 32 * w + lane] : zero4();
             const uint32_t g[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-            for (uint32_t k = 0; k < 4; k++) {
-                if (k >= groups) {
-                    break;
-                }
+            for (uint32_t k = 0; k < GROUPS; k++) {
                 const uint32_t x = turn(g[k]), shot = 32 * k + lane;
                 for (uint32_t b = 0; b < 4 && 4 * w + b < orow; b++) {
                     if (shot < nvalid) {
@@ -145,7 +139,7 @@ __global__ void __launch_bounds__(kThreads) convert_kernel(const ConvertArgs a, 
         }
     }
     if (a.dets && drow) {
-        rows_out(S, 0, dcols, drow, reinterpret_cast<uint8_t *>(R), groups, turn);
+        rows_out<GROUPS>(S, 0, dcols, drow, reinterpret_cast<uint8_t *>(R), turn);
         __syncthreads();
         store_bytes(a.dets + shot0 * drow, R, nvalid * drow);
     }
@@ -167,6 +161,19 @@ size_t convert_smem_bytes(uint32_t M, uint32_t D, uint32_t O, bool append) {
     return ((size_t)r + s) * sizeof(uint4);
 }
 
+template <uint32_t GROUPS>
+static cudaError_t launch_groups(const ConvertArgs &args, uint64_t grid, cudaStream_t stream) {
+    uint32_t r, s;
+    regions(args.M, args.D, args.O, args.append != 0, &r, &s);
+    const size_t smem = ((size_t)r + s) * sizeof(uint4);
+    cudaError_t e = allow_smem<convert_kernel<GROUPS>>(smem);
+    if (e != cudaSuccess) {
+        return e;
+    }
+    convert_kernel<GROUPS><<<(unsigned)grid, kThreads, smem, stream>>>(args, r);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_convert(const ConvertArgs &args, cudaStream_t stream) {
     const uint64_t grid = (args.nshots + kShots - 1) / kShots;
     if (grid == 0) {
@@ -175,15 +182,7 @@ cudaError_t launch_convert(const ConvertArgs &args, cudaStream_t stream) {
     if (grid > 0x7FFFFFFFull) {
         return cudaErrorInvalidValue;
     }
-    uint32_t r, s;
-    regions(args.M, args.D, args.O, args.append != 0, &r, &s);
-    const size_t smem = ((size_t)r + s) * sizeof(uint4);
-    cudaError_t e = allow_smem<convert_kernel>(smem);
-    if (e != cudaSuccess) {
-        return e;
-    }
-    convert_kernel<<<(unsigned)grid, kThreads, smem, stream>>>(args, r);
-    return cudaGetLastError();
+    return args.nshots <= 32 ? launch_groups<1>(args, grid, stream) : launch_groups<4>(args, grid, stream);
 }
 
 }  // namespace gfs
