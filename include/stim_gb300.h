@@ -230,16 +230,16 @@ gfs_status gfs_sampler_get_stream_position(const gfs_sampler *s, uint64_t *shot)
 /*
  * Noise generation: -1 (default) samples detection events by output lists where the circuit allows it (each noise hit
  * flips its precomputed detectors and observables in one kernel, without frames; also after gfs_sampler_set_shape),
- * otherwise as 1; 1 draws every noise
- * hit of a chunk in a separate kernel into a list that the frame kernel then applies; 0 draws noise inside the frame
- * kernel.  Results are identical either way.  No counterpart in the reference.
+ * otherwise as 1; 1 draws every noise hit of a chunk in a separate kernel into a list that the frame kernel then
+ * applies; 0 draws noise inside the frame kernel.  Results are identical either way.  No counterpart in the reference.
  */
 gfs_status gfs_sampler_set_noise_mode(gfs_sampler *s, int mode);
 /*
  * Frame kernel for hit-list launches (a choice other than -1 also keeps detection events from being sampled by output
  * lists): 1 (-1 = automatic) the lean kernel when the program has a lean phase list (no correlated errors, heralds or
- * sweep feedback; compact unit lists; at most two loop levels), 0 the generic kernel.  Results are identical either way.  gfs_sampler_get_frame_kernel reports which one the
- * next hit-list launch uses (1 lean, 0 generic).  No counterpart in the reference.
+ * sweep feedback; compact unit lists; at most two loop levels), 0 the generic kernel.  Results are identical either
+ * way.  gfs_sampler_get_frame_kernel reports which one the next hit-list launch uses (1 lean, 0 generic).  No
+ * counterpart in the reference.
  */
 gfs_status gfs_sampler_set_frame_kernel(gfs_sampler *s, int kind);
 gfs_status gfs_sampler_get_frame_kernel(const gfs_sampler *s, int *kind);
@@ -265,10 +265,11 @@ gfs_status gfs_sampler_last_counts(const gfs_sampler *s, uint64_t *counts4);
 gfs_status gfs_sampler_autotune(gfs_sampler *s, uint64_t trial_shots, double *best_ms);
 
 /*
- * Batched sampling: the next shots of many detection samplers in ONE persistent frame-kernel launch
- * (work items = (circuit, 128-shot slice), claimed dynamically by the CTAs, most expensive circuits
- * first), followed by each circuit's transpose; the launch sequence is captured as a CUDA graph and
- * replayed while shot counts, destinations and launch shape stay the same.  Entry j returns exactly what
+ * Batched sampling: the next shots of many detection samplers in a few launches: up to four for the circuits that
+ * are sampled by output lists (gfs_sampler_set_noise_mode), which write the rows as they are, and for the others ONE
+ * persistent frame-kernel launch (work items = (circuit, 128-shot slice), claimed dynamically by the CTAs, most
+ * expensive circuits first) followed by each circuit's transpose.  The launch sequence is captured as a CUDA graph and
+ * replayed while shot counts, destinations, launch shape and each circuit's way stay the same.  Entry j returns exactly what
  * gfs_sample_detections(samplers[j], shots[j], ...) would have returned at that point, and advances that
  * sampler the same way (a sampler listed twice continues its stream from the first entry to the second).
  * The samplers must stay alive, on one device, and unused elsewhere while the batch is in use.
@@ -285,7 +286,8 @@ gfs_status gfs_batch_sample_detections_device(gfs_batch *b, const uint64_t *shot
 /* Same with host destinations (copied out of a device staging arena). */
 gfs_status gfs_batch_sample_detections(gfs_batch *b, const uint64_t *shots, uint32_t flags, uint8_t *const *dets,
                                        const uint64_t *dets_stride, uint8_t *const *obs, const uint64_t *obs_stride);
-/* Launch shape of the batched kernel (ring_placement as in gfs_sampler_set_ring_placement). */
+/* Launch shape of the batched frame kernel (ring_placement as in gfs_sampler_set_ring_placement).  A chosen shape also
+ * chooses that kernel for every circuit of the batch, until gfs_batch_autotune. */
 gfs_status gfs_batch_set_shape(gfs_batch *b, int blocks_per_cta, int threads, int ring_placement);
 gfs_status gfs_batch_get_shape(const gfs_batch *b, int *blocks_per_cta, int *threads, int *grid, uint64_t *smem_bytes,
                                int *ring_global);

@@ -684,7 +684,8 @@ class CompiledDemSampler:
 
 
 class BatchSampler:
-    """The next shots of many detection samplers in one persistent kernel launch (replayed as a CUDA graph).
+    """The next shots of many detection samplers in a few kernel launches (replayed as a CUDA graph): up to four for the
+    circuits sampled by output lists, one persistent one for those that need frames.
 
     Entry j of a call returns exactly what ``samplers[j].sample(shots[j], ...)`` would have returned at that
     point and advances that sampler the same way.  No counterpart in the reference, where each circuit has
@@ -773,6 +774,7 @@ class BatchSampler:
         check(lib().gfs_batch_sample_detections_device(self._h, cshots, flags, dptr, dstr, optr, ostr))
 
     def set_launch_shape(self, blocks_per_cta: int, threads: int = 256, ring_placement: int = -1):
+        """Shape of the batched frame kernel, which a chosen shape also selects for every circuit (until autotune)."""
         check(lib().gfs_batch_set_shape(self._h, int(blocks_per_cta), int(threads), int(ring_placement)))
 
     def launch_shape(self):

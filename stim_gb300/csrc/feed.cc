@@ -53,7 +53,7 @@ void sample_for_decoder(gfs_sampler *s, uint64_t shots, const uint8_t *mask, uin
     const bool symptoms = s->symptoms_active(GFS_BIT_PACKED);
     if (symptoms) {
         // Symptom sampling has no waves to fill: 40 MiB of rows per chunk, so that copies of kept rows overlap the next
-        // chunk's kernels from early on (d=15, 2^18 shots: 667 us; 24 MiB 705, 32 689, 48 688, one chunk 809).
+        // chunk's kernels from early on (d=15, 2^18 shots, in one run: 667 us; 24 MiB 705, 32 689, 48 688, one chunk 809; other runs 676-700).
         chunk = std::max<uint64_t>(128, ((uint64_t)40 << 20) / per_shot / 128 * 128);
     }
     chunk = std::min<uint64_t>(chunk, (shots + 127) / 128 * 128);

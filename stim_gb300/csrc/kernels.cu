@@ -1888,7 +1888,7 @@ __global__ void __launch_bounds__(256) feed_popcount_kernel(const uint8_t *p, ui
 }
 
 // Masks of a few bytes: one thread per shot, 256 shots of one group per CTA (the warp-per-shot kernel below spends a warp
-// on three bytes: 36 us per 2^18 shots of d=15, 24 detectors; this 8).
+// on three bytes: 36 us per 2^18 shots of d=15, 24 detectors; this 11).
 constexpr uint32_t kFewMaskBytes = 16;
 __global__ void __launch_bounds__(256) feed_few_flags_kernel(const FeedArgs a) {
     const uint64_t s = (uint64_t)blockIdx.x * 256 + threadIdx.x;

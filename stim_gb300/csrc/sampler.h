@@ -285,7 +285,7 @@ struct SymptomDevice {
     // device has no room (the other kernels need none of it).
     //
     // All outputs of a block at once while its rows take at most 50 KB, else a window: 124 words a shot, the most that
-    // leaves three CTAs per SM, where the stages fit (d=25: 2.04 ms per 2^20 shots; 112 words, six stages for five: 2.12;
+    // leaves three CTAs per SM, where the stages fit (d=25, CTAs of eight warps: 2.04 ms per 2^20 shots; 112 words, six stages for five: 2.12;
     // 76, four CTAs: 2.58; 56, five: 3.25), otherwise 248.
     template <typename Plan>
     void init(int device, cudaStream_t stream, const gfs::SymLists &lists, uint64_t D, uint64_t O, uint64_t seed,

@@ -11,10 +11,11 @@
 // full; where few segments have a hit (error models), the first gap decides which are drawn at all.  Hits go to a second
 // queue and are applied 32 at a time, one per lane, each list loaded one step before it is applied.
 //
-// What bounds it: instruction issue (d=25: 203 K warp instructions per block, a quarter of them Philox and gap
-// arithmetic that the contract asks for; 0.55 of the issue slots used, the rest fixed latencies and barriers).  The output
-// alone would take 0.31 ms at d=25 (2.05 GB per 2^20 shots at 6.7 TB/s), the contract's Philox calls 0.18 ms (580 G
-// calls/s).  d=25, p=1e-3, 2^20 shots: 1.97 ms where noise, frame and transpose kernels took 7.81; d=11, p=5e-3: 0.56 ms
+// What bounds it: instruction issue (d=25: 192 K warp instructions per block, 0.58 of the issue slots used, the rest fixed
+// latencies and barriers).  A quarter of the instructions are the Philox and gap arithmetic that the contract asks for, and a
+// quarter apply the hits, fill the queues, move the window and write the rows; what the other half goes to has not been taken
+// apart.  The output alone would take 0.31 ms at d=25 (2.05 GB per 2^20 shots at 6.7 TB/s), the contract's Philox calls 0.18
+// ms (580 G calls/s).  d=25, p=1e-3, 2^20 shots: 1.97 ms where noise, frame and transpose kernels took 7.81; d=11, p=5e-3: 0.56 ms
 // (2.22); d=13 colour code, p=1e-2, 200,001 shots: 0.24 ms (0.97).  On the way at d=25: hits applied as each lane draws
 // them, with the gap table for every draw, 5.2 ms; the float estimate of the gap instead of the table and prefetched
 // descriptors 3.7; the hit queue 2.9; rows written by bulk copies instead of word stores 2.46; queued segments instead of

@@ -34,8 +34,10 @@ static_assert(sizeof(SymItem) == 32, "SymItem layout");
 
 constexpr uint32_t kSymAlign = 128;  // detectors per 16 bytes of a packed row, the unit of bulk copies
 
-// A stage draws items [item0, item1) and then writes detectors [flush0, flush1) out (flush0 and, except in the last
-// stage, flush1 are multiples of 32): no later item reaches them.  `keep` words past flush1 may hold flips already.
+// A stage draws items [item0, item1) and then writes detectors [flush0, flush1) out: no later item reaches them.  flush0 and,
+// except in the last stage, flush1 are multiples of kSymAlign: rows leave by bulk copies of 16 bytes and move by 16-byte
+// units.  The `keep` words past flush1, a whole number of such units, are those that may hold flips already, and one unit more:
+// rows lie shifted by up to one unit, as their destinations do.
 struct alignas(16) SymStage {
     uint32_t item0, item1, flush0, flush1, keep, pad[3];
 };
