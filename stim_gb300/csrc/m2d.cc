@@ -243,8 +243,9 @@ void convert(gfs_m2d *m, uint64_t shots, const uint8_t *meas, uint64_t meas_stri
     // copy from pageable memory holds the calling thread and runs at half the link's rate (d=11, 2^18 shots: 508 us with
     // copies, 468 without).  From page-locked memory the copy engine is the faster one, except for small calls, which a
     // copy only delays (d=3, 1,024 shots: 31 us).
-    const bool direct = fused && m->reads_host && meas_stride == mrow && ((uintptr_t)meas & 15) == 0 &&
-                        (shots * mrow <= (1u << 20) || !page_locked({meas}));
+    const cudaMemoryType kind = fused && m->reads_host ? memory_kind(meas) : cudaMemoryTypeDevice;
+    const bool direct = kind != cudaMemoryTypeDevice && meas_stride == mrow && ((uintptr_t)meas & 15) == 0 &&
+                        (shots * mrow <= (1u << 20) || kind != cudaMemoryTypeHost);
     // Chunks of up to 2^16 shots, fewer when a circuit's rows are large (about 1 GiB of device buffers).
     const uint64_t per_block = (M + D + O) * 16 + 128 * (mrow + drow + orow);
     uint64_t cb = std::max<uint64_t>(1, std::min<uint64_t>(512, ((uint64_t)1 << 30) / std::max<uint64_t>(1, per_block)));
@@ -277,9 +278,9 @@ void convert(gfs_m2d *m, uint64_t shots, const uint8_t *meas, uint64_t meas_stri
     auto compute = [&](int k, uint64_t done, uint64_t cs, const uint4 *base_dets, const uint4 *base_obs) {
         cudaStream_t st = m->streams[k];
         const uint64_t nblk = (cs + 127) / 128;
-        if (direct) {
+        if (direct && kind != cudaMemoryTypeHost) {
             touch_pages({meas + done * mrow, cs, mrow, mrow}, false);
-        } else {
+        } else if (!direct) {
             copy2d(m->in_buf[k].p, mrow, meas + done * meas_stride, meas_stride, mrow, cs, cudaMemcpyHostToDevice, st,
                    "copy measurements");
         }
